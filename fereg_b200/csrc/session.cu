@@ -220,56 +220,76 @@ void GpuSession::phase_times(double* ms, u64* counts) const {
     }
 }
 
-// dof.rs:222-256 mobility_groups of terms qa, qb on the device; save: keep the row labels.
-// Runs on the dof pass's stream with its buffers.
-u64 GpuSession::mobility_groups(size_t qa, size_t qb, bool save, DofScratch& s) {
+// dof.rs:222-256 mobility_groups of terms qa, qb on the device, the count into out[0] and the
+// union-find's error flag into out[1] (device words, zeroed by the caller); save: keep the row
+// labels. Queued on the dof pass's stream with its buffers.
+void GpuSession::mobility_groups(size_t qa, size_t qb, bool save, u32* out, DofScratch& s) {
     SessionDev& d = *d_;
     const cudaStream_t st = s.st.s;
     const u32 ga = tg_[qa], gb = tg_[qb], nv = ga + gb;
     s.uf.alloc(nv);
-    s.flags.alloc(ga);
-    s.scan.alloc(ga);
-    s.bsum.alloc((ga + SCAN_TILE - 1) / SCAN_TILE + 1);
-    s.total.alloc(1);
-    s.err.alloc(1);
-    CK(cudaMemsetAsync(s.err.p, 0, sizeof(int), st));
     k_uf_init<<<blocks_for(nv, 256), 256, 0, st>>>(s.uf.p, nv);
-    k_uf_union<<<blocks_for(n_, 256), 256, 0, st>>>(d.tcodes[qa].p, d.tcodes[qb].p, ga, n_, s.uf.p, s.err.p);
-    k_uf_flatten<<<blocks_for(nv, 256), 256, 0, st>>>(s.uf.p, nv);
-    k_uf_roots<<<blocks_for(ga, 256), 256, 0, st>>>(s.uf.p, ga, s.flags.p);
-    const u32 nblk = (ga + SCAN_TILE - 1) / SCAN_TILE;
-    k_scan_sums<<<nblk, SCAN_TB, 0, st>>>(s.flags.p, ga, s.bsum.p);
-    k_scan_top<<<1, SCAN_TB, 0, st>>>(s.bsum.p, nblk, s.total.p);
-    k_scan_apply<<<nblk, SCAN_TB, 0, st>>>(s.flags.p, ga, s.bsum.p, s.scan.p);
-    s.launches += 7;
-    if (save) {
-        s.gv.alloc(n_);
-        k_uf_label<<<blocks_for(n_, 256), 256, 0, st>>>(d.tcodes[qa].p, n_, s.uf.p, s.scan.p, s.gv.p);
+    // two prefixes and the rest (k_uf_union); short samples in one launch
+    for (size_t at = 0, part = n_ >= UF_SPLIT_MIN ? 256 : 1; at < n_; part = std::max<size_t>(1, part / 16)) {
+        const size_t to = n_ / part;
+        k_uf_union<<<blocks_for((to - at + UF_ROWS - 1) / UF_ROWS, 256), 256, 0, st>>>(
+            d.tcodes[qa].p, d.tcodes[qb].p, ga, at, to, s.uf.p, reinterpret_cast<int*>(out + 1));
         s.launches++;
+        at = to;
+        if (at < n_) {
+            k_uf_flatten<<<blocks_for(nv, 256), 256, 0, st>>>(s.uf.p, nv);
+            s.launches++;
+        }
     }
-    u32 total = 0;
-    int err = 0;
-    CK(cudaMemcpyAsync(&total, s.total.p, sizeof(u32), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&err, s.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (err) throw Error(RC_INTERNAL, "fereg: union-find did not settle");
-    return total;
+    k_uf_count<<<blocks_for(ga, 256), 256, 0, st>>>(s.uf.p, ga, out);
+    s.launches += 2;
+    if (save) {
+        s.flags.alloc(ga);
+        s.scan.alloc(ga);
+        s.bsum.alloc((ga + SCAN_TILE - 1) / SCAN_TILE + 1);
+        s.total.alloc(1);
+        s.gv.alloc(n_);
+        k_uf_flatten<<<blocks_for(nv, 256), 256, 0, st>>>(s.uf.p, nv);
+        k_uf_roots<<<blocks_for(ga, 256), 256, 0, st>>>(s.uf.p, ga, s.flags.p);
+        const u32 nblk = (ga + SCAN_TILE - 1) / SCAN_TILE;
+        k_scan_sums<<<nblk, SCAN_TB, 0, st>>>(s.flags.p, ga, s.bsum.p);
+        k_scan_top<<<1, SCAN_TB, 0, st>>>(s.bsum.p, nblk, s.total.p);
+        k_scan_apply<<<nblk, SCAN_TB, 0, st>>>(s.flags.p, ga, s.bsum.p, s.scan.p);
+        k_uf_label<<<blocks_for(n_, 256), 256, 0, st>>>(d.tcodes[qa].p, n_, s.uf.p, s.scan.p, s.gv.p);
+        s.launches += 6;
+    }
+    CK(cudaGetLastError());
 }
 
-// dof.rs:184 nested_within: every level of term q lies in one level of cluster dimension c.
-bool GpuSession::nested_within(size_t q, size_t c, DofScratch& s) {
+// dof.rs:184 nested_within: for each term of qs, whether every level lies in one level of cluster
+// dimension c. One read-back for all of them.
+std::vector<uint8_t> GpuSession::nested_within(const std::vector<size_t>& qs, size_t c, DofScratch& s) {
     SessionDev& d = *d_;
     const cudaStream_t st = s.st.s;
-    s.map.alloc(tg_[q]);
-    s.err.alloc(1);
-    CK(cudaMemsetAsync(s.map.p, 0xff, size_t(tg_[q]) * sizeof(u32), st));
-    CK(cudaMemsetAsync(s.err.p, 0, sizeof(int), st));
-    k_nested<<<blocks_for(n_, 256), 256, 0, st>>>(d.tcodes[q].p, d.ccodes[c].p, n_, s.map.p, s.err.p);
-    s.launches++;
-    int flag = 0;
-    CK(cudaMemcpyAsync(&flag, s.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    size_t len = qs.size();  // the flags, then each term's map
+    for (size_t q : qs) len += tg_[q];
+    s.map.alloc(len);
+    CK(cudaMemsetAsync(s.map.p, 0, qs.size() * sizeof(u32), st));
+    CK(cudaMemsetAsync(s.map.p + qs.size(), 0xff, (len - qs.size()) * sizeof(u32), st));
+    u32* map = s.map.p + qs.size();
+    for (size_t i = 0; i < qs.size(); i++) {
+        // a prefix and the rest (k_nested); short samples in one launch
+        for (size_t at = 0, part = n_ >= UF_SPLIT_MIN ? 256 : 1; at < n_; part = 1) {
+            const size_t to = n_ / part;
+            k_nested<<<blocks_for(to - at, 256), 256, 0, st>>>(d.tcodes[qs[i]].p, d.ccodes[c].p, at, to, map,
+                                                               reinterpret_cast<int*>(s.map.p + i));
+            s.launches++;
+            at = to;
+        }
+        map += tg_[qs[i]];
+    }
+    CK(cudaGetLastError());
+    std::vector<u32> flag(qs.size());
+    CK(cudaMemcpyAsync(flag.data(), s.map.p, qs.size() * sizeof(u32), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    return flag == 0;
+    std::vector<uint8_t> nested(qs.size());
+    for (size_t i = 0; i < qs.size(); i++) nested[i] = flag[i] == 0;
+    return nested;
 }
 
 // Starts the dof pass (dof.rs:64-180 does not depend on the data columns) on a host thread of
@@ -361,15 +381,21 @@ GpuSession::Dof GpuSession::dof_pass(bool clusters, bool firstpair, bool want_gr
     for (size_t i = 0; i < ns; i++) live[i] = icpt_term[i] >= 0;
     if (clusters && !firstpair)
         for (size_t c = 0; c < ccodes_.size(); c++) {
-            if (std::none_of(live.begin(), live.end(), [](bool x) { return x; })) break;
-            for (size_t i = 0; i < ns; i++) {
-                if (!live[i] || dof.slots[i].exact) continue;
-                if (nested_within(size_t(icpt_term[i]), c, s)) {
-                    dof.slots[i].m = dof.slots[i].k;
-                    dof.slots[i].exact = dof.slots[i].nested = true;
-                    dof.df_a_nested += dof.slots[i].k;
-                    live[i] = false;
+            std::vector<size_t> at, qs;  // the live intercept slots and their terms
+            for (size_t i = 0; i < ns; i++)
+                if (live[i] && !dof.slots[i].exact) {
+                    at.push_back(i);
+                    qs.push_back(size_t(icpt_term[i]));
                 }
+            if (at.empty()) break;
+            const std::vector<uint8_t> nested = nested_within(qs, c, s);
+            for (size_t a = 0; a < at.size(); a++) {
+                if (!nested[a]) continue;
+                const size_t i = at[a];
+                dof.slots[i].m = dof.slots[i].k;
+                dof.slots[i].exact = dof.slots[i].nested = true;
+                dof.df_a_nested += dof.slots[i].k;
+                live[i] = false;
             }
         }
     const size_t remaining = size_t(std::count(live.begin(), live.end(), true));
@@ -394,22 +420,27 @@ GpuSession::Dof GpuSession::dof_pass(bool clusters, bool firstpair, bool want_gr
     std::vector<size_t> idx;
     for (size_t i = 0; i < ns; i++)
         if (live[i]) idx.push_back(i);
-    int pairs = 0;
-    for (size_t a = 0; a < idx.size(); a++) {
-        bool stop = false;
-        for (size_t b = a + 1; b < idx.size(); b++) {
-            pairs++;
-            const bool save = pairs == 1 && want_groupvar;
-            const u64 m = mobility_groups(size_t(icpt_term[idx[a]]), size_t(icpt_term[idx[b]]), save, s);
-            if (save) dof.has_groupvar = true;
-            dof.slots[idx[b]].m = std::max(dof.slots[idx[b]].m, m);
-            if (pairs == 1) dof.slots[idx[b]].exact = true;
-            if (firstpair) {
-                stop = true;
-                break;
-            }
+    // the pairs in order (firstpair: the first alone), all queued before the one read-back
+    std::vector<std::pair<size_t, size_t>> pairs;
+    for (size_t a = 0; a < idx.size(); a++)
+        for (size_t b = a + 1; b < idx.size(); b++)
+            if (!firstpair || pairs.empty()) pairs.push_back({idx[a], idx[b]});
+    if (!pairs.empty()) {
+        s.out.alloc(2 * pairs.size());
+        CK(cudaMemsetAsync(s.out.p, 0, 2 * pairs.size() * sizeof(u32), s.st.s));
+        for (size_t p = 0; p < pairs.size(); p++)
+            mobility_groups(size_t(icpt_term[pairs[p].first]), size_t(icpt_term[pairs[p].second]),
+                            p == 0 && want_groupvar, s.out.p + 2 * p, s);
+        std::vector<u32> got(2 * pairs.size());
+        CK(cudaMemcpyAsync(got.data(), s.out.p, got.size() * sizeof(u32), cudaMemcpyDeviceToHost, s.st.s));
+        CK(cudaStreamSynchronize(s.st.s));
+        dof.has_groupvar = want_groupvar;
+        dof.slots[pairs[0].second].exact = true;
+        for (size_t p = 0; p < pairs.size(); p++) {
+            if (got[2 * p + 1]) throw Error(RC_INTERNAL, "fereg: union-find did not settle");
+            DofSlot& sl = dof.slots[pairs[p].second];
+            sl.m = std::max<u64>(sl.m, got[2 * p]);
         }
-        if (stop) break;
     }
     // slopes constant (term with intercept) or zero (term without) within a level
     for (size_t q = 0; q < nt; q++)

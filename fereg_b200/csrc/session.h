@@ -217,8 +217,8 @@ class GpuSession {
         bool y_absorbed = false;
     };
     FitState fit_;
-    u64 mobility_groups(size_t qa, size_t qb, bool save, DofScratch& s);
-    bool nested_within(size_t q, size_t c, DofScratch& s);
+    void mobility_groups(size_t qa, size_t qb, bool save, u32* out, DofScratch& s);
+    std::vector<uint8_t> nested_within(const std::vector<size_t>& qs, size_t c, DofScratch& s);
 };
 
 }  // namespace fereg

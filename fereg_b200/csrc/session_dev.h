@@ -27,8 +27,7 @@ struct DofScratch {
     OwnedStream st;              // declared first: destroyed after the buffers allocated on it
     cudaEvent_t ready = nullptr; // recorded on the session's stream before the pass starts
     cudaEvent_t ta = nullptr, tb = nullptr;  // phase timing of the pass (when profiling)
-    DBuf<u32> uf, flags, scan, bsum, total, gv, map;
-    DBuf<int> err;
+    DBuf<u32> uf, flags, scan, bsum, total, gv, map, out;
     u64 launches = 0;
     ~DofScratch() {
         if (ready) cudaEventDestroy(ready);
