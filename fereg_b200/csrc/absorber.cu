@@ -428,19 +428,16 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
             d_->cw_list_off.upload(loff, stream_);
         }
         if (hs_.m_small > 0 && hs_.m_small <= DENSE_SMALL_MAX) {
-            // runs of each small coordinate's entries, at least `run` long, never splitting a segment
+            // runs of each small coordinate's entries, a few thousand in all, a warp each
             const u32 es = pl_off[hs_.m_small];
-            const u32 run = std::max<u32>(256, es / 4096);
+            const u32 run = std::max<u32>(128, (es / 4096 + 31) / 32 * 32);
             std::vector<u32> ik, ia, ib, first(hs_.m_small + 1, 0);
             for (u32 k = 0; k < u32(hs_.m_small); k++) {
                 first[k] = u32(ik.size());
-                for (u32 a = pl_off[k]; a < pl_off[k + 1];) {
-                    u32 b = std::min(pl_off[k + 1], a + run);
-                    while (b < pl_off[k + 1] && pl_seg[b] == pl_seg[b - 1]) b++;
+                for (u32 a = pl_off[k]; a < pl_off[k + 1]; a += run) {
                     ik.push_back(k);
                     ia.push_back(a);
-                    ib.push_back(b);
-                    a = b;
+                    ib.push_back(std::min(pl_off[k + 1], a + run));
                 }
             }
             first[hs_.m_small] = u32(ik.size());
@@ -848,8 +845,7 @@ void GpuAbsorber::ensure_precond() {
 }
 
 // The dense small factor from the device assembly of S_SS (weights.cuh) for the device weight
-// state: by rows (k_small_rows over the work items built with the coordinate lists), each row's
-// items summed in item order.
+// state: as a Gram matrix over the segments, or by the lists' entries where that is less work.
 void GpuAbsorber::build_small_device() {
     const HostStructure& st = hs_;
     const size_t ms = st.m_small, M = st.ncells;
@@ -857,21 +853,39 @@ void GpuAbsorber::build_small_device() {
     int ns = 0;
     for (auto& b : st.blocks) ns += b.small;
     const size_t len = ms * ms;
-    DBuf<double> part, a, ak, dd, dx, dscale;
+    DBuf<double> part, gpart, a, ak, dd, dx, dscale;
     DBuf<u32> dkeep;
     a.alloc(len);
-    if (d.sr_n > 0) {
-        part.alloc(size_t(d.sr_n) * ms);
-        const size_t shm = size_t(8) * ms * sizeof(double);
+    const size_t T = (ms + (ms <= 16 ? 15 : 63)) / (ms <= 16 ? 16 : 64), tiles = T * (T + 1) / 2;
+    const bool gram = tiles * st.g1 <= M * size_t(ns);  // see k_small_gram
+    const size_t shm = size_t(8) * ms * sizeof(double);
+    const u32 ni = d.sr_n;
+    if (ni > 0 && (ns > 1 || !gram)) part.alloc(size_t(ni) * ms);
+    if (part.p && gram) {
+        allow_smem(k_small_cross, shm);
+        k_small_cross<<<(ni + 7) / 8, 256, shm, stream_>>>(d.coord.p, u32(M), ns, u32(ms), d.cell_w.p, d.pl_cell.p,
+                                                           d.sr_k.p, d.sr_a.p, d.sr_b.p, ni, part.p);
+    } else if (part.p) {
         allow_smem(k_small_rows, shm);
-        k_small_rows<<<(d.sr_n + 7) / 8, 256, shm, stream_>>>(d.seg_off.p, d.coord.p, u32(M), ns, u32(ms),
-                                                               d.cell_w.p, d.n1inv.p, d.pl_cell.p, d.pl_seg.p,
-                                                               d.sr_k.p, d.sr_a.p, d.sr_b.p, d.sr_n, part.p);
-        k_small_rows_sum<<<u32(ms), 256, 0, stream_>>>(part.p, d.sr_first.p, u32(ms), a.p);
-        d.launches += 2;
-    } else {  // no small coordinate has a cell
-        CK(cudaMemsetAsync(a.p, 0, len * sizeof(double), stream_));
+        k_small_rows<<<(ni + 7) / 8, 256, shm, stream_>>>(d.seg_off.p, d.coord.p, u32(M), ns, u32(ms), d.cell_w.p,
+                                                           d.n1inv.p, d.pl_off.p, d.pl_cell.p, d.pl_seg.p, d.sr_k.p,
+                                                           d.sr_a.p, d.sr_b.p, ni, part.p);
     }
+    auto assemble = [&](auto btc) {
+        constexpr int BT = decltype(btc)::value;
+        const u32 chunks = (st.g1 + SgTile<BT>::TS - 1) / SgTile<BT>::TS;
+        const u32 nsplit = std::max<u32>(1, std::min<u32>(chunks, u32(148 * 4 / tiles)));
+        if (gram) {
+            gpart.alloc(size_t(tiles) * nsplit * BT * BT);
+            k_small_gram<BT><<<dim3(nsplit, u32(tiles)), 256, 0, stream_>>>(d.seg_off.p, d.coord.p, u32(M), st.g1, ns,
+                                                                       d.cell_w.p, d.n1inv.p, gpart.p);
+        }
+        k_small_combine<BT><<<grid_for(len * 32), THREADS, 0, stream_>>>(part.p, d.sr_first.p, gpart.p, nsplit,
+                                                                         d.nr.p, u32(ms), a.p);
+    };
+    if (ms <= 16) assemble(std::integral_constant<int, 16>{});
+    else assemble(std::integral_constant<int, 64>{});
+    d.launches += 1 + (part.p != nullptr) + gram;
     // kept coordinates (not redundant, positive diagonal) and their unit-diagonal scaling
     std::vector<double> diag(ms);
     std::vector<uint8_t> red(ms);
@@ -921,10 +935,9 @@ void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st,
     if (k <= 0) return;
     auto factor = [&](auto nbc) {
         constexpr int NB = decltype(nbc)::value;
-        allow_smem(k_ldlt_panel<NB>, size_t(k) * NB * sizeof(double));
         for (int jb = 0; jb < k; jb += NB) {
             const int nb = std::min(NB, k - jb);
-            k_ldlt_panel<NB><<<1, 1024, size_t(k - jb) * NB * sizeof(double), st>>>(a, d, k, jb);
+            k_ldlt_panel<NB><<<1, 1024, 0, st>>>(a, d, k, jb);
             launches++;
             const int T = (k - jb - nb + 31) / 32;  // trailing tiles per side
             if (T > 0) {
@@ -933,10 +946,31 @@ void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st,
             }
         }
     };
-    if (k <= 1024) factor(std::integral_constant<int, 16>{});
-    else factor(std::integral_constant<int, 8>{});
-    allow_smem(k_ldlt_inverse, size_t(8) * k * sizeof(double));
-    k_ldlt_inverse<<<(k + 7) / 8, 256, size_t(8) * k * sizeof(double), st>>>(a, d, k, x);
+    if (k <= LDLT_WHOLE) {
+        if (k <= 32) k_ldlt_whole<2><<<1, 256, 0, st>>>(a, d, k);
+        else if (k <= 64) k_ldlt_whole<4><<<1, 256, 0, st>>>(a, d, k);
+        else if (k <= 112) k_ldlt_whole<7><<<1, 256, 0, st>>>(a, d, k);
+        else k_ldlt_whole<LDLT_WHOLE / 16><<<1, 256, 0, st>>>(a, d, k);
+        launches++;
+    } else if (k <= 1024) {
+        factor(std::integral_constant<int, 16>{});
+    } else {
+        factor(std::integral_constant<int, 8>{});
+    }
+    auto inverse = [&](auto nrc, auto ncc) {
+        constexpr int NR = decltype(nrc)::value, NC = decltype(ncc)::value;
+        k_ldlt_inverse<NR, NC><<<(k + 4 * NC - 1) / (4 * NC), 128, 0, st>>>(a, d, k, x);
+    };
+    using std::integral_constant;
+    const integral_constant<int, 1> one;
+    if (k <= 32) inverse(one, one);
+    else if (k <= 128) inverse(integral_constant<int, 4>{}, one);
+    else if (k <= 512) inverse(integral_constant<int, 16>{}, one);
+    else if (k <= 1024) inverse(integral_constant<int, 32>{}, integral_constant<int, 2>{});
+    else {
+        allow_smem(k_ldlt_inverse_wide, size_t(8) * k * sizeof(double));
+        k_ldlt_inverse_wide<<<(k + 7) / 8, 256, size_t(8) * k * sizeof(double), st>>>(a, d, k, x);
+    }
     launches++;
     CK(cudaGetLastError());
 }

@@ -275,39 +275,128 @@ __global__ void k_small_apply(const double* __restrict__ minv, u32 ms, const T* 
 constexpr double PIVOT_TOL = 1e-10;
 constexpr double GROUND = 1e30;
 
+// The panel: thread t holds the panel elements of rows t, t + 1024, ... in registers, the pivot
+// rows' current column passes through shared memory, one barrier per column, the divisions by
+// the first warp alone. k = 910: the panel in shared memory with a division per element and two
+// barriers a column 59 us, here 19 us.
 template <int NB>
 __global__ void __launch_bounds__(1024) k_ldlt_panel(double* __restrict__ a, double* __restrict__ d, int k, int jb) {
-    extern __shared__ double P[];  // rows jb..k-1 of the panel columns jb..jb+NB-1, NB per row
+    constexpr int RPT = 16 / NB;  // rows per thread: k is at most 1024 with 16 columns, 2048 with 8
+    __shared__ double top[2][NB], piv[2];
     const int nb = min(NB, k - jb), rows = k - jb;
-    for (int idx = threadIdx.x; idx < rows * NB; idx += blockDim.x) {
-        const int r = idx / NB, c = idx % NB;
-        P[idx] = (c < nb && r >= c) ? a[size_t(jb + r) * k + jb + c] : 0.0;
+    double p[RPT][NB];
+#pragma unroll
+    for (int q = 0; q < RPT; q++) {
+        const int r = int(threadIdx.x) + 1024 * q;
+#pragma unroll
+        for (int c = 0; c < NB; c++) p[q][c] = (r < rows && c < nb && r >= c) ? a[size_t(jb + r) * k + jb + c] : 0.0;
     }
-    for (int jj = 0; jj < nb; jj++) {
-        __syncthreads();
-        double dj = P[jj * NB + jj];
-        if (dj <= PIVOT_TOL) dj = GROUND;
-        if (threadIdx.x == 0) d[jb + jj] = dj;
-        // the panel's later columns: P[r][l] -= P[r][jj] P[l][jj] / dj for jj < l <= r
-        for (int idx = threadIdx.x; idx < (rows - jj - 1) * NB; idx += blockDim.x) {
-            const int r = jj + 1 + idx / NB, l = idx % NB;
-            if (l > jj && l < nb && l <= r) P[r * NB + l] -= P[r * NB + jj] * P[l * NB + jj] / dj;
+#pragma unroll
+    for (int jj = 0; jj < NB; jj++) {
+        if (jj < nb) {
+            // the pivot rows divide; the others would spend the FP64 pipe on the same quotients
+            if (int(threadIdx.x) < 32) {
+                double dj = __shfl_sync(FULL, p[0][jj], jj);
+                if (dj <= PIVOT_TOL) dj = GROUND;
+                if (threadIdx.x == 0) {
+                    d[jb + jj] = dj;
+                    piv[jj & 1] = 1.0 / dj;
+                }
+                if (int(threadIdx.x) < NB) top[jj & 1][threadIdx.x] = p[0][jj] / dj;
+            }
+            __syncthreads();
+            const double inv = piv[jj & 1];
+#pragma unroll
+            for (int q = 0; q < RPT; q++) {
+                const int r = int(threadIdx.x) + 1024 * q;
+                const double m = p[q][jj];
+#pragma unroll
+                for (int l = jj + 1; l < NB; l++)
+                    if (l < nb) p[q][l] -= m * top[jj & 1][l];
+                if (r > jj) p[q][jj] = m * inv;  // L
+            }
         }
-        __syncthreads();
-        for (int r = jj + 1 + int(threadIdx.x); r < rows; r += blockDim.x) P[r * NB + jj] /= dj;
     }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < rows * NB; idx += blockDim.x) {
-        const int r = idx / NB, c = idx % NB;
-        if (c < nb && r > c) {
-            a[size_t(jb + r) * k + jb + c] = P[idx];
-            a[size_t(jb + c) * k + jb + r] = P[idx];
-        }
+#pragma unroll
+    for (int q = 0; q < RPT; q++) {
+        const int r = int(threadIdx.x) + 1024 * q;
+#pragma unroll
+        for (int c = 0; c < NB; c++)
+            if (r < rows && c < nb && r > c) {
+                a[size_t(jb + r) * k + jb + c] = p[q][c];
+                a[size_t(jb + c) * k + jb + r] = p[q][c];
+            }
     }
 }
 
-// Tile (ti, tl), tl <= ti, of the trailing lower triangle (rows and columns from jb + nb): a[i][l]
-// -= sum over the panel's columns p of L[i][p] d_p L[l][p], for l <= i.
+// The whole factor by one CTA for k up to LDLT_WHOLE, without a launch per panel: thread (x, y)
+// holds the elements (y + 16 p, x + 16 q) of what is left of the matrix in registers, the current
+// column passes through shared memory, one barrier and one reciprocal per column. After 16 columns
+// the finished block column is written out and the registers move up one block, so that one body
+// serves every column (a body per block column took 40 us at k = 110 with its code in the
+// instruction cache and 90 us without). 256 threads: with 1024 the FP64 pipe spends more on
+// reciprocals than on products (67 us). By panels 111 us, here 43 us.
+constexpr int LDLT_WHOLE = 160;
+template <int NR>  // k <= 16 NR
+__global__ void __launch_bounds__(256) k_ldlt_whole(double* __restrict__ a, double* __restrict__ d, int k) {
+    __shared__ double col[2][16 * NR], rec[16];
+    const int x = int(threadIdx.x % 16), y = int(threadIdx.x / 16);
+    double e[NR][NR];
+#pragma unroll
+    for (int p = 0; p < NR; p++)
+#pragma unroll
+        for (int q = 0; q <= p; q++) {
+            const int r = y + 16 * p, c = x + 16 * q;
+            e[p][q] = (r < k && c <= r) ? a[size_t(r) * k + c] : 0.0;
+        }
+    for (int b = 0; b < k; b += 16) {
+        const int n = k - b;  // rows left
+        for (int j = 0; j < min(16, n); j++) {
+            double* cj = col[j & 1];
+            if (x == j) {
+#pragma unroll
+                for (int p = 0; p < NR; p++) cj[y + 16 * p] = e[p][0];
+            }
+            __syncthreads();
+            double dj = cj[j];
+            if (dj <= PIVOT_TOL) dj = GROUND;
+            const double inv = 1.0 / dj;
+            if (threadIdx.x == 0) {
+                d[b + j] = dj;
+                rec[j] = inv;
+            }
+            // 0 in the finished columns and rows, which keep their values; no branch on the blocks
+            // left, which would serialize the loads
+            double f[NR], m[NR];
+#pragma unroll
+            for (int q = 0; q < NR; q++) {
+                f[q] = cj[x + 16 * q] * inv;
+                m[q] = cj[y + 16 * q];
+            }
+            if (x <= j) f[0] = 0.0;
+            if (y <= j) m[0] = 0.0;
+#pragma unroll
+            for (int p = 0; p < NR; p++)
+#pragma unroll
+                for (int q = 0; q <= p; q++) e[p][q] -= m[p] * f[q];
+        }
+        __syncthreads();
+        const double ri = rec[x];
+#pragma unroll
+        for (int p = 0; p < NR; p++) {
+            const int r = y + 16 * p;
+            if (r < n && r > x && x < n) a[size_t(b + r) * k + b + x] = a[size_t(b + x) * k + b + r] = e[p][0] * ri;
+        }
+        __syncthreads();  // rec is written again
+#pragma unroll
+        for (int p = 0; p + 1 < NR; p++)
+#pragma unroll
+            for (int q = 0; q <= p; q++) e[p][q] = e[p + 1][q + 1];
+#pragma unroll
+        for (int q = 0; q < NR; q++) e[NR - 1][q] = 0.0;
+    }
+}
+
 template <int NB>
 __global__ void __launch_bounds__(256) k_ldlt_trail(double* __restrict__ a, const double* __restrict__ d, int k, int jb,
                                                     int nb) {
@@ -337,10 +426,89 @@ __global__ void __launch_bounds__(256) k_ldlt_trail(double* __restrict__ a, cons
     }
 }
 
-// X = L^-T D^-1 L^-1, one warp per column of X (8 per block), the column held in shared memory:
+// X = L^-T D^-1 L^-1 for k up to 32 NR, one warp per NC columns of X, the columns in registers (lane
+// l holds the rows l, l + 32, ...). Column-oriented: once v[p] is final every lane subtracts its
+// rows' multiples of it, so a step costs one shuffle and one product on the chain, and the rows of
+// L of the next U steps are in flight meanwhile. What bounds it is that chain (small k) and the
+// matrix's passes through L2, which NC = 2 halves (large k). Against the row-oriented form with a
+// warp-wide sum per row: k = 110 114 -> 17 us, k = 310 422 -> 102 us, k = 910 2039 -> 576 us.
+template <int NR, int NC>
+__global__ void __launch_bounds__(128) k_ldlt_inverse(const double* __restrict__ a, const double* __restrict__ d, int k,
+                                                      double* __restrict__ x) {
+    constexpr int U = NR >= 32 ? 1 : NR >= 16 ? 2 : 8;
+    const int lane = int(threadIdx.x % 32);
+    const int col = (int(blockIdx.x) * 4 + int(threadIdx.x / 32)) * NC;
+    if (col >= k) return;  // whole warps
+    double v[NC][NR];
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int r = 0; r < NR; r++) v[c][r] = lane + 32 * r == col + c ? 1.0 : 0.0;
+    // forward: v[i] -= L[i][p] v[p], i > p (row p of the upper triangle is L's column p)
+#pragma unroll
+    for (int q = 0; q < NR; q++) {
+        if (32 * q + 31 < col || 32 * q >= k) continue;
+        for (int l0 = 0; l0 < 32; l0 += U) {
+            double row[U][NR];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int r = q; r < NR; r++) {
+                    const int p = 32 * q + l0 + u, i = lane + 32 * r;
+                    row[u][r] = (p < i && i < k) ? a[size_t(p) * k + i] : 0.0;
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    const double vp = __shfl_sync(FULL, v[c][q], l0 + u);
+#pragma unroll
+                    for (int r = q; r < NR; r++) v[c][r] -= row[u][r] * vp;
+                }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+        if (lane + 32 * r < k) {
+            const double dr = d[lane + 32 * r];
+#pragma unroll
+            for (int c = 0; c < NC; c++) v[c][r] /= dr;
+        }
+    // backward: v[i] -= L[p][i] v[p], i < p (row p of the lower triangle)
+#pragma unroll
+    for (int q = NR - 1; q >= 0; q--) {
+        if (32 * q >= k) continue;
+        for (int l0 = 32 - U; l0 >= 0; l0 -= U) {
+            double row[U][NR];
+#pragma unroll
+            for (int u = U - 1; u >= 0; u--)
+#pragma unroll
+                for (int r = 0; r <= q; r++) {
+                    const int p = 32 * q + l0 + u, i = lane + 32 * r;
+                    row[u][r] = (p < k && i < p) ? a[size_t(p) * k + i] : 0.0;
+                }
+#pragma unroll
+            for (int u = U - 1; u >= 0; u--)
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    const double vp = __shfl_sync(FULL, v[c][q], l0 + u);
+#pragma unroll
+                    for (int r = 0; r <= q; r++) v[c][r] -= row[u][r] * vp;
+                }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+            if (lane + 32 * r < k && col + c < k) x[size_t(lane + 32 * r) * k + col + c] = v[c][r];
+}
+
+// The same past 1024 rows, where the registers do not hold a column: one warp per column of X (8 per
+// block), the column held in shared memory:
 // forward over L's rows (strict lower part), the pivots, backward over L^T's rows (strict upper
 // part), each step a warp-wide dot product combined by a fixed butterfly.
-__global__ void __launch_bounds__(256) k_ldlt_inverse(const double* __restrict__ a, const double* __restrict__ d, int k,
+__global__ void __launch_bounds__(256) k_ldlt_inverse_wide(const double* __restrict__ a, const double* __restrict__ d, int k,
                                                       double* __restrict__ x) {
     extern __shared__ double xs[];
     const int w = int(threadIdx.x / 32), lane = int(threadIdx.x % 32);

@@ -165,21 +165,42 @@ __global__ void k_coord_combine(const u32* __restrict__ list_chunk_off, u32 m, c
 }
 
 // Dense small super-block S_SS (ms x ms, the first ms coordinates, ns small blocks) for the current
-// cell weights, on the device (operator.rs:1457-1523, as the host assembly of the dense factor):
+// cell weights (operator.rs:1457-1523, as the host assembly of the dense factor):
 //   S_SS[k][l] = sum_c W_c [k in c][l in c] - sum_s c_{s,k} c_{s,l} / n1_s,
-// by rows: one warp per work item (row k, a run of k's coordinate-list entries that never splits a segment),
-// accumulating the item's dense partial row in shared memory. Per entry (cell c of segment s):
-// S[k][l] += W_c for the small codes l of c; once per segment of the run, with
-// c_{s,k} = sum over the segment's cells and small blocks of W [code == k] (a warp sum in fixed
-// order), S[k][l] -= c_{s,k} W_c' / n1_s for the small codes l of every cell c' of s. Lane 0
-// applies the updates in entry and cell order, so the row does not depend on timing;
-// k_small_rows_sum adds a row's items in item order.
-__global__ void __launch_bounds__(256) k_small_rows(const u32* __restrict__ seg_off, const u32* __restrict__ coord,
-                                                    u32 M, int ns, u32 ms, const double* __restrict__ cw,
-                                                    const double* __restrict__ n1inv, const u32* __restrict__ pl_cell,
-                                                    const u32* __restrict__ pl_seg, const u32* __restrict__ item_k,
-                                                    const u32* __restrict__ item_a, const u32* __restrict__ item_b,
-                                                    u32 nitems, double* __restrict__ part) {
+// c_{s,k} the weight of the cells of segment s that hold k. The first sum's diagonal is nr_k, the
+// rest of it is nonzero between different small blocks only (k_small_cross). The second sum is a
+// Gram matrix over the segments, formed as one (k_small_gram) where the segments times the tiles of
+// the matrix do not pass the cells times ns, and by walking the few pairs that a segment's cells
+// have (k_small_rows) beyond: a tile costs about 0.6 ns a segment, a cell's code about 1 ns. Measured
+// with 10 cells a segment, both sums: 1e6 segments and 10 coordinates 0.16 ms (7.5 ms by lists, a
+// lane at a time, before), 1e6 and 110 2.2 ms (20.0), 2e4 and 310 0.20 ms by tiles and 0.31 by
+// lists, 2e5 and 910 4.2 ms by lists (6.4), where the 120 tiles would take 14. Every sum has a fixed
+// order.
+//
+// Partial row k of the first sum by work items (row k, a run of its list's entries): a warp takes
+// 32 entries at a time, the lanes that meet in a code are added in lane order by the first of
+// them, and that lane adds the sum to the item's row in shared memory. What bounds it is the
+// latency of the gathers of the cells' codes, which some thousand items hide.
+__device__ __forceinline__ void add_by_code(double* row, u32 code, double w, bool on, u32 lane) {
+    const unsigned same = __match_any_sync(FULL, on ? code : 0x80000000u + lane);
+    unsigned rest = same & ~((2u << lane) - 1u);  // the lanes after this one with its code
+    if ((same & ((1u << lane) - 1u)) != 0) rest = 0;  // a lane before this one adds
+    double sum = w;
+    for (unsigned any = __ballot_sync(FULL, rest != 0); any; any = __ballot_sync(FULL, rest != 0)) {
+        const int src = rest ? __ffs(int(rest)) - 1 : int(lane);
+        const double v = __shfl_sync(FULL, w, src);
+        if (rest) sum += v;
+        rest &= rest - 1;
+    }
+    if (on && (same & ((1u << lane) - 1u)) == 0) row[code] += sum;
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(256) k_small_cross(const u32* __restrict__ coord, u32 M, int ns, u32 ms,
+                                                     const double* __restrict__ cw, const u32* __restrict__ pl_cell,
+                                                     const u32* __restrict__ item_k, const u32* __restrict__ item_a,
+                                                     const u32* __restrict__ item_b, u32 nitems,
+                                                     double* __restrict__ part) {
     extern __shared__ double rows_s[];
     const u32 w = threadIdx.x / 32, lane = threadIdx.x % 32;
     const u32 it = blockIdx.x * 8 + w;
@@ -187,48 +208,168 @@ __global__ void __launch_bounds__(256) k_small_rows(const u32* __restrict__ seg_
     double* row = rows_s + size_t(w) * ms;
     for (u32 l = lane; l < ms; l += 32) row[l] = 0.0;
     __syncwarp();
-    const u32 k = item_k[it];
-    u32 prev = 0xffffffffu;
-    for (u32 e = item_a[it]; e < item_b[it]; e++) {
-        const u32 c = pl_cell[e], s = pl_seg[e];
-        if (lane == 0) {
-            const double wc = cw ? cw[c] : 1.0;
-            for (int b = 0; b < ns; b++) row[coord[size_t(b) * M + c]] += wc;
+    const u32 k = item_k[it], b = item_b[it];
+    for (u32 base = item_a[it]; base < b; base += 32) {
+        const u32 e = base + lane;
+        const bool valid = e < b;
+        const u32 c = valid ? pl_cell[e] : 0u;
+        const double wc = valid ? (cw ? cw[c] : 1.0) : 0.0;
+        for (int q = 0; q < ns; q++) {
+            const u32 code = valid ? coord[size_t(q) * M + c] : k;
+            add_by_code(row, code, wc, code != k, lane);  // the diagonal is nr_k
         }
-        if (s != prev) {
-            prev = s;
-            const u32 c0 = seg_off[s], c1 = seg_off[s + 1];
-            double ck = 0.0;
-            for (u32 cc = c0 + lane; cc < c1; cc += 32) {
-                const double wc = cw ? cw[cc] : 1.0;
-                for (int b = 0; b < ns; b++)
-                    if (coord[size_t(b) * M + cc] == k) ck += wc;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o /= 2) ck += __shfl_xor_sync(FULL, ck, o);
-            const double f = ck * n1inv[s];
-            if (lane == 0)
-                for (u32 cc = c0; cc < c1; cc++) {
-                    const double v = f * (cw ? cw[cc] : 1.0);
-                    for (int b = 0; b < ns; b++) row[coord[size_t(b) * M + cc]] -= v;
-                }
-        }
-        __syncwarp();
     }
     for (u32 l = lane; l < ms; l += 32) part[size_t(it) * ms + l] = row[l];
 }
 
-// Row k of S_SS: the partial rows of k's items (first[k] .. first[k+1]) added in item order.
-__global__ void k_small_rows_sum(const double* __restrict__ part, const u32* __restrict__ first, u32 ms,
-                                 double* __restrict__ out) {
-    const u32 k = blockIdx.x;
-    for (u32 l = threadIdx.x; l < ms; l += blockDim.x) {
-        double v = 0.0;
-        for (u32 it = first[k]; it < first[k + 1]; it++) v += part[size_t(it) * ms + l];
-        out[size_t(k) * ms + l] = v;
+// The same items when the second sum is added here too: for every segment of the run (an entry
+// opens one where its segment differs from the list's entry before it), with c_{s,k} from the
+// segment's cells, S[k][l] -= c_{s,k} W_c' / n1_s for the small codes l of every cell c' of s.
+__global__ void __launch_bounds__(256) k_small_rows(const u32* __restrict__ seg_off, const u32* __restrict__ coord,
+                                                    u32 M, int ns, u32 ms, const double* __restrict__ cw,
+                                                    const double* __restrict__ n1inv, const u32* __restrict__ pl_off,
+                                                    const u32* __restrict__ pl_cell, const u32* __restrict__ pl_seg,
+                                                    const u32* __restrict__ item_k, const u32* __restrict__ item_a,
+                                                    const u32* __restrict__ item_b, u32 nitems,
+                                                    double* __restrict__ part) {
+    extern __shared__ double rows_s[];
+    const u32 w = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const u32 it = blockIdx.x * 8 + w;
+    if (it >= nitems) return;  // whole warps
+    double* row = rows_s + size_t(w) * ms;
+    for (u32 l = lane; l < ms; l += 32) row[l] = 0.0;
+    __syncwarp();
+    const u32 k = item_k[it], b = item_b[it], first = pl_off[k];
+    for (u32 base = item_a[it]; base < b; base += 32) {
+        const u32 e = base + lane;
+        const bool valid = e < b;
+        const u32 c = valid ? pl_cell[e] : 0u, s = valid ? pl_seg[e] : 0u;
+        const double wc = valid ? (cw ? cw[c] : 1.0) : 0.0;
+        for (int q = 0; q < ns; q++) {
+            const u32 code = valid ? coord[size_t(q) * M + c] : k;
+            add_by_code(row, code, wc, code != k, lane);
+        }
+        const bool opens = valid && (e == first || pl_seg[e - 1] != s);
+        const u32 c0 = opens ? seg_off[s] : 0u, c1 = opens ? seg_off[s + 1] : 0u;
+        const double ni = opens ? n1inv[s] : 0.0;
+        for (unsigned todo = __ballot_sync(FULL, opens); todo; todo &= todo - 1) {
+            const int src = __ffs(int(todo)) - 1;
+            const u32 a0 = __shfl_sync(FULL, c0, src), a1 = __shfl_sync(FULL, c1, src);
+            double ck = 0.0;
+            for (u32 cc = a0 + lane; cc < a1; cc += 32) {
+                const double v = cw ? cw[cc] : 1.0;
+                for (int q = 0; q < ns; q++)
+                    if (coord[size_t(q) * M + cc] == k) ck += v;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o /= 2) ck += __shfl_xor_sync(FULL, ck, o);
+            const double f = ck * __shfl_sync(FULL, ni, src);
+            for (u32 cb = a0; cb < a1; cb += 32) {
+                const u32 cc = cb + lane;
+                const bool on = cc < a1;
+                const double v = on ? -f * (cw ? cw[cc] : 1.0) : 0.0;
+                for (int q = 0; q < ns; q++) add_by_code(row, on ? coord[size_t(q) * M + cc] : 0u, v, on, lane);
+            }
+        }
     }
+    for (u32 l = lane; l < ms; l += 32) part[size_t(it) * ms + l] = row[l];
 }
 
+// The Gram matrix sum_s c_s c_s' / n1_s by tiles of BT x BT (tile (ti, tj), tj <= ti, in blockIdx.y;
+// blockIdx.x takes the segment chunks x, x + gridDim.x, ...): a chunk's rows c_s are summed into
+// shared memory, thread (segment, small block) walking the segment's cells in order (a block's
+// codes have their own columns, so no two threads share a slot), then every thread adds the
+// products of its PT x PT outputs, segments in order. part[(y gridDim.x + x) BT BT + r BT + c].
+template <int BT>
+struct SgTile {
+    static constexpr int TS = BT == 16 ? 64 : 32;   // segments per chunk
+    static constexpr int PT = BT / 16;              // outputs per thread and side (16 x 16 threads)
+    static constexpr int LD = BT + 1;
+};
+template <int BT>
+__global__ void __launch_bounds__(256) k_small_gram(const u32* __restrict__ seg_off, const u32* __restrict__ coord,
+                                                    u32 M, u32 g1, int ns, const double* __restrict__ cw,
+                                                    const double* __restrict__ n1inv, double* __restrict__ part) {
+    using T = SgTile<BT>;
+    __shared__ double Ci[T::TS * T::LD], Cj[T::TS * T::LD], ni[T::TS];
+    int ti = 0;
+    while ((ti + 1) * (ti + 2) / 2 <= int(blockIdx.y)) ti++;
+    const int tj = int(blockIdx.y) - ti * (ti + 1) / 2;
+    const u32 ki = u32(ti * BT), kj = u32(tj * BT);
+    const int tx = int(threadIdx.x % 16), ty = int(threadIdx.x / 16);
+    double acc[T::PT][T::PT] = {};
+    const double* B = ti == tj ? Ci : Cj;
+    for (u32 s0 = blockIdx.x * T::TS; s0 < g1; s0 += gridDim.x * T::TS) {
+        const u32 nseg = min(u32(T::TS), g1 - s0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < T::TS * T::LD; i += 256) {
+            Ci[i] = 0.0;
+            if (ti != tj) Cj[i] = 0.0;
+        }
+        if (threadIdx.x < T::TS) ni[threadIdx.x] = threadIdx.x < nseg ? n1inv[s0 + threadIdx.x] : 0.0;
+        __syncthreads();
+        for (u32 i = threadIdx.x; i < nseg * u32(ns); i += 256) {
+            const u32 sl = i % nseg, q = i / nseg;
+            const u32* cd = coord + size_t(q) * M;
+            const u32 c1 = seg_off[s0 + sl + 1];
+#pragma unroll 4
+            for (u32 c = seg_off[s0 + sl]; c < c1; c++) {
+                const u32 code = cd[c];
+                const double w = cw ? cw[c] : 1.0;
+                if (code - ki < u32(BT)) Ci[sl * T::LD + (code - ki)] += w;
+                if (ti != tj && code - kj < u32(BT)) Cj[sl * T::LD + (code - kj)] += w;
+            }
+        }
+        __syncthreads();
+        for (u32 sl = 0; sl < nseg; sl++) {
+            double x[T::PT], y[T::PT];
+            const double n = ni[sl];
+#pragma unroll
+            for (int r = 0; r < T::PT; r++) {
+                x[r] = Ci[sl * T::LD + ty + 16 * r] * n;
+                y[r] = B[sl * T::LD + tx + 16 * r];
+            }
+#pragma unroll
+            for (int r = 0; r < T::PT; r++)
+#pragma unroll
+                for (int c = 0; c < T::PT; c++) acc[r][c] += x[r] * y[c];
+        }
+    }
+    double* o = part + (size_t(blockIdx.y) * gridDim.x + blockIdx.x) * (BT * BT);
+#pragma unroll
+    for (int r = 0; r < T::PT; r++)
+#pragma unroll
+        for (int c = 0; c < T::PT; c++) o[(ty + 16 * r) * BT + tx + 16 * c] = acc[r][c];
+}
+
+// S_SS[k][l] from nr, the items' partial rows (row k: items first[k] .. first[k+1], in order; null:
+// none) and, when gram is set, the tiles of k_small_gram (nsplit partials each): a warp per
+// element of the lower triangle, lane i adding the partials i, i + 32, ... and a fixed butterfly;
+// the upper triangle is its mirror.
+template <int BT>
+__global__ void k_small_combine(const double* __restrict__ items, const u32* __restrict__ first,
+                                const double* __restrict__ gram, u32 nsplit, const double* __restrict__ nr, u32 ms,
+                                double* __restrict__ out) {
+    const u32 lane = threadIdx.x & 31u;
+    const size_t gw = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, nw = (size_t(gridDim.x) * blockDim.x) >> 5;
+    for (size_t e = gw; e < size_t(ms) * ms; e += nw) {
+        const u32 k = u32(e / ms), l = u32(e % ms);
+        if (l > k) continue;
+        double v = 0.0, g = 0.0;
+        if (items)
+            for (u32 it = first[k] + lane; it < first[k + 1]; it += 32) v += items[size_t(it) * ms + l];
+        if (gram) {
+            const u32 ti = k / BT, tj = l / BT;
+            const double* t = gram + size_t(ti * (ti + 1) / 2 + tj) * nsplit * (BT * BT) + (k % BT) * BT + l % BT;
+            for (u32 x = lane; x < nsplit; x += 32) g += t[size_t(x) * (BT * BT)];
+        }
+        v -= g;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+        if (k == l) v += nr[k];
+        if (lane == 0) out[size_t(k) * ms + l] = out[size_t(l) * ms + k] = v;
+    }
+}
 
 // ak (k x k) = the kept rows / columns of a (ms x ms), scaled to unit diagonal.
 __global__ void k_small_gather(const double* __restrict__ a, u32 ms, const u32* __restrict__ keep,
