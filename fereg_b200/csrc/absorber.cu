@@ -32,6 +32,8 @@ constexpr int THREADS = TB;
 constexpr int GRID_T = 148 * 6;  // tile kernels: up to 6 resident CTAs per SM
 constexpr int GRID_V = 148 * 2;  // vector kernels with per-CTA partials
 constexpr int GRID_S = 148 * 4;  // warp-tile kernels (CTAs of WPB warps)
+// CTAs of the dense small rows' product over m coordinates (k_srow_apply).
+inline u32 small_row_ctas(u32 m) { return std::max<u32>(1, std::min<u32>(4 * GRID_V, (m + 31) / 32)); }
 constexpr size_t SMALL_STAGE_MAX = 16 * 1024;  // shared memory for the staged small rows of a chunk
 constexpr u32 VSEG_MAX = 256;  // longest segment (cells) a lane group walks in the operator's segment pass
 constexpr double REDUNDANT = 1e-12;  // operator.rs:21
@@ -44,7 +46,7 @@ constexpr size_t DENSE_SMALL_MAX = 1024;
 constexpr double REFINE_DROP = 1e-9;
 constexpr int REFINE_ROUNDS = 30;
 
-void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st, u64& launches);
+void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st, u64& launches, bool keep_order = false);
 template <class K>
 void allow_smem(K kernel, size_t bytes);
 
@@ -213,7 +215,7 @@ struct Scratch {
     DBuf<double> rows, rhs, b1, coefs, r, z, p, q, t, part, cta, cta2, colsum, along, small;
     DBuf<double> rhsv, xv;  // the padded right-hand side and iterate of the PCG
     // inner FP32 buffers of the refined solve
-    DBuf<float> fx, fb, fr, fz, fp, fq, ft, fpart, frhs, fx0, fsmall;
+    DBuf<float> fx, fb, fr, fz, fp, fq, ft, fpart, frhs, fx0;
     DBuf<double> cg_rho, cg_rho_new, cg_pq, cg_gamma, cg_beta, cg_xb, cg_ss1, cg_floor, cg_ring, cg_xconst, cg_pfloor;
     DBuf<int> cg_active, cg_nactive;
     DBuf<double> cg_ss0;
@@ -225,14 +227,16 @@ struct Scratch {
     DBuf<int> lp_ctl, lp_act;
     DBuf<double> lp_tol;
     DBuf<unsigned> lp_ticket;
+    DBuf<double> vpart;  // the vector kernels' per-CTA partials
     DBuf<double> lp_rho_from, lp_rho_at;
     struct PcgGraph {
         std::vector<u64> key;
         cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
-        u64 body_launches = 0;  // kernels of one body
+        u64 body_launches = 0;  // kernels of one iteration
     };
     std::vector<PcgGraph> graphs;
+    std::vector<std::vector<u64>> seen;  // keys of the bodies run by launches so far (the latest few)
     // grids of the S*P passes chosen by the autotuner, per (padded width, element size)
     struct ApplyGrids {
         int seg = 148 * 4, pull = 148 * 4;
@@ -283,6 +287,24 @@ struct Scratch {
         return CgState{cg_rho.p, cg_rho_new.p, cg_pq.p,   cg_gamma.p,  cg_beta.p,   cg_xb.p,     cg_ss1.p,
                        cg_floor.p, cg_ring.p, cg_xconst.p, cg_pfloor.p, cg_active.p, cg_nactive.p};
     }
+    // The PCG loop's device state for R columns; the buffers of the vector kernels.
+    void loop_alloc(u32 m, int R, cudaStream_t st) {
+        lp_ctl.alloc(8);
+        const size_t nt = 3 * VTICKETS * size_t(vec_tiles(R)) + 2;
+        if (nt > lp_ticket.n) {
+            lp_ticket.alloc(nt);
+            CK(cudaMemsetAsync(lp_ticket.p, 0, nt * sizeof(unsigned), st));  // every kernel leaves its counters at 0
+        }
+        lp_rho_from.alloc(size_t(R));
+        lp_rho_at.alloc(size_t(R));
+        lp_act.alloc(size_t(R));
+        lp_tol.alloc(1);
+        // the wide kernels' partials, or the narrow ones' and the small rows' (at most 1184 CTAs)
+        const size_t wide = size_t(std::max(296, vec_tiles(R))) * (4 * (SACC_MAX / 4) + 1) * VT;
+        vpart.alloc(std::max({wide, size_t(VEC_GRID) * 3 * std::min(R, WIDE_R),
+                              size_t(small_row_ctas(m)) * ms_acc * std::min(R, WIDE_R)}));
+    }
+    CgLoop loop() const { return CgLoop{lp_ctl.p, lp_ctl.p + 4, nullptr, lp_tol.p, lp_ticket.p, lp_rho_from.p, lp_rho_at.p, lp_act.p}; }
     cudaEvent_t get_event() {
         if (!pool_.empty()) {
             cudaEvent_t e = pool_.back();
@@ -351,7 +373,7 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
     }
     AllocScope alloc_scope(stream_);
     d_ = std::make_unique<Scratch>();
-    CK(cudaHostAlloc(&d_->h_nactive, 8 * sizeof(int), cudaHostAllocDefault));
+    CK(cudaHostAlloc(&d_->h_nactive, 16 * sizeof(int), cudaHostAllocDefault));
     // the cell structure and coordinate lists, built on the device from device codes
     std::vector<u32> pl_off, pl_seg;
     {
@@ -428,16 +450,20 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
             d_->cw_list_off.upload(loff, stream_);
         }
         if (hs_.m_small > 0 && hs_.m_small <= DENSE_SMALL_MAX) {
-            // runs of each small coordinate's entries, a few thousand in all, a warp each
+            // runs of each small coordinate's entries, a few thousand in all, a warp each; with one
+            // small block (k_small_ordered) at least `run` long, never splitting a segment
             const u32 es = pl_off[hs_.m_small];
-            const u32 run = std::max<u32>(128, (es / 4096 + 31) / 32 * 32);
+            const bool one = small_ordered();
+            const u32 run = one ? std::max<u32>(256, es / 4096) : std::max<u32>(128, (es / 4096 + 31) / 32 * 32);
             std::vector<u32> ik, ia, ib, first(hs_.m_small + 1, 0);
             for (u32 k = 0; k < u32(hs_.m_small); k++) {
                 first[k] = u32(ik.size());
-                for (u32 a = pl_off[k]; a < pl_off[k + 1]; a += run) {
+                for (u32 a = pl_off[k], b; a < pl_off[k + 1]; a = b) {
+                    b = std::min(pl_off[k + 1], a + run);
+                    while (one && b < pl_off[k + 1] && pl_seg[b] == pl_seg[b - 1]) b++;
                     ik.push_back(k);
                     ia.push_back(a);
-                    ib.push_back(std::min(pl_off[k + 1], a + run));
+                    ib.push_back(b);
                 }
             }
             first[hs_.m_small] = u32(ik.size());
@@ -666,7 +692,7 @@ void GpuAbsorber::build_amg() {
             dx.alloc(k * k);
             dscale.upload(scale, stream_);
             dkeep.upload(keep, stream_);
-            dense_ldlt_inverse(da.p, dd.p, int(k), dx.p, stream_, d_->launches);
+            dense_ldlt_inverse(da.p, dd.p, int(k), dx.p, stream_, d_->launches, true);
             k_expand_minv<<<grid_for(k * k), THREADS, 0, stream_>>>(dx.p, dkeep.p, dscale.p, int(k), nL, A.minv.p);
             CK(cudaGetLastError());
             d_->launches++;
@@ -844,6 +870,14 @@ void GpuAbsorber::ensure_precond() {
     pre_fresh_ = true;
 }
 
+// One small block of at most 32 coordinates on cells of one row: its assembly without weights keeps
+// the order of its sums (k_small_ordered).
+bool GpuAbsorber::small_ordered() const {
+    int ns = 0;
+    for (auto& b : hs_.blocks) ns += b.small;
+    return ns == 1 && hs_.m_small <= 32 && hs_.trivial();
+}
+
 // The dense small factor from the device assembly of S_SS (weights.cuh) for the device weight
 // state: as a Gram matrix over the segments, or by the lists' entries where that is less work.
 void GpuAbsorber::build_small_device() {
@@ -856,12 +890,21 @@ void GpuAbsorber::build_small_device() {
     DBuf<double> part, gpart, a, ak, dd, dx, dscale;
     DBuf<u32> dkeep;
     a.alloc(len);
+    const bool ordered = small_ordered() && !d.cell_w.p;
     const size_t T = (ms + (ms <= 16 ? 15 : 63)) / (ms <= 16 ? 16 : 64), tiles = T * (T + 1) / 2;
-    const bool gram = tiles * st.g1 <= M * size_t(ns);  // see k_small_gram
+    const bool gram = !ordered && tiles * st.g1 <= M * size_t(ns);  // see k_small_gram
     const size_t shm = size_t(8) * ms * sizeof(double);
     const u32 ni = d.sr_n;
     if (ni > 0 && (ns > 1 || !gram)) part.alloc(size_t(ni) * ms);
-    if (part.p && gram) {
+    if (ordered && ni > 0) {
+        DBuf<double> csk;
+        csk.alloc(size_t(st.g1) * ms);
+        k_seg_small_w<<<grid_for(size_t(st.g1) * ms), THREADS, 0, stream_>>>(d.seg_off.p, d.coord.p, u32(M), st.g1, ns,
+                                                                             u32(ms), nullptr, csk.p);
+        k_small_ordered<<<(ni + 7) / 8, 256, 0, stream_>>>(u32(ms), d.n1inv.p, csk.p, d.pl_seg.p, d.sr_k.p, d.sr_a.p,
+                                                           d.sr_b.p, ni, part.p);
+        k_small_items_sum<<<u32(ms * ms + 63) / 64, 64, 0, stream_>>>(part.p, d.sr_first.p, u32(ms), a.p);
+    } else if (part.p && gram) {
         allow_smem(k_small_cross, shm);
         k_small_cross<<<(ni + 7) / 8, 256, shm, stream_>>>(d.coord.p, u32(M), ns, u32(ms), d.cell_w.p, d.pl_cell.p,
                                                            d.sr_k.p, d.sr_a.p, d.sr_b.p, ni, part.p);
@@ -883,7 +926,8 @@ void GpuAbsorber::build_small_device() {
         k_small_combine<BT><<<grid_for(len * 32), THREADS, 0, stream_>>>(part.p, d.sr_first.p, gpart.p, nsplit,
                                                                          d.nr.p, u32(ms), a.p);
     };
-    if (ms <= 16) assemble(std::integral_constant<int, 16>{});
+    if (ordered && ni > 0) {
+    } else if (ms <= 16) assemble(std::integral_constant<int, 16>{});
     else assemble(std::integral_constant<int, 64>{});
     d.launches += 1 + (part.p != nullptr) + gram;
     // kept coordinates (not redundant, positive diagonal) and their unit-diagonal scaling
@@ -929,15 +973,25 @@ void allow_smem(K kernel, size_t bytes) {
 }
 
 // Grounded LDL^T of the k x k row-major `a` (lower triangle read, overwritten) and its inverse
-// into x (k x k), on `st`: panels of NB columns (16 up to k = 1024, 8 beyond, so that a panel of
-// k rows fits the shared memory of one CTA), each followed by its trailing update.
-void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st, u64& launches) {
+// into x (k x k), on `st`: by one CTA up to LDLT_WHOLE rows, else by panels of NB columns (16 up to
+// k = 1024, 8 beyond), each followed by its trailing update; the inverse by columns in registers up
+// to 1024 rows. keep_order (a hierarchy's coarsest level; blocks of at most 16 rows, where the
+// launches are all there is to gain) takes the elementwise divisions and row sums instead: on the
+// ill-conditioned graphs that reach a hierarchy the last bits of the preconditioner decide the
+// answer's eighth digit, and the same graph should give the same answer on every release.
+void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st, u64& launches, bool keep_order) {
     if (k <= 0) return;
+    keep_order = keep_order || k <= 16;
     auto factor = [&](auto nbc) {
         constexpr int NB = decltype(nbc)::value;
         for (int jb = 0; jb < k; jb += NB) {
             const int nb = std::min(NB, k - jb);
-            k_ldlt_panel<NB><<<1, 1024, 0, st>>>(a, d, k, jb);
+            if (keep_order) {
+                allow_smem(k_ldlt_panel_div<NB>, size_t(k) * NB * sizeof(double));
+                k_ldlt_panel_div<NB><<<1, 1024, size_t(k - jb) * NB * sizeof(double), st>>>(a, d, k, jb);
+            } else {
+                k_ldlt_panel<NB><<<1, 1024, 0, st>>>(a, d, k, jb);
+            }
             launches++;
             const int T = (k - jb - nb + 31) / 32;  // trailing tiles per side
             if (T > 0) {
@@ -946,7 +1000,7 @@ void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st,
             }
         }
     };
-    if (k <= LDLT_WHOLE) {
+    if (k <= LDLT_WHOLE && !keep_order) {
         if (k <= 32) k_ldlt_whole<2><<<1, 256, 0, st>>>(a, d, k);
         else if (k <= 64) k_ldlt_whole<4><<<1, 256, 0, st>>>(a, d, k);
         else if (k <= 112) k_ldlt_whole<7><<<1, 256, 0, st>>>(a, d, k);
@@ -963,14 +1017,13 @@ void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st,
     };
     using std::integral_constant;
     const integral_constant<int, 1> one;
-    if (k <= 32) inverse(one, one);
+    if (keep_order || k > 1024) {
+        allow_smem(k_ldlt_inverse_rows, size_t(8) * k * sizeof(double));
+        k_ldlt_inverse_rows<<<(k + 7) / 8, 256, size_t(8) * k * sizeof(double), st>>>(a, d, k, x);
+    } else if (k <= 32) inverse(one, one);
     else if (k <= 128) inverse(integral_constant<int, 4>{}, one);
     else if (k <= 512) inverse(integral_constant<int, 16>{}, one);
-    else if (k <= 1024) inverse(integral_constant<int, 32>{}, integral_constant<int, 2>{});
-    else {
-        allow_smem(k_ldlt_inverse_wide, size_t(8) * k * sizeof(double));
-        k_ldlt_inverse_wide<<<(k + 7) / 8, 256, size_t(8) * k * sizeof(double), st>>>(a, d, k, x);
-    }
+    else inverse(integral_constant<int, 32>{}, integral_constant<int, 2>{});
     launches++;
     CK(cudaGetLastError());
 }
@@ -989,14 +1042,52 @@ void launch_small_reduce(Scratch& d, const DevStruct& S, T* small, int R, T* Y, 
     d.launches++;
 }
 
+// k_wide_pq on the m x R vectors p and q with ms small coordinates (0: p'q alone).
+template <class T, bool DOT>
+void launch_wide_pq(Scratch& d, u32 ms, const T* p, T* q, u32 m, int R, const CgState& cg, const CgLoop& lp,
+                    cudaStream_t st) {
+    if (ms > 0 && !d.srow_on) throw Error(RC_INTERNAL, "fereg: the dense small rows are missing");
+    auto go = [&](auto kq) {
+        constexpr int KQ = decltype(kq)::value;
+        const dim3 grid(vec_splits(m, R, std::max(1, KQ)), vec_tiles(R));
+        k_wide_pq<T, KQ, DOT><<<grid, THREADS, 0, st>>>(d.srow.p, ms, p, q, m, R, d.vpart.p, cg, lp);
+    };
+    using std::integral_constant;
+    switch ((ms + 3) / 4) {
+        case 0: go(integral_constant<int, 0>{}); break;
+        case 1: go(integral_constant<int, 1>{}); break;
+        case 2: go(integral_constant<int, 2>{}); break;
+        case 3: go(integral_constant<int, 3>{}); break;
+        default: go(integral_constant<int, 4>{}); break;
+    }
+    d.launches++;
+}
+
+// The small coordinates' rows of Y = S P from the dense rows of S.
+template <class T>
+void launch_small_rows(Scratch& d, const DevStruct& S, const T* P, int Rv, T* Y, cudaStream_t st) {
+    if (!d.srow_on) throw Error(RC_INTERNAL, "fereg: the dense small rows are missing");
+    if (Rv > WIDE_R) {
+        launch_wide_pq<T, false>(d, S.ms_acc, P, Y, S.m, Rv, CgState{}, d.loop(), st);
+        return;
+    }
+    const u32 len = S.ms_acc * u32(Rv);
+    const u32 grid = small_row_ctas(S.m);
+    T* part = reinterpret_cast<T*>(d.vpart.p);
+    k_srow_apply<T><<<grid, THREADS, 0, st>>>(d.srow.p, S.m, S.ms_acc, P, Rv, part, S.halt);
+    k_small_reduce<T><<<std::max<u32>(1, std::min<u32>((len + 7) / 8, GRID_V)), THREADS, 0, st>>>(
+        part, int(grid), nullptr, 0, nullptr, 0, len, Y);
+    d.launches += 2;
+}
+
 // Y = S P on the PCG's padded vectors (Rv a multiple of 4). Short segments: one lane group per
 // segment (k_vseg_apply); long segments: CTA tiles, their slices' partials completed by k_fix.
 // Short coordinate lists: warp tiles (k_vpull_apply); long ones: CTA tiles and k_fix. The small
-// coordinates' rows (ms_acc > 0) come from the dense rows of S (k_srow_apply), their CTA
-// partials added by k_small_reduce.
+// coordinates' rows (ms_acc > 0) come from the dense rows of S: here, or, without small_rows_too,
+// from the caller's k_wide_pq.
 template <class T>
 void launch_apply(Scratch& d, const DevStruct& S, const DevWeights& W, const T* P, int Rv, T* Y, T* t, T* part,
-                  T* small, cudaStream_t st) {
+                  cudaStream_t st, bool small_rows_too = true) {
     if (Rv % 4 != 0) throw Error(RC_INTERNAL, "fereg: the operator takes padded vectors (a multiple of 4 columns)");
     const bool weighted = W.cell_w != nullptr;
     const auto gi = d.grids.find({Rv, int(sizeof(T))});
@@ -1059,15 +1150,7 @@ void launch_apply(Scratch& d, const DevStruct& S, const DevWeights& W, const T* 
             d.launches++;
         }
     }
-    if (S.ms_acc > 0) {
-        if (!d.srow_on) throw Error(RC_INTERNAL, "fereg: the dense small rows are missing");
-        const u32 len = S.ms_acc * u32(Rv);
-        const u32 grid = std::max<u32>(1, std::min<u32>(4 * GRID_V, (S.m + 31) / 32));
-        k_srow_apply<T><<<grid, THREADS, 0, st>>>(d.srow.p, S.m, S.ms_acc, P, Rv, small);
-        k_small_reduce<T><<<std::max<u32>(1, std::min<u32>((len + 7) / 8, GRID_V)), THREADS, 0, st>>>(
-            small, int(grid), nullptr, 0, nullptr, 0, len, Y);
-        d.launches += 2;
-    }
+    if (S.ms_acc > 0 && small_rows_too) launch_small_rows<T>(d, S, P, Rv, Y, st);
     CK(cudaGetLastError());
     d.end(h, st);
 }
@@ -1084,7 +1167,7 @@ std::mutex g_tune_mu;
 std::map<std::vector<u64>, Scratch::ApplyGrids> g_tuned;
 
 template <class T>
-void autotune_apply(Scratch& d, const DevStruct& S, const DevWeights& W, T* P, int Rv, T* Y, T* t, T* part, T* small,
+void autotune_apply(Scratch& d, const DevStruct& S, const DevWeights& W, T* P, int Rv, T* Y, T* t, T* part,
                     cudaStream_t st) {
     const std::pair<int, int> key{Rv, int(sizeof(T))};
     if (d.grids.count(key) || d.prof || S.M < (1u << 20)) return;
@@ -1113,7 +1196,7 @@ void autotune_apply(Scratch& d, const DevStruct& S, const DevWeights& W, T* P, i
         float mn = 1e30f;
         for (int rep = 0; rep < 3; rep++) {
             CK(cudaEventRecord(e0, st));
-            launch_apply<T>(d, S, W, P, Rv, Y, t, part, small, st);
+            launch_apply<T>(d, S, W, P, Rv, Y, t, part, st);
             CK(cudaEventRecord(e1, st));
             CK(cudaEventSynchronize(e1));
             float ms = 0;
@@ -1197,10 +1280,11 @@ void launch_amg(Scratch& d, DevAmgBlock& A, const T* r, T* z, int R, cudaStream_
 }
 
 template <class T>
-void launch_precond(Scratch& d, const DevStruct& S, bool small_ok, const T* r, T* z, int R, cudaStream_t st) {
+void launch_precond(Scratch& d, const DevStruct& S, bool small_ok, const T* r, T* z, int R, cudaStream_t st,
+                    bool jacobi = true) {
     const int h = d.begin(GpuAbsorber::P_PRECOND, st);
     const u32 ms = small_ok ? S.ms : 0;
-    if (S.m > ms) {
+    if (S.m > ms && jacobi) {
         k_jacobi<T><<<grid_for(size_t(S.m - ms) * R), THREADS, 0, st>>>(r, z, d.inv_diag.p, ms, S.m, R);
         d.launches++;
     }
@@ -1395,10 +1479,10 @@ void GpuAbsorber::apply_host(const double* p, size_t r, double* y) {
     d_->q.alloc(m * rv);
     d_->t.alloc(size_t(hs_.g1) * rv);
     d_->part.alloc(std::max<size_t>(1, size_t(std::max(S.seg.nparts, S.pull.nparts)) * rv));
-    d_->small.alloc(std::max<size_t>(1, small_rows() * d_->ms_acc * rv));
+    d_->loop_alloc(u32(m), int(rv), stream_);
     CK(cudaMemsetAsync(d_->p.p, 0, m * rv * 8, stream_));
     CK(cudaMemcpy2DAsync(d_->p.p, rv * 8, p, r * 8, r * 8, m, cudaMemcpyHostToDevice, stream_));
-    launch_apply<double>(*d_, S, d_->dw(), d_->p.p, int(rv), d_->q.p, d_->t.p, d_->part.p, d_->small.p, stream_);
+    launch_apply<double>(*d_, S, d_->dw(), d_->p.p, int(rv), d_->q.p, d_->t.p, d_->part.p, stream_);
     CK(cudaMemcpy2DAsync(y, r * 8, d_->q.p, rv * 8, r * 8, m, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
     d_->collect();
@@ -1495,6 +1579,12 @@ constexpr double PROBE_RATIO = 0.6;
 // Iterations a graph launch may run at most before the host looks at the loop state again.
 constexpr int GRAPH_CAP = 64;
 
+// Iterations in the body of a captured graph: 19 us a turn of its WHILE node against 2 us for each
+// kernel of an iteration that finds the halt word set (1.5 iterations of 5 kernels on average).
+constexpr int BODY_ITERS = 4;
+// Iterations launched one by one between two looks at the loop state.
+constexpr int FIRST_BATCH = 6;
+
 // The operator of a PCG run on the intercept-only structure: q = S p (launch_apply) and
 // z = M^-1 r (launch_precond), with the device addresses their launches touch.
 template <class T>
@@ -1503,14 +1593,34 @@ struct FeOp {
     const DevStruct& S;
     const DevWeights& W;
     bool small_ok;
-    T *t, *part, *small;
+    T *t, *part;
     u32 m() const { return S.m; }
-    void apply(T* p, int R, T* q, cudaStream_t st) const { launch_apply<T>(d, S, W, p, R, q, t, part, small, st); }
+    void apply(T* p, int R, T* q, cudaStream_t st) const { launch_apply<T>(d, S, W, p, R, q, t, part, st); }
+    // the operator in the loop: with the tiled vector steps without the small coordinates' rows,
+    // which k_wide_pq forms (ms_acc of them)
+    void apply_rest(T* p, int R, T* q, const int* halt, cudaStream_t st) const {
+        DevStruct H = S;
+        H.halt = halt;
+        launch_apply<T>(d, H, W, p, R, q, t, part, st, !tiled(R));
+    }
+    // The vector steps by column tiles (k_wide_*): wide blocks, and weighted systems with a small
+    // preconditioner, where fewer kernels pay (1.07e6 weighted rows, 8 columns, an iteration's vector
+    // kernels: 43 us by the narrow ones, 30). Unweighted ones keep the narrow kernels' order of sums.
+    bool tiled(int R) const { return R > WIDE_R || (W.cell_w && fused(R)); }
+    u32 ms_acc() const { return S.ms_acc; }
+    // iterations in a graph's body: a hierarchy's V-cycle does not look at the halt word
+    int unroll() const { return d.amg.empty() ? BODY_ITERS : 1; }
+    // the preconditioner inside k_wide_xr: Jacobi and a dense small block, no hierarchy
+    bool fused(int R) const { return d.amg.empty() && pre_fused(ms(), R); }
+    // its Jacobi part inside k_update_xr, the rest by precond_rest
+    static constexpr bool JACOBI = true;
+    u32 ms() const { return small_ok ? S.ms : 0; }
+    void precond_rest(T* r, T* z, int R, cudaStream_t st) const { launch_precond<T>(d, S, small_ok, r, z, R, st, false); }
     void precond(T* r, T* z, int R, cudaStream_t st) const { launch_precond<T>(d, S, small_ok, r, z, R, st); }
     void key(std::vector<u64>& k) const {
         auto put = [&](const void* ptr) { k.push_back(u64(reinterpret_cast<uintptr_t>(ptr))); };
         k.push_back(small_ok);
-        for (const void* ptr : {(const void*)t, (const void*)part, (const void*)small, (const void*)W.w_rows,
+        for (const void* ptr : {(const void*)t, (const void*)part, (const void*)W.w_rows,
                                 (const void*)W.cell_w, (const void*)W.n1inv, (const void*)W.nr, (const void*)d.inv_diag.p,
                                 (const void*)d.minv.p, (const void*)d.srow.p})
             put(ptr);
@@ -1541,7 +1651,7 @@ std::vector<u64> body_key(Scratch& d, const Op& op, const T* x, const T* rhs_tru
     for (const void* ptr : {(const void*)x, (const void*)rhs_true, (const void*)x0, (const void*)r, (const void*)z,
                             (const void*)p, (const void*)q})
         put(ptr);
-    for (const void* ptr : {(const void*)d.cta.p, (const void*)d.lp_ctl.p, (const void*)d.lp_ticket.p,
+    for (const void* ptr : {(const void*)d.vpart.p, (const void*)d.lp_ctl.p, (const void*)d.lp_ticket.p,
                             (const void*)d.cg_rho.p, (const void*)d.cg_active.p, (const void*)d.cg_ring.p,
                             (const void*)d.cg_xb.p, (const void*)d.cg_beta.p, (const void*)d.cg_gamma.p,
                             (const void*)d.cg_pfloor.p, (const void*)d.cg_xconst.p, (const void*)d.cg_floor.p,
@@ -1553,26 +1663,52 @@ std::vector<u64> body_key(Scratch& d, const Op& op, const T* x, const T* rhs_tru
     return k;
 }
 
-// The iteration body (cg.rs:207-290): q = S p, gamma, x and r (with the stopping rule's dot
-// products), z = M^-1 r, rho and the stopping rule, p. In a graph (use_cond) its last kernel sets
-// the WHILE condition.
+// rho = r'z with the stopping rule (START: the rho of a start).
+template <class T, bool START>
+void launch_rz(Scratch& d, const T* r, const T* z, u32 m, int R, bool tiled, const CgState& cg, const CgLoop& lp,
+               double drop, cudaStream_t st) {
+    if (tiled)
+        k_wide_rz<T, START><<<dim3(vec_splits(m, R, 1), vec_tiles(R)), THREADS, 0, st>>>(r, z, m, R, d.vpart.p, cg, lp,
+                                                                                         PROBE_FROM, PROBE_AT, drop);
+    else
+        k_rz_stop<T, START><<<VEC_GRID, THREADS, 0, st>>>(r, z, m, R, d.vpart.p, cg, lp, PROBE_FROM, PROBE_AT, drop);
+    d.launches++;
+}
+
+// The iteration body (cg.rs:207-290): q = S p, gamma, x and r (with the stopping rule's sums),
+// z = M^-1 r, rho and the stopping rule, p. In a graph (use_cond) its last kernel sets the WHILE
+// condition.
 template <class T, class Op>
 void enqueue_iteration(Scratch& d, const Op& op, T* x, const T* rhs_true, const T* x0, T* r, T* z, T* p, T* q, int R,
                        const CgState& cg, const CgLoop& lp, cudaGraphConditionalHandle cond, bool use_cond,
                        cudaStream_t st) {
     const u32 m = op.m();
-    const size_t tot = size_t(m) * R;
-    op.apply(p, R, q, st);
+    op.apply_rest(p, R, q, lp.halt, st);
     int h = d.begin(GpuAbsorber::P_VECTOR, st);
-    k_pq_gamma<T><<<GRID_V, THREADS, 0, st>>>(p, q, m, R, d.cta.p, cg, lp);
-    k_update_xr_sum<T><<<GRID_V, THREADS, 0, st>>>(x, r, p, q, rhs_true, x0, m, R, d.cta.p, cg, lp);
-    d.launches += 2;
-    d.end(h, st);
-    op.precond(r, z, R, st);
-    h = d.begin(GpuAbsorber::P_VECTOR, st);
-    k_rz_stop<T><<<GRID_V, THREADS, 0, st>>>(r, z, m, R, d.cta.p, cg, lp, PROBE_FROM, PROBE_AT);
-    k_update_p_cond<T><<<grid_for(tot), THREADS, 0, st>>>(p, z, cg.beta, cg.active, m, R, lp, cond, use_cond ? 1 : 0);
-    d.launches += 2;
+    const bool wide = op.tiled(R), fused = wide && op.fused(R);
+    const dim3 grid(vec_splits(m, R, 1), vec_tiles(R));
+    if (wide) launch_wide_pq<T, true>(d, op.ms_acc(), p, q, m, R, cg, lp, st);
+    else k_pq_gamma<T><<<VEC_GRID, THREADS, 0, st>>>(p, q, m, R, d.vpart.p, cg, lp);
+    if (fused)
+        k_wide_xr<T, true><<<grid, THREADS, 0, st>>>(x, r, p, q, rhs_true, x0, m, R, d.vpart.p, cg, lp, z,
+                                                     d.inv_diag.p, d.minv.p, op.ms(), PROBE_FROM, PROBE_AT);
+    else if (wide)
+        k_wide_xr<T, false><<<grid, THREADS, 0, st>>>(x, r, p, q, rhs_true, x0, m, R, d.vpart.p, cg, lp, nullptr,
+                                                      nullptr, nullptr, 0, PROBE_FROM, PROBE_AT);
+    else
+        k_update_xr<T, Op::JACOBI><<<VEC_GRID, THREADS, 0, st>>>(x, r, p, q, rhs_true, x0, m, R, d.vpart.p, cg, lp, z,
+                                                                 d.inv_diag.p, op.ms());
+    d.launches += wide ? 1 : 2;
+    if (!fused) {
+        d.end(h, st);
+        if (wide) op.precond(r, z, R, st);
+        else op.precond_rest(r, z, R, st);
+        h = d.begin(GpuAbsorber::P_VECTOR, st);
+        launch_rz<T, false>(d, r, z, m, R, wide, cg, lp, 0.0, st);
+    }
+    k_update_p<T, false><<<grid_for(size_t(m) * (R / 4)), THREADS, 0, st>>>(p, z, cg.beta, cg.active, m, R, lp, cond,
+                                                                            use_cond ? 1 : 0);
+    d.launches++;
     d.end(h, st);
     CK(cudaGetLastError());
 }
@@ -1592,7 +1728,7 @@ Scratch::PcgGraph capture_iteration(Scratch& d, const Op& op, T* x, const T* rhs
     // a first node sets the condition from the active count and the launch's cap, so that a launch
     // with no active column runs no iteration (the host need not look before launching)
     CK(cudaStreamBeginCaptureToGraph(st, gr.g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    k_cond_first<<<1, 32, 0, st>>>(cond, cg.n_active, lp);
+    k_loop_first<<<1, 32, 0, st>>>(cond, 1, cg.n_active, lp);
     CK(cudaStreamEndCapture(st, &gr.g));
     cudaGraphNode_t first = nullptr;
     size_t nn = 1;
@@ -1608,9 +1744,11 @@ Scratch::PcgGraph capture_iteration(Scratch& d, const Op& op, T* x, const T* rhs
     cudaGraph_t body = np.conditional.phGraph_out[0];
     const u64 launches0 = d.launches;
     CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    enqueue_iteration<T>(d, op, x, rhs_true, x0, r, z, p, q, R, cg, lp, cond, true, st);
+    const int U = op.unroll();
+    for (int u = 0; u < U; u++)
+        enqueue_iteration<T>(d, op, x, rhs_true, x0, r, z, p, q, R, cg, lp.at(u, U > 1), cond, u == U - 1, st);
     CK(cudaStreamEndCapture(st, &body));
-    gr.body_launches = d.launches - launches0;
+    gr.body_launches = (d.launches - launches0) / u64(op.unroll());
     d.launches = launches0;  // counted when the graph runs
     CK(cudaGraphInstantiate(&gr.exec, gr.g, 0));
     d.graph_captures++;
@@ -1638,20 +1776,14 @@ static u64 run_pcg(Scratch& d, const Op& op, T* x, const T* b, const T* rhs_true
                    cudaStream_t st, const std::function<bool(double)>& escalate) {
     const size_t m = op.m(), tot = m * size_t(R);
     CgState cg = d.cg();
-    d.lp_ctl.alloc(4);
-    d.lp_ticket.alloc(4);
-    d.lp_rho_from.alloc(size_t(R));
-    d.lp_rho_at.alloc(size_t(R));
-    d.lp_act.alloc(size_t(R));
-    d.lp_tol.alloc(1);
-    CK(cudaMemsetAsync(d.lp_ticket.p, 0, 4 * sizeof(unsigned), st));
-    std::memcpy(d.h_nactive + 6, &tol, sizeof(double));  // pinned words 6-7
-    CK(cudaMemcpyAsync(d.lp_tol.p, d.h_nactive + 6, sizeof(double), cudaMemcpyHostToDevice, st));
-    const CgLoop lp{d.lp_ctl.p, d.lp_tol.p, d.lp_ticket.p, d.lp_rho_from.p, d.lp_rho_at.p, d.lp_act.p};
+    d.loop_alloc(u32(m), R, st);
+    std::memcpy(d.h_nactive + 8, &tol, sizeof(double));  // pinned words 8-9
+    CK(cudaMemcpyAsync(d.lp_tol.p, d.h_nactive + 8, sizeof(double), cudaMemcpyHostToDevice, st));
+    const CgLoop lp = d.loop();
     u64 it = 0;
     std::vector<double> rho_from(R), rho_at(R);
     std::vector<int> act(R);
-    int* hc = d.h_nactive;  // pinned [n_active, k, k of the launch, cap]
+    int* hc = d.h_nactive;  // pinned: the control words read back, then (4, 5) those sent
 restart:
     if (x_is_start) {
         op.apply(x, R, q, st);
@@ -1662,28 +1794,22 @@ restart:
     }
     op.precond(r, z, R, st);
     int h = d.begin(GpuAbsorber::P_VECTOR, st);
-    k_dot<T><<<GRID_V, THREADS, 0, st>>>(r, z, u32(m), R, d.cta.p);
-    reduce_cols(d, d.cta.p, GRID_V, R, d.cg_rho.p, st);
-    k_cg_start<<<1, THREADS, 0, st>>>(cg, R, drop);
-    k_mask_copy<T><<<grid_for(tot), THREADS, 0, st>>>(p, z, d.cg_active.p, tot, R);
-    d.launches += 3;
-    CK(cudaMemsetAsync(d.lp_ctl.p, 0, 4 * sizeof(int), st));  // k = 0 since the (re)start
-    CK(cudaMemcpyAsync(hc, d.cg_nactive.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // rho, the active columns (k = 0 since the (re)start) and the first direction
+    launch_rz<T, true>(d, r, z, u32(m), R, op.tiled(R), cg, lp, drop, st);
+    k_update_p<T, true><<<grid_for(m * size_t(R / 4)), THREADS, 0, st>>>(p, z, cg.beta, d.cg_active.p, u32(m), R, lp, 0, 0);
+    d.launches++;
     d.end(h, st);
-    // with the body's graph captured already, the graph's first node decides whether the first
-    // launch runs an iteration: the host launches it without reading the active count first
-    bool look = d.prof || maxiter <= iters_done + it;
-    if (!look) {
-        op.prepare(R);
-        const std::vector<u64> key0 = body_key<T>(d, op, x, rhs_true, x0, r, z, p, q, R);
-        look = true;
-        for (auto& q_ : d.graphs)
-            if (q_.key == key0) look = false;
+    // the batch's first kernel decides whether an iteration runs: the host need not read the active
+    // count first, unless it may have to say that no iteration is left
+    bool any_active = true;
+    if (maxiter <= iters_done + it) {
+        CK(cudaMemcpyAsync(hc, d.cg_nactive.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        any_active = hc[0] > 0;
     }
-    if (look) CK(cudaStreamSynchronize(st));
-    bool any_active = look ? hc[0] > 0 : true;
     int k = 0;
     bool probed = false;
+    bool fresh = false;  // the body is new in this solve
     while (any_active) {
         ctx.check();
         // iterations this launch may run: up to the probe, the cap and maxiter
@@ -1701,23 +1827,35 @@ restart:
         hc[5] = int(cap);
         CK(cudaMemcpyAsync(d.lp_ctl.p + 2, hc + 4, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
         const Scratch::PcgGraph* gr = nullptr;
+        int batch = 1;
         if (!d.prof) {
             op.prepare(R);
             std::vector<u64> key = body_key<T>(d, op, x, rhs_true, x0, r, z, p, q, R);
             for (auto& q_ : d.graphs)
                 if (q_.key == key) gr = &q_;
-            if (!gr) {
-                // a new body: this batch runs one iteration by launches (first uses of its kernels
-                // set their attributes), and the body is captured for the next batches
-                enqueue_iteration<T>(d, op, x, rhs_true, x0, r, z, p, q, R, cg, lp, 0, false, st);
+            if (!gr && !fresh && std::find(d.seen.begin(), d.seen.end(), key) != d.seen.end()) {
+                // the body ran by launches in an earlier solve: this and later ones replay its graph
                 if (d.graphs.size() >= 8) d.drop_graphs();
                 d.graphs.push_back(capture_iteration<T>(d, op, x, rhs_true, x0, r, z, p, q, R, cg, lp, st, std::move(key)));
-            } else {
-                CK(cudaGraphLaunch(gr->exec, st));
-                d.graph_launches++;
+                gr = &d.graphs.back();
+            } else if (!gr) {
+                // a new body runs by launches, a few iterations between two looks at the loop state (a
+                // capture and its instantiation cost the first solve of a session 0.3 ms and more)
+                batch = int(std::min<long long>(cap, FIRST_BATCH));
+                if (!fresh) {
+                    if (d.seen.size() >= 8) d.seen.erase(d.seen.begin());
+                    d.seen.push_back(std::move(key));
+                    fresh = true;
+                }
             }
+        }
+        if (gr) {
+            CK(cudaGraphLaunch(gr->exec, st));
+            d.graph_launches++;
         } else {
-            enqueue_iteration<T>(d, op, x, rhs_true, x0, r, z, p, q, R, cg, lp, 0, false, st);
+            k_loop_first<<<1, 32, 0, st>>>(0, 0, cg.n_active, lp);
+            for (int u = 0; u < batch; u++)
+                enqueue_iteration<T>(d, op, x, rhs_true, x0, r, z, p, q, R, cg, lp.at(u, u + 1 < batch), 0, false, st);
         }
         CK(cudaMemcpyAsync(hc, d.lp_ctl.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaGetLastError());
@@ -1782,7 +1920,8 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
     d.colsum.alloc(3 * r);
     d.t.alloc(g1 * rv);
     d.cta2.alloc(size_t(GRID_S) * 2 * r);
-    d.small.alloc(std::max<size_t>(1, small_rows() * d.ms_acc * rv));
+    d.small.alloc(std::max<size_t>(1, small_rows() * d.ms_acc * r));
+    d.loop_alloc(u32(m), RV, st);
     launch_rhs(d, S, W, rows, R, d.b1.p, d.rhs.p, d.colsum.p, st);
     ctx_.check();
     // ss0 and ss1 (solve.rs:1210-1217) and the PCG's start state on the device from the column sums;
@@ -1849,11 +1988,11 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
         CK(cudaMemsetAsync(d.cg_ring.p, 0, rv * WINDOW * 8, st));
         const bool exact_pre = small_ok_ && hs_.m_small == hs_.m;
         const std::function<bool(double)> esc = [this](double rho_hat) { return escalate(rho_hat); };
-        const FeOp<double> op64{d, S, W, small_ok_, d.t.p, d.part.p, d.small.p};
+        const FeOp<double> op64{d, S, W, small_ok_, d.t.p, d.part.p};
         if (exact_pre) {
             // x* = x + M^-1 (rhs - S x) (cg.rs:171-198)
             if (warm || have_last) {
-                launch_apply<double>(d, S, W, x, RV, d.q.p, d.t.p, d.part.p, d.small.p, st);
+                launch_apply<double>(d, S, W, x, RV, d.q.p, d.t.p, d.part.p, st);
                 k_sub<double><<<grid_for(tot), THREADS, 0, st>>>(d.r.p, d.rhsv.p, d.q.p, tot);
                 d.launches++;
             } else {
@@ -1864,7 +2003,7 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
             d.launches++;
             CK(cudaGetLastError());
         } else if (prec == Precision::F64) {
-            if (ctx_.autotune) autotune_apply<double>(d, S, W, d.rhsv.p, RV, d.q.p, d.t.p, d.part.p, d.small.p, st);
+            if (ctx_.autotune) autotune_apply<double>(d, S, W, d.rhsv.p, RV, d.q.p, d.t.p, d.part.p, st);
             iterations = run_pcg<double>(d, op64, x, d.rhsv.p, d.rhsv.p, nullptr, d.r.p, d.z.p, d.p.p, d.q.p, RV, tol,
                                          0.0, 0, maxiter, warm != nullptr || have_last, ctx_, st, esc);
             exact = false;
@@ -1873,11 +2012,10 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
             for (auto* b : {&d.fx, &d.fb, &d.fr, &d.fz, &d.fp, &d.fq, &d.frhs, &d.fx0}) b->alloc(tot);
             d.ft.alloc(g1 * rv);
             d.fpart.alloc(nparts * rv);
-            d.fsmall.alloc(std::max<size_t>(1, small_rows() * d.ms_acc * rv));
             k_convert<double, float><<<grid_for(tot), THREADS, 0, st>>>(d.rhsv.p, d.frhs.p, tot);
             d.launches++;
-            if (ctx_.autotune) autotune_apply<float>(d, S, W, d.frhs.p, RV, d.fq.p, d.ft.p, d.fpart.p, d.fsmall.p, st);
-            if (ctx_.autotune) autotune_apply<double>(d, S, W, d.rhsv.p, RV, d.q.p, d.t.p, d.part.p, d.small.p, st);
+            if (ctx_.autotune) autotune_apply<float>(d, S, W, d.frhs.p, RV, d.fq.p, d.ft.p, d.fpart.p, st);
+            if (ctx_.autotune) autotune_apply<double>(d, S, W, d.rhsv.p, RV, d.q.p, d.t.p, d.part.p, st);
             iterations = 0;
             std::vector<double> rho64(rv, 0.0), rho_prev(rv, 0.0);
             bool have_r = false;  // d.r holds the FP64 true residual of x
@@ -1887,7 +2025,7 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
                 // true residual b = rhs - S x in FP64 (kept from the previous round's check), x'rhs,
                 // and the FP32 copies
                 if (!have_r && start_nonzero) {
-                    launch_apply<double>(d, S, W, x, RV, d.q.p, d.t.p, d.part.p, d.small.p, st);
+                    launch_apply<double>(d, S, W, x, RV, d.q.p, d.t.p, d.part.p, st);
                     k_sub<double><<<grid_for(tot), THREADS, 0, st>>>(d.r.p, d.rhsv.p, d.q.p, tot);
                     d.launches++;
                 } else if (!have_r) {
@@ -1900,13 +2038,13 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
                 CK(cudaMemsetAsync(d.fx.p, 0, tot * 4, st));
                 CK(cudaMemsetAsync(d.cg_ring.p, 0, rv * WINDOW * 8, st));
                 d.launches += 3;
-                const FeOp<float> op32{d, S, W, small_ok_, d.ft.p, d.fpart.p, d.fsmall.p};
+                const FeOp<float> op32{d, S, W, small_ok_, d.ft.p, d.fpart.p};
                 iterations += run_pcg<float>(d, op32, d.fx.p, d.fb.p, d.frhs.p, d.fx0.p, d.fr.p, d.fz.p, d.fp.p, d.fq.p,
                                              RV, tol, REFINE_DROP, iterations, maxiter, false, ctx_, st, esc);
                 k_add_correction<<<grid_for(tot), THREADS, 0, st>>>(x, d.fx.p, tot);
                 d.launches++;
                 // the round's check in FP64: true residual, its preconditioned norm and ss_k
-                launch_apply<double>(d, S, W, x, RV, d.q.p, d.t.p, d.part.p, d.small.p, st);
+                launch_apply<double>(d, S, W, x, RV, d.q.p, d.t.p, d.part.p, st);
                 k_sub<double><<<grid_for(tot), THREADS, 0, st>>>(d.r.p, d.rhsv.p, d.q.p, tot);
                 launch_precond<double>(d, S, small_ok_, d.r.p, d.z.p, RV, st);
                 k_dot<double><<<GRID_V, THREADS, 0, st>>>(d.r.p, d.z.p, u32(m), RV, d.cta.p);
@@ -2113,13 +2251,25 @@ struct VirtOp {
     DevOperator& o;
     u32 m() const { return o.m(); }
     void apply(double* p, int R, double* q, cudaStream_t st) const { o.apply(p, R, q, st); }
+    bool tiled(int R) const { return R > WIDE_R; }
+    void apply_rest(double* p, int R, double* q, const int* halt, cudaStream_t st) const {
+        o.halt = halt;
+        o.apply(p, R, q, st);
+        o.halt = nullptr;
+    }
+    int unroll() const { return BODY_ITERS; }
+    u32 ms_acc() const { return 0; }
+    bool fused(int) const { return false; }
+    static constexpr bool JACOBI = false;
+    u32 ms() const { return 0; }
+    void precond_rest(double* r, double* z, int R, cudaStream_t st) const { o.precond(r, z, R, st); }
     void precond(double* r, double* z, int R, cudaStream_t st) const { o.precond(r, z, R, st); }
     void key(std::vector<u64>& k) const { o.key(k); }
     void prepare(int) const {}
 };
 
 PcgDriver::PcgDriver() : d_(std::make_unique<Scratch>()) {
-    CK(cudaHostAlloc(&d_->h_nactive, 8 * sizeof(int), cudaHostAllocDefault));
+    CK(cudaHostAlloc(&d_->h_nactive, 16 * sizeof(int), cudaHostAllocDefault));
 }
 PcgDriver::~PcgDriver() = default;
 
@@ -2155,6 +2305,7 @@ u64 PcgDriver::run(DevOperator& op, double* x, const double* b, int R, const std
     CK(cudaMemsetAsync(d.cg_xconst.p, 0, rv * 8, st));
     CK(cudaMemsetAsync(d.cg_pfloor.p, 0, rv * 8, st));
     CK(cudaMemsetAsync(d.cg_ring.p, 0, rv * WINDOW * 8, st));
+    d.loop_alloc(u32(m), R, st);
     const VirtOp vo{op};
     const u64 it = run_pcg<double>(d, vo, x, b, b, nullptr, d.r.p, d.z.p, d.p.p, d.q.p, R, tol, 0.0, 0, maxiter,
                                    x_is_start, ctx, st, std::function<bool(double)>());

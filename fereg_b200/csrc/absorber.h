@@ -209,6 +209,7 @@ class GpuAbsorber : public DeviceAbsorber {
     void refresh_small();
     void refresh_coord() const;
     void build_small_device();
+    bool small_ordered() const;
 
     void unit_weights_device();
     void build_srow();

@@ -83,23 +83,6 @@ struct CgState {
 
 constexpr int WINDOW = 5;
 
-// After rho = r'z of a (re)start: columns with rho <= 0 stop (cg.rs:201-205); the precision
-// floor is drop * rho; counts the active columns. Single block.
-__global__ void k_cg_start(CgState st, int R, double drop) {
-    __shared__ int cnt;
-    if (threadIdx.x == 0) cnt = 0;
-    __syncthreads();
-    int local = 0;
-    for (int j = threadIdx.x; j < R; j += blockDim.x) {
-        if (st.active[j] == 1 && !(st.rho[j] > 0.0)) st.active[j] = 0;
-        st.pfloor[j] = drop * st.rho[j];
-        local += st.active[j] == 1;
-    }
-    atomicAdd(&cnt, local);  // integer count: order independent
-    __syncthreads();
-    if (threadIdx.x == 0) *st.n_active = cnt;
-}
-
 // End of an FP32 refinement round, on the FP64 quantities of the refined iterate x: rho = r'M^-1 r
 // of its true residual, xconst = x'rhs, pq = x'r. A column is accepted (state 0) only when
 // rho <= max(tol^2 ss_k, floor) with ss_k = ss1 - x'(rhs + r), whether the round ended it by the
@@ -141,13 +124,6 @@ template <class T>
 __global__ void k_sub(T* __restrict__ r, const T* __restrict__ a, const T* __restrict__ b, size_t total) {
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x)
         r[i] = a[i] - b[i];
-}
-
-// p = z masked by the active columns.
-template <class T>
-__global__ void k_mask_copy(T* __restrict__ p, const T* __restrict__ z, const int* __restrict__ active, size_t total, int R) {
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x)
-        p[i] = active[i % R] == 1 ? z[i] : T(0);
 }
 
 // x = 0 on the columns whose mask is 1 (warm starts of zero columns, solve.rs:1209-1217).
@@ -202,8 +178,10 @@ __global__ void k_add_active(T* __restrict__ x, const T* __restrict__ z, const i
 // order.
 template <class T>
 __global__ void __launch_bounds__(TB) k_srow_apply(const double* __restrict__ srow, u32 m, u32 ms,
-                                                   const T* __restrict__ P, int R, T* __restrict__ part) {
+                                                    const T* __restrict__ P, int R, T* __restrict__ part,
+                                                    const int* halt) {
     __shared__ T red[TB];
+    if (halt && __ldcg(halt)) return;  // the PCG loop has ended (pcg.cuh)
     const u32 npairs = ms * u32(R);
     const u32 chunk = (m + gridDim.x - 1) / gridDim.x;
     const u32 f0 = min(m, blockIdx.x * chunk), f1 = min(m, f0 + chunk);
@@ -329,6 +307,41 @@ __global__ void __launch_bounds__(1024) k_ldlt_panel(double* __restrict__ a, dou
     }
 }
 
+// The panel in shared memory with a division per element: the rounding of the blocks that keep it
+// (dense_ldlt_inverse).
+template <int NB>
+__global__ void __launch_bounds__(1024) k_ldlt_panel_div(double* __restrict__ a, double* __restrict__ d, int k, int jb) {
+    extern __shared__ double P[];  // rows jb..k-1 of the panel columns jb..jb+NB-1, NB per row
+    const int nb = min(NB, k - jb), rows = k - jb;
+    for (int idx = threadIdx.x; idx < rows * NB; idx += blockDim.x) {
+        const int r = idx / NB, c = idx % NB;
+        P[idx] = (c < nb && r >= c) ? a[size_t(jb + r) * k + jb + c] : 0.0;
+    }
+    for (int jj = 0; jj < nb; jj++) {
+        __syncthreads();
+        double dj = P[jj * NB + jj];
+        if (dj <= PIVOT_TOL) dj = GROUND;
+        if (threadIdx.x == 0) d[jb + jj] = dj;
+        // the panel's later columns: P[r][l] -= P[r][jj] P[l][jj] / dj for jj < l <= r
+        for (int idx = threadIdx.x; idx < (rows - jj - 1) * NB; idx += blockDim.x) {
+            const int r = jj + 1 + idx / NB, l = idx % NB;
+            if (l > jj && l < nb && l <= r) P[r * NB + l] -= P[r * NB + jj] * P[l * NB + jj] / dj;
+        }
+        __syncthreads();
+        for (int r = jj + 1 + int(threadIdx.x); r < rows; r += blockDim.x) P[r * NB + jj] /= dj;
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < rows * NB; idx += blockDim.x) {
+        const int r = idx / NB, c = idx % NB;
+        if (c < nb && r > c) {
+            a[size_t(jb + r) * k + jb + c] = P[idx];
+            a[size_t(jb + c) * k + jb + r] = P[idx];
+        }
+    }
+}
+
+// Tile (ti, tl), tl <= ti, of the trailing lower triangle (rows and columns from jb + nb): a[i][l]
+// -= sum over the panel's columns p of L[i][p] d_p L[l][p], for l <= i.
 // The whole factor by one CTA for k up to LDLT_WHOLE, without a launch per panel: thread (x, y)
 // holds the elements (y + 16 p, x + 16 q) of what is left of the matrix in registers, the current
 // column passes through shared memory, one barrier and one reciprocal per column. After 16 columns
@@ -504,11 +517,12 @@ __global__ void __launch_bounds__(128) k_ldlt_inverse(const double* __restrict__
             if (lane + 32 * r < k && col + c < k) x[size_t(lane + 32 * r) * k + col + c] = v[c][r];
 }
 
-// The same past 1024 rows, where the registers do not hold a column: one warp per column of X (8 per
+// The same by rows, past 1024 rows (the registers do not hold a column) and for the blocks that keep
+// its rounding (dense_ldlt_inverse): one warp per column of X (8 per
 // block), the column held in shared memory:
 // forward over L's rows (strict lower part), the pivots, backward over L^T's rows (strict upper
 // part), each step a warp-wide dot product combined by a fixed butterfly.
-__global__ void __launch_bounds__(256) k_ldlt_inverse_wide(const double* __restrict__ a, const double* __restrict__ d, int k,
+__global__ void __launch_bounds__(256) k_ldlt_inverse_rows(const double* __restrict__ a, const double* __restrict__ d, int k,
                                                       double* __restrict__ x) {
     extern __shared__ double xs[];
     const int w = int(threadIdx.x / 32), lane = int(threadIdx.x % 32);

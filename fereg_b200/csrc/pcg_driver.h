@@ -21,6 +21,8 @@ struct DevOperator {
     virtual void apply(double* p, int R, double* q, cudaStream_t st) = 0;
     virtual void precond(double* r, double* z, int R, cudaStream_t st) = 0;
     virtual void key(std::vector<u64>& k) const = 0;
+    // set during apply() inside the loop: a device word at which its kernels return when it is not 0
+    const int* halt = nullptr;
 };
 
 struct Scratch;

@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vseg_apply(DevStruct S, DevWeig
     const bool on = int(4 * j) < Rc;
     const size_t Ru = size_t(Rv);
     const T* Pj = P + j0 + 4 * j;
+    if (halted(S)) return;
     T* sp = reinterpret_cast<T*>(smem_raw);
     const int nsm = stage ? int(S.ns_acc) : 0;
     if (nsm) stage_small(sp, P, Ru, j0, Rc, S.ms_acc);
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWei
     const u32 no = S.nb - 1;
     const T* Pj = P + j0 + 4 * j;
     const T* tj = t + j0 + 4 * j;
+    if (halted(S)) return;
     // the lists are of large coordinates: the small blocks come first among a cell's other blocks
     T* sp = reinterpret_cast<T*>(smem_raw + size_t(WPB) * WS);
     const int nsm = stage ? int(S.ns_acc) : 0;

@@ -237,9 +237,9 @@ struct SlopeOp final : DevOperator {
     void apply(double* p, int R, double* q, cudaStream_t st) override {
         d.Z.alloc(std::max<size_t>(1, h.n * size_t(R)));
         k_sl_seg<SL_APPLY><<<sl_grid(size_t(h.ge) * R), SL_TB, 0, st>>>(D, p, R, R, nullptr, 0, d.Z.p, R, nullptr,
-                                                                        nullptr, 0, nullptr);
+                                                                        nullptr, 0, nullptr, halt);
         k_sl_pull<<<sl_grid(size_t(h.m) * R), SL_TB, 0, st>>>(h.m, R, d.pl_off.p, d.pl_row.p, d.pl_val.p, d.Z.p, R, q,
-                                                               R);
+                                                               R, halt);
         d.launches += 2;
     }
     void precond(double* r, double* z, int R, cudaStream_t st) override {

@@ -61,7 +61,8 @@ template <int MODE>
 __global__ void __launch_bounds__(SL_TB) k_sl_seg(SlopeDev D, const double* src, int lds, int C,
                                                    const double* __restrict__ x, int ldx, double* __restrict__ Z,
                                                    int ldz, double* rows_out, double* __restrict__ alpha, int lda,
-                                                   double* __restrict__ part) {
+                                                   double* __restrict__ part, const int* halt = nullptr) {
+    if (halt && __ldcg(halt)) return;  // the PCG loop has ended (pcg.cuh)
     const size_t total = size_t(D.ge) * C;
     const int be = int(D.be);
     for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < total; q += size_t(gridDim.x) * blockDim.x) {
@@ -125,7 +126,8 @@ __global__ void __launch_bounds__(SL_TB) k_sl_seg(SlopeDev D, const double* src,
 __global__ void __launch_bounds__(SL_TB) k_sl_pull(u32 m, int C, const u32* __restrict__ pl_off,
                                                     const u32* __restrict__ pl_row, const double* __restrict__ pl_val,
                                                     const double* __restrict__ Z, int ldz, double* __restrict__ Y,
-                                                    int ldy) {
+                                                    int ldy, const int* halt = nullptr) {
+    if (halt && __ldcg(halt)) return;
     const size_t total = size_t(m) * C;
     for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < total; q += size_t(gridDim.x) * blockDim.x) {
         const u32 c = u32(q / C);

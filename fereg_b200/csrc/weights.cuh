@@ -174,7 +174,8 @@ __global__ void k_coord_combine(const u32* __restrict__ list_chunk_off, u32 m, c
 // have (k_small_rows) beyond: a tile costs about 0.6 ns a segment, a cell's code about 1 ns. Measured
 // with 10 cells a segment, both sums: 1e6 segments and 10 coordinates 0.16 ms (7.5 ms by lists, a
 // lane at a time, before), 1e6 and 110 2.2 ms (20.0), 2e4 and 310 0.20 ms by tiles and 0.31 by
-// lists, 2e5 and 910 4.2 ms by lists (6.4), where the 120 tiles would take 14. Every sum has a fixed
+// lists, 2e5 and 910 4.2 ms by lists (6.4), where the 120 tiles would take 14; one unweighted block
+// keeps the order it always had (k_small_ordered). Every sum has a fixed
 // order.
 //
 // Partial row k of the first sum by work items (row k, a run of its list's entries): a warp takes
@@ -273,6 +274,69 @@ __global__ void __launch_bounds__(256) k_small_rows(const u32* __restrict__ seg_
         }
     }
     for (u32 l = lane; l < ms; l += 32) part[size_t(it) * ms + l] = row[l];
+}
+
+// One unweighted small block of at most 32 coordinates, by the lists' entries in order: the partial
+// row of an item (row k, a run of its list that never splits a segment), a lane per coordinate l.
+// For every entry S[k][k] += 1; once per segment s of the run S[k][l] -= c_{s,k} / n1_s for each of the
+// c_{s,l} cells that hold l (csk: the counts, g1 x ms). A lane's sum is one chain over the item, in
+// entry order; the loads of 8 entries are in flight together. This is the block of a panel's years
+// on a one-row-per-cell panel; its rounding steers the PCG's path, which on an ill-conditioned graph
+// decides the answer's eighth digit, so the order of the sums is the one this block always had.
+// 1e6 segments of 10 cells, 10 coordinates: 7.5 ms with one lane an item, 0.70 ms here (0.16 as tiles).
+__global__ void __launch_bounds__(256) k_small_ordered(u32 ms, const double* __restrict__ n1inv,
+                                                       const double* __restrict__ csk, const u32* __restrict__ pl_seg,
+                                                       const u32* __restrict__ item_k, const u32* __restrict__ item_a,
+                                                       const u32* __restrict__ item_b, u32 nitems,
+                                                       double* __restrict__ part) {
+    constexpr int U = 8;
+    constexpr u32 NONE = 0xffffffffu;
+    const u32 lane = threadIdx.x % 32;
+    const u32 it = blockIdx.x * 8 + threadIdx.x / 32;
+    if (it >= nitems) return;  // whole warps
+    const u32 k = item_k[it], b = item_b[it];
+    double acc = 0.0;
+    u32 prev = NONE;
+    for (u32 base = item_a[it]; base < b; base += 32) {
+        const u32 e = base + lane;
+        const u32 s = e < b ? pl_seg[e] : NONE;
+        const double ni = e < b ? n1inv[s] : 0.0;
+        const u32 left = __shfl_up_sync(FULL, s, 1);
+        const bool opens = e < b && s != (lane == 0 ? prev : left);  // a segment's entries are consecutive
+        const unsigned open = __ballot_sync(FULL, opens);
+        const int n = int(min(32u, b - base));
+        for (int j0 = 0; j0 < n; j0 += U) {
+            double c[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const u32 sj = __shfl_sync(FULL, s, j0 + u);
+                c[u] = (j0 + u < n && lane < ms) ? csk[size_t(sj) * ms + lane] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const double f = __shfl_sync(FULL, c[u], int(k)) * __shfl_sync(FULL, ni, j0 + u);
+                if (j0 + u < n) {
+                    if (lane == k) acc += 1.0;
+                    if ((open >> (j0 + u)) & 1u)
+                        for (int q = int(c[u]); q > 0; q--) acc -= f;
+                }
+            }
+        }
+        prev = __shfl_sync(FULL, s, n - 1);
+    }
+    if (lane < ms) part[size_t(it) * ms + lane] = acc;
+}
+
+// Row k of S_SS: the partial rows of k's items (first[k] .. first[k+1]) added in item order.
+__global__ void k_small_items_sum(const double* __restrict__ part, const u32* __restrict__ first, u32 ms,
+                                  double* __restrict__ out) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ms * ms) return;
+    const u32 k = i / ms, l = i % ms;
+    double v = 0.0;
+#pragma unroll 16
+    for (u32 it = first[k]; it < first[k + 1]; it++) v += part[size_t(it) * ms + l];
+    out[i] = v;
 }
 
 // The Gram matrix sum_s c_s c_s' / n1_s by tiles of BT x BT (tile (ti, tj), tj <= ti, in blockIdx.y;
