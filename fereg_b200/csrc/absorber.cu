@@ -1,9 +1,9 @@
 // GpuAbsorber: structure on the host, the solve on the B200.
 //
-// residualize (solve.rs:1141-1311) runs the rhs pass over the rows (k_seg_rhs + k_pull_rhs),
-// lockstep PCG on the reduced system (k_seg_apply + k_pull_apply per matvec; Jacobi / grounded
+// residualize (solve.rs:1141-1311) runs the rhs pass over the rows (segments, then coordinate lists),
+// lockstep PCG on the reduced system (the same two passes per matvec; Jacobi / grounded
 // dense small-block preconditioner; per-column scalars on the device), and the in-place
-// residualization pass (k_residualize). With Precision::F32_REFINED the PCG iterations run in
+// residualization pass. With Precision::F32_REFINED the PCG iterations run in
 // FP32 on the correction of an FP64 iterate whose true residual is recomputed in FP64 between
 // rounds (iterative refinement); the stopping rule is evaluated on the FP64 quantities.
 
@@ -32,10 +32,10 @@ constexpr int THREADS = TB;
 constexpr int GRID_T = 148 * 6;  // tile kernels: up to 6 resident CTAs per SM
 constexpr int GRID_V = 148 * 2;  // vector kernels with per-CTA partials
 constexpr int GRID_S = 148 * 4;  // warp-tile kernels (CTAs of WPB warps)
+constexpr int LT_GRID = 148 * 4; // long-list kernels (CTAs of LT_WPB warps)
 // CTAs of the dense small rows' product over m coordinates (k_srow_apply).
 inline u32 small_row_ctas(u32 m) { return std::max<u32>(1, std::min<u32>(4 * GRID_V, (m + 31) / 32)); }
 constexpr size_t SMALL_STAGE_MAX = 16 * 1024;  // shared memory for the staged small rows of a chunk
-constexpr u32 VSEG_MAX = 256;  // longest segment (cells) a lane group walks in the operator's segment pass
 constexpr double REDUNDANT = 1e-12;  // operator.rs:21
 // Largest small super-block factored densely on the device. Beyond it the small coordinates keep
 // Jacobi, as the reference does when the dense factor costs more than a few PCG iterations
@@ -189,11 +189,14 @@ struct Scratch {
     DevTiles seg_tiles, pull_tiles;      // CTA tiles of the long lists
     DevWarpTiles wseg, wpull;            // warp tiles of the short lists
     DBuf<u32> wseg_segs;                 // the segments of the warp tiles, in order
-    DBuf<u32> aseg_segs;                 // the operator's lane-group segments (at most VSEG_MAX cells)
+    DBuf<u32> aseg_segs;                 // the operator's lane-group segments (at most LONG_SEG cells)
     DevTiles aseg_tiles;                 // the operator's CTA tiles (longer segments)
     u32 ms_acc = 0, ns_acc = 0;  // small coordinates / blocks summed in the segment passes
+    size_t nrows = 0;
     // weights
     DBuf<double> w_rows, cell_w, n1inv, nr, inv_diag, minv;
+    DBuf<double> pl_w;             // the cells' weights in list order
+    DBuf<double> cellsum;          // the cells' row sums of a right-hand side pass
     DBuf<double> n1, diag, wpart;  // device weight refresh
     DBuf<u32> pi;                  // the row order (kept observation of each row)
     DBuf<u32> cw_e0, cw_e1, cw_list_off;  // chunks of the coordinate lists (weights.cuh)
@@ -282,7 +285,7 @@ struct Scratch {
         s.pull = pull_tiles.set();
         return s;
     }
-    DevWeights dw() const { return DevWeights{w_rows.p, cell_w.p, n1inv.p, nr.p}; }
+    DevWeights dw() const { return DevWeights{w_rows.p, cell_w.p, n1inv.p, nr.p, pl_w.p}; }
     CgState cg() {
         return CgState{cg_rho.p, cg_rho_new.p, cg_pq.p,   cg_gamma.p,  cg_beta.p,   cg_xb.p,     cg_ss1.p,
                        cg_floor.p, cg_ring.p, cg_xconst.p, cg_pfloor.p, cg_active.p, cg_nactive.p};
@@ -411,19 +414,20 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
         WarpTileList wt;
         TileList ct;
         split_tiles(hs_.seg_off, &wgt, 0, hs_.g1, WT, WT, WSEG, TILE, wt, ct);
+            d_->nrows = n;
         d_->wseg.upload(wt, stream_);
         std::vector<u32> segs;  // the short segments in order (one per lane group in k_vseg_apply)
         for (size_t i = 0; i < wt.k0.size(); i++)
             for (u32 s = wt.k0[i]; s < wt.k1[i]; s++) segs.push_back(s);
         d_->wseg_segs.upload(segs, stream_);
         d_->seg_tiles.upload(ct, stream_);
-        // the operator's segment pass: lane groups walk every segment of at most VSEG_MAX cells (in
+        // the operator's segment pass: lane groups walk every segment of at most LONG_SEG cells (in
         // order), CTA tiles take the longer ones
         std::vector<u32> asegs;
         for (u32 s = 0; s < hs_.g1; s++)
-            if (hs_.seg_off[s + 1] - hs_.seg_off[s] <= VSEG_MAX) asegs.push_back(s);
+            if (hs_.seg_off[s + 1] - hs_.seg_off[s] <= LONG_SEG) asegs.push_back(s);
         d_->aseg_segs.upload(asegs, stream_);
-        d_->aseg_tiles.upload(build_tiles(hs_.seg_off, 0, hs_.g1, TILE, VSEG_MAX), stream_);
+        d_->aseg_tiles.upload(build_tiles(hs_.seg_off, 0, hs_.g1, TILE, LONG_SEG), stream_);
         CK(cudaStreamSynchronize(stream_));
     }
     {
@@ -496,7 +500,13 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
         }
         WarpTileList wt;
         TileList ct;
-        split_tiles(pl_off, nullptr, d_->ms_acc, u32(hs_.m), PULL_WARP_MAX, PULL_WARP_MAX, WLIST, PULL_SLICE, wt, ct);
+        // the long lists' slices: PULL_SLICE entries, fewer where that gives less than three CTAs an SM
+        // (at most 888 slices then)
+        u64 el = 0;
+        for (u32 k = d_->ms_acc; k < u32(hs_.m); k++)
+            if (pl_off[k + 1] - pl_off[k] > PULL_WARP_MAX) el += pl_off[k + 1] - pl_off[k];
+        const u32 slice = u32(std::min<u64>(PULL_SLICE, (el / 444 + 255) / 256 * 256 + 256));
+        split_tiles(pl_off, nullptr, d_->ms_acc, u32(hs_.m), PULL_WARP_MAX, PULL_WARP_MAX, WLIST, slice, wt, ct);
         d_->wpull.upload(wt, stream_);
         d_->pull_tiles.upload(ct, stream_);
         CK(cudaStreamSynchronize(stream_));  // host tables die here
@@ -782,6 +792,14 @@ void GpuAbsorber::refresh_coord() const {
     k_coord_combine<<<grid_for(m), THREADS, 0, stream_>>>(d.cw_list_off.p, u32(m), ch, d.n1inv.p, d.nr.p, d.diag.p,
                                                           d.red.p, d.inv_diag.p);
     d.launches += 2;
+    if (d.cell_w.p) {
+        const size_t E = hs_.ncells * hs_.nb();
+        d.pl_w.alloc(E);
+        k_list_weights<<<grid_for(E), THREADS, 0, stream_>>>(d.cell_w.p, d.pl_cell.p, E, d.pl_w.p);
+        d.launches++;
+    } else {
+        d.pl_w.release();
+    }
     CK(cudaGetLastError());
     coord_stale_ = false;
 }
@@ -1114,8 +1132,19 @@ void launch_apply(Scratch& d, const DevStruct& S, const DevWeights& W, const T* 
             d.launches++;
         }
     if (SA.seg.n) {
-        k_seg_apply<T><<<GRID_T, THREADS, 0, st>>>(SA, W, P, Rv, t, part, false, nullptr);
-        d.launches++;
+        for (int j0 = 0; j0 < Rv; j0 += VCOLS) {
+            const int Rc = std::min(VCOLS, Rv - j0);
+            const size_t sm = small_stage_bytes<T>(S.ms_acc, Rc);
+            const int stage = S.ns_acc > 0 && sm <= SMALL_STAGE_MAX;
+            with_vlanes(Rc, S.nb, [&](auto lc, auto nbk) {
+                constexpr int L = decltype(lc)::value, NBK = decltype(nbk)::value;
+                if (weighted)
+                    k_ltile_apply<T, L, NBK, true><<<LT_GRID, LT_WPB * 32, stage ? sm : 0, st>>>(SA, W, P, Rv, j0, Rc, t, part, stage);
+                else
+                    k_ltile_apply<T, L, NBK, false><<<LT_GRID, LT_WPB * 32, stage ? sm : 0, st>>>(SA, W, P, Rv, j0, Rc, t, part, stage);
+            });
+            d.launches++;
+        }
         if (SA.seg.nfix) {
             k_fix<T><<<std::min<u32>(SA.seg.nfix, GRID_T), THREADS, 0, st>>>(SA.seg, W, P, part, Rv, 1, t);
             d.launches++;
@@ -1143,8 +1172,17 @@ void launch_apply(Scratch& d, const DevStruct& S, const DevWeights& W, const T* 
             d.launches++;
         }
     if (S.pull.n) {
-        k_pull_apply<T><<<GRID_T, THREADS, 0, st>>>(S, W, P, t, Rv, Y, part);
-        d.launches++;
+        for (int j0 = 0; j0 < Rv; j0 += VCOLS) {
+            const int Rc = std::min(VCOLS, Rv - j0);
+            with_vlanes(Rc, S.nb, [&](auto lc, auto nbk) {
+                constexpr int L = decltype(lc)::value, NBK = decltype(nbk)::value;
+                if (weighted)
+                    k_ltile_pull<T, L, NBK, true><<<LT_GRID, LT_WPB * 32, 0, st>>>(S, W, P, t, Rv, j0, Rc, Y, part);
+                else
+                    k_ltile_pull<T, L, NBK, false><<<LT_GRID, LT_WPB * 32, 0, st>>>(S, W, P, t, Rv, j0, Rc, Y, part);
+            });
+            d.launches++;
+        }
         if (S.pull.nfix) {
             k_fix<T><<<std::min<u32>(S.pull.nfix, GRID_T), THREADS, 0, st>>>(S.pull, W, P, part, Rv, 0, Y);
             d.launches++;
@@ -1305,6 +1343,30 @@ void reduce_cols(Scratch& d, const double* part, int nparts, int ncols, double* 
     CK(cudaGetLastError());
 }
 
+// The long segments' share of the right-hand side (cta: GRID_T x 2R): small (when given) takes the
+// small coordinates' partials, cs the cells' sums.
+void launch_long_rhs(Scratch& d, const DevStruct& S, const DevWeights& W, const double* rows, int R, double* b1,
+                     double* part, double* cta, double* small, double* cs, cudaStream_t st) {
+    if (small) {
+        k_seg_rhs<<<GRID_T, THREADS, 0, st>>>(S, W, rows, R, b1, part, cta, small, cs);
+        d.launches++;
+        return;
+    }
+    for (int j0 = 0; j0 < R; j0 += WCOLS) {
+        k_ltile_rhs<<<GRID_T, LT_WPB * 32, 0, st>>>(S, W, rows, R, j0, std::min(WCOLS, R - j0), b1, part, cta, cs);
+        d.launches++;
+    }
+}
+
+// The long lists' share of the right-hand side.
+void launch_long_pull_rhs(Scratch& d, const DevStruct& S, const DevWeights& W, const double* rows, int R,
+                          const double* b1, double* rhs, double* part, const double* cs, cudaStream_t st) {
+    for (int j0 = 0; j0 < R; j0 += WCOLS) {
+        k_ltile_pull_rhs<<<GRID_T, LT_WPB * 32, 0, st>>>(S, W, rows, b1, R, j0, std::min(WCOLS, R - j0), rhs, part, cs);
+        d.launches++;
+    }
+}
+
 // rhs pass: b1 per segment, [sum w v^2, sum w v, sum b1^2/n1] per column into colsum (3R), and
 // the reduced right-hand side (small coordinates in the segment passes, the others pulled).
 void launch_rhs(Scratch& d, const DevStruct& S, const DevWeights& W, const double* rows, int R, double* b1,
@@ -1312,6 +1374,13 @@ void launch_rhs(Scratch& d, const DevStruct& S, const DevWeights& W, const doubl
     const bool acc = S.ms_acc > 0;
     const u32 len = S.ms_acc * u32(R);
     double* small = d.small.p;
+    // cells of several rows: pass 1 leaves their sums for the lists (twice as many rows as cells pay
+    // for the write)
+    double* cs = nullptr;
+    if (S.cell_row && S.m > 0 && d.nrows >= 2 * size_t(S.M)) {
+        d.cellsum.alloc(size_t(S.M) * R);
+        cs = d.cellsum.p;
+    }
     int h = d.begin(GpuAbsorber::P_RHS_SEG, st);
     if (d.wseg.n) {
         for (int j0 = 0; j0 < R; j0 += WCOLS) {
@@ -1323,7 +1392,7 @@ void launch_rhs(Scratch& d, const DevStruct& S, const DevWeights& W, const doubl
                     constexpr int NSA = decltype(nsa)::value;
                     allow_smem(k_grhs<RCP, NSA>, shm);
                     k_grhs<RCP, NSA><<<GRID_S, WPB * 32, shm, st>>>(S, W, d.wseg_segs.p, u32(d.wseg_segs.n), rows, R,
-                                                                     j0, Rc, b1, d.cta2.p, acc ? small : nullptr);
+                                                                     j0, Rc, b1, d.cta2.p, acc ? small : nullptr, cs);
                 });
             });
             d.launches++;
@@ -1334,8 +1403,7 @@ void launch_rhs(Scratch& d, const DevStruct& S, const DevWeights& W, const doubl
     }
     if (S.seg.n) {
         double* sb = small + size_t(GRID_S) * len;
-        k_seg_rhs<<<GRID_T, THREADS, 0, st>>>(S, W, rows, R, b1, d.part.p, d.cta.p, acc ? sb : nullptr);
-        d.launches++;
+        launch_long_rhs(d, S, W, rows, R, b1, d.part.p, d.cta.p, acc ? sb : nullptr, cs, st);
         if (S.seg.nfix) {
             k_fix<double><<<std::min<u32>(S.seg.nfix, GRID_T), THREADS, 0, st>>>(S.seg, W, nullptr, d.part.p, R, 2, b1);
             d.launches++;
@@ -1360,13 +1428,12 @@ void launch_rhs(Scratch& d, const DevStruct& S, const DevWeights& W, const doubl
                 with_rcp<WNB>(Rc, WNB, [&](auto c, auto) {
                     constexpr int RCP = decltype(c)::value;
                     k_wpull_rhs<RCP><<<GRID_S, WPB * 32, wpull_smem(), st>>>(S, W, d.wpull.set(), rows, b1, R, j0, Rc,
-                                                                              rhs);
+                                                                              rhs, cs);
                 });
                 d.launches++;
             }
         if (S.pull.n) {
-            k_pull_rhs<<<GRID_T, THREADS, 0, st>>>(S, W, rows, b1, R, rhs, d.part.p);
-            d.launches++;
+            launch_long_pull_rhs(d, S, W, rows, R, b1, rhs, d.part.p, cs, st);
             if (S.pull.nfix) {
                 k_fix<double><<<std::min<u32>(S.pull.nfix, GRID_T), THREADS, 0, st>>>(S.pull, W, nullptr, d.part.p, R, 2, rhs);
                 d.launches++;
@@ -1386,7 +1453,7 @@ struct RhsScratch {
 };
 inline size_t rhs_scratch_part(size_t doubles) { return (doubles + 31) / 32 * 32; }  // 256-byte steps
 inline size_t rhs_scratch_need(const DevStruct& S, size_t r, u32 ms_acc) {
-    return rhs_scratch_part(size_t(GRID_S) * 2 * r) + rhs_scratch_part(size_t(std::max(GRID_T, GRID_V)) * 3 * r) +
+    return rhs_scratch_part(size_t(GRID_S) * 2 * r) + rhs_scratch_part(size_t(GRID_T) * 2 * r) +
            rhs_scratch_part(std::max<size_t>(1, size_t(std::max(S.seg.nparts, S.pull.nparts)) * r)) +
            rhs_scratch_part(std::max<size_t>(1, small_rows() * ms_acc * r));
 }
@@ -1395,7 +1462,7 @@ inline RhsScratch rhs_scratch_carve(double* p, const DevStruct& S, size_t r, u32
     s.cta2 = p;
     p += rhs_scratch_part(size_t(GRID_S) * 2 * r);
     s.cta = p;
-    p += rhs_scratch_part(size_t(std::max(GRID_T, GRID_V)) * 3 * r);
+    p += rhs_scratch_part(size_t(GRID_T) * 2 * r);
     s.part = p;
     p += rhs_scratch_part(std::max<size_t>(1, size_t(std::max(S.seg.nparts, S.pull.nparts)) * r));
     s.small = p;
@@ -1417,7 +1484,7 @@ void launch_rhs_scratch(Scratch& d, const DevStruct& S, const DevWeights& W, con
                     constexpr int NSA = decltype(nsa)::value;
                     allow_smem(k_grhs<RCP, NSA>, shm);
                     k_grhs<RCP, NSA><<<GRID_S, WPB * 32, shm, st>>>(S, W, d.wseg_segs.p, u32(d.wseg_segs.n), rows, R,
-                                                                     j0, Rc, b1, x.cta2, acc ? x.small : nullptr);
+                                                                     j0, Rc, b1, x.cta2, acc ? x.small : nullptr, nullptr);
                 });
             });
             d.launches++;
@@ -1429,8 +1496,7 @@ void launch_rhs_scratch(Scratch& d, const DevStruct& S, const DevWeights& W, con
     }
     if (S.seg.n) {
         double* sb = x.small + size_t(GRID_S) * len;
-        k_seg_rhs<<<GRID_T, THREADS, 0, st>>>(S, W, rows, R, b1, x.part, x.cta, acc ? sb : nullptr);
-        d.launches++;
+        launch_long_rhs(d, S, W, rows, R, b1, x.part, x.cta, acc ? sb : nullptr, nullptr, st);
         if (S.seg.nfix) {
             k_fix<double><<<std::min<u32>(S.seg.nfix, GRID_T), THREADS, 0, st>>>(S.seg, W, nullptr, x.part, R, 2, b1);
             d.launches++;
@@ -1451,13 +1517,12 @@ void launch_rhs_scratch(Scratch& d, const DevStruct& S, const DevWeights& W, con
                 with_rcp<WNB>(Rc, WNB, [&](auto c, auto) {
                     constexpr int RCP = decltype(c)::value;
                     k_wpull_rhs<RCP><<<GRID_S, WPB * 32, wpull_smem(), st>>>(S, W, d.wpull.set(), rows, b1, R, j0, Rc,
-                                                                              rhs);
+                                                                              rhs, nullptr);
                 });
                 d.launches++;
             }
         if (S.pull.n) {
-            k_pull_rhs<<<GRID_T, THREADS, 0, st>>>(S, W, rows, b1, R, rhs, x.part);
-            d.launches++;
+            launch_long_pull_rhs(d, S, W, rows, R, b1, rhs, x.part, nullptr, st);
             if (S.pull.nfix) {
                 k_fix<double><<<std::min<u32>(S.pull.nfix, GRID_T), THREADS, 0, st>>>(S.pull, W, nullptr, x.part, R, 2,
                                                                                       rhs);
@@ -1621,7 +1686,7 @@ struct FeOp {
         auto put = [&](const void* ptr) { k.push_back(u64(reinterpret_cast<uintptr_t>(ptr))); };
         k.push_back(small_ok);
         for (const void* ptr : {(const void*)t, (const void*)part, (const void*)W.w_rows,
-                                (const void*)W.cell_w, (const void*)W.n1inv, (const void*)W.nr, (const void*)d.inv_diag.p,
+                                (const void*)W.cell_w, (const void*)W.n1inv, (const void*)W.nr, (const void*)W.pl_w, (const void*)d.inv_diag.p,
                                 (const void*)d.minv.p, (const void*)d.srow.p})
             put(ptr);
         k.push_back(d.amg.size());
@@ -2131,13 +2196,21 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
         }
     if (S.seg.nfix) {
         d.along.alloc(size_t(S.seg.nfix) * r);
-        k_seg_apply<double><<<GRID_T, THREADS, 0, st>>>(S, W, x, R, d.t.p, d.part.p, true, nullptr);
+        k_slice_wu<<<GRID_T, THREADS, 0, st>>>(S, W, x, R, d.part.p);
         k_fix_alpha<<<std::min<u32>(S.seg.nfix, GRID_T), THREADS, 0, st>>>(S.seg, W, d.part.p, d.b1.p, R, d.along.p, alpha);
         d.launches += 2;
     }
     if (S.seg.n) {
-        k_residualize<<<GRID_T, THREADS, 0, st>>>(S, W, rows, R, x, d.b1.p, d.along.p, alpha);
-        d.launches++;
+        for (int j0 = 0; j0 < R; j0 += LR_COLS) {
+            const int Rc = std::min(LR_COLS, R - j0);
+            const size_t shm = LR_WPB * ltile_resid_bytes(Rc);
+            with_nbk<1, 0>(S.nb, [&](auto, auto nbk) {
+                constexpr int NBK = decltype(nbk)::value;
+                allow_smem(k_ltile_resid<NBK>, shm);
+                k_ltile_resid<NBK><<<148 * 8, LR_WPB * 32, shm, st>>>(S, W, rows, R, j0, Rc, x, d.b1.p, d.along.p, alpha);
+            });
+            d.launches++;
+        }
     }
     d.end(h, st);
     CK(cudaGetLastError());

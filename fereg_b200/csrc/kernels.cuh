@@ -15,6 +15,7 @@
 // fixed per-CTA partials in CTA order. No floating-point atomics.
 #pragma once
 
+#include "long.cuh"
 #include "short.cuh"
 
 namespace fereg {

@@ -420,43 +420,39 @@ __device__ __forceinline__ void stage_pull(const DevStruct& S, u32 k0, u32 k1, u
 }
 
 // Per-warp buffer of the list pass's software pipeline: the tile's list ends (pl_off, global
-// entry indices), and per entry its segment, cell (weighted cells only) and NO other coordinates.
-template <int NO, bool WEIGHTED>
+// entry indices), and per entry its segment and NO other coordinates.
+template <int NO>
 __host__ __device__ constexpr size_t vpull_buf_bytes() {
-    return al16(WLIST * 4) + al16(PULL_WARP_MAX * 4) * (1 + (WEIGHTED ? 1 : 0) + NO);
+    return al16(WLIST * 4) + al16(PULL_WARP_MAX * 4) * (1 + NO);
 }
-// Per-warp shared memory of the list pass: two pipeline buffers, or (weighted cells) one stage.
+// Per-warp shared memory of the list pass: two pipeline buffers (weighted cells: none).
 template <int NO, bool WEIGHTED>
 __host__ __device__ constexpr size_t vpull_warp_bytes() {
-    return WEIGHTED ? pull_bytes() : 2 * vpull_buf_bytes<NO, WEIGHTED>();
+    return WEIGHTED ? 0 : 2 * vpull_buf_bytes<NO>();
 }
 struct VPullBuf {
     u32* kend;
     u32* seg;
-    u32* cell;
     u32* oth;  // NO x PULL_WARP_MAX
 };
-template <int NO, bool WEIGHTED>
+template <int NO>
 __device__ __forceinline__ VPullBuf vpull_buf_at(unsigned char* p) {
     VPullBuf b;
     b.kend = reinterpret_cast<u32*>(p);
     p += al16(WLIST * 4);
     b.seg = reinterpret_cast<u32*>(p);
     p += al16(PULL_WARP_MAX * 4);
-    b.cell = reinterpret_cast<u32*>(p);
-    if (WEIGHTED) p += al16(PULL_WARP_MAX * 4);
     b.oth = reinterpret_cast<u32*>(p);
     return b;
 }
 // Issues the copies of list tile tb into buffer b (the caller commits the group).
-template <int NO, bool WEIGHTED>
+template <int NO>
 __device__ __forceinline__ void vpull_prefetch(const DevStruct& S, const uint4& tb, const VPullBuf& b) {
     const u32 lane = wlane(), k0 = tb.x, k1 = tb.y, e0 = tb.z, ne = tb.w - tb.z;
     const u32 no = S.nb - 1;
     if (lane < k1 - k0) cp_async4(b.kend + lane, S.pl_off + k0 + lane + 1);
     for (u32 i = lane; i < ne; i += 32) {
         cp_async4(b.seg + i, S.pl_seg + e0 + i);
-        if (WEIGHTED) cp_async4(b.cell + i, S.pl_cell + e0 + i);
 #pragma unroll
         for (int o = 0; o < NO; o++) cp_async4(b.oth + o * PULL_WARP_MAX + i, S.pl_other + size_t(e0 + i) * no + o);
     }
@@ -468,9 +464,10 @@ __device__ __forceinline__ void vpull_prefetch(const DevStruct& S, const uint4& 
 // columns), and the groups' sums are added by a fixed xor butterfly. Unweighted cells: software
 // pipelined, cp.async copies bring the next tile's list ends and entries' segments and other
 // coordinates into the second of two shared buffers while a warp works on one tile (measured:
-// the 1e6-row bootstrap panel's list pass 8% faster). Weighted cells stage each tile before
-// working on it, in the shared memory they always took (the pipelined form, with its larger
-// buffers, measured 1.7x slower on the gravity panel's weighted lists).
+// the 1e6-row bootstrap panel's list pass 8% faster). Weighted cells read the indices and the
+// weights (in list order, W.pl_w) straight from memory: on the gravity panel's lists of 200 entries,
+// one entry a lane, staging and its barriers cost more than they hid (4e6 entries, 4 columns: 67 us
+// staged with the weights gathered by cell, 65 staged with them in order, 53 here).
 template <class T, int L, int NBK, bool WEIGHTED>
 __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWeights W, WarpTiles wt,
                                                              const T* __restrict__ P, const T* __restrict__ t, int Rv,
@@ -478,7 +475,7 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWei
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int G = 32 / L;
     constexpr int NO = NBK - 1;  // staged other blocks (all of them below WNB blocks)
-    constexpr u32 BB = u32(vpull_buf_bytes<NO, WEIGHTED>());
+    constexpr u32 BB = u32(vpull_buf_bytes<NO>());
     constexpr u32 WS = u32(vpull_warp_bytes<NO, WEIGHTED>());
     unsigned char* mine = smem_raw + size_t(wid_in_cta()) * WS;
     const u32 lane = wlane(), g = lane / L, j = lane % L;
@@ -498,9 +495,9 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWei
         for (int o = L; o < 32; o <<= 1) v += __shfl_xor_sync(FULL, v, o);
         return v;
     };
-    // the lists of one staged tile; kend[kl] - kbase: local end of list kl
-    auto work = [&](const u32* kend, u32 kbase, const u32* seg, const u32* cell, const u32* oth, u32 k0, u32 k1,
-                    u32 e0) {
+    // the lists of one tile, the entries' indices from the staging; kend[kl] - kbase: local end of list
+    // kl. Weighted: straight from the structure (indices and weights in list order, kend = pl_off).
+    auto work = [&](const u32* kend, u32 kbase, const u32* seg, const u32* oth, u32 k0, u32 k1, u32 e0) {
         u32 i0 = 0;
         for (u32 kl = 0; kl < k1 - k0; kl++) {
             const u32 ie = kend[kl] - kbase;
@@ -508,20 +505,20 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWei
             if (on) {
 #pragma unroll 4
                 for (u32 i = i0 + g; i < ie; i += G) {
-                    V4<T> v = ld4cg(tj + size_t(seg[i]) * Ru);
+                    V4<T> v = ld4cg(tj + size_t(WEIGHTED ? __ldcs(S.pl_seg + e0 + i) : seg[i]) * Ru);
                     v.a = -v.a;
                     v.b = -v.b;
                     v.c = -v.c;
                     v.d = -v.d;
 #pragma unroll
                     for (int o = 0; o < NO; o++) {
-                        const u32 x = oth[o * PULL_WARP_MAX + i];
+                        const u32 x = WEIGHTED ? __ldcs(S.pl_other + size_t(e0 + i) * no + o) : oth[o * PULL_WARP_MAX + i];
                         add4(v, o < nsm ? ld4s(spj + size_t(x) * Rc) : ld4(Pj + size_t(x) * Ru));
                     }
                     if constexpr (NBK == WNB)
                         for (u32 o = WNO; o < no; o++)
                             add4(v, ld4(Pj + size_t(S.pl_other[size_t(e0 + i) * no + o]) * Ru));
-                    if constexpr (WEIGHTED) fma4(acc, T(W.cell_w[cell[i]]), v);
+                    if constexpr (WEIGHTED) fma4(acc, T(__ldcs(W.pl_w + e0 + i)), v);
                     else add4(acc, v);
                 }
             }
@@ -541,31 +538,27 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWei
     const u32 wid = blockIdx.x * WPB + wid_in_cta(), nw = gridDim.x * WPB;
     uint4 tb = wid < wt.n ? wt.t[wid] : make_uint4(0, 0, 0, 0);
     if constexpr (WEIGHTED) {
-        const PullStage st = pull_stage_at(mine);
         for (u32 tile = wid; tile < wt.n; tile += nw) {
-            const u32 k0 = tb.x, k1 = tb.y, e0 = tb.z;
-            stage_pull(S, k0, k1, e0, tb.w, st, true, u32(NO));
+            const uint4 tc = tb;
             if (tile + nw < wt.n) tb = wt.t[tile + nw];
-            __syncwarp();
-            work(st.kend, 0u, st.seg, st.cell, st.oth, k0, k1, e0);
-            __syncwarp();
+            work(S.pl_off + tc.x + 1, tc.z, nullptr, nullptr, tc.x, tc.y, tc.z);
         }
     } else {
         uint4 tn = wid + nw < wt.n ? wt.t[wid + nw] : make_uint4(0, 0, 0, 0);  // the next tile
-        if (wid < wt.n) vpull_prefetch<NO, WEIGHTED>(S, tb, vpull_buf_at<NO, WEIGHTED>(mine));
+        if (wid < wt.n) vpull_prefetch<NO>(S, tb, vpull_buf_at<NO>(mine));
         cp_async_commit();
         u32 it = 0;
         for (u32 tile = wid; tile < wt.n; tile += nw, it++) {
-            const VPullBuf b = vpull_buf_at<NO, WEIGHTED>(mine + (it & 1) * BB);
+            const VPullBuf b = vpull_buf_at<NO>(mine + (it & 1) * BB);
             if (tile + nw < wt.n)
-                vpull_prefetch<NO, WEIGHTED>(S, tn, vpull_buf_at<NO, WEIGHTED>(mine + ((it + 1) & 1) * BB));
+                vpull_prefetch<NO>(S, tn, vpull_buf_at<NO>(mine + ((it + 1) & 1) * BB));
             cp_async_commit();
             const uint4 tc = tb;
             tb = tn;
             if (tile + 2 * nw < wt.n) tn = wt.t[tile + 2 * nw];
             cp_async_wait_prior();  // this tile's copies
             __syncwarp();
-            work(b.kend, tc.z, b.seg, b.cell, b.oth, tc.x, tc.y, tc.z);
+            work(b.kend, tc.z, b.seg, b.oth, tc.x, tc.y, tc.z);
             __syncwarp();
         }
         cp_async_wait_all();
@@ -580,12 +573,13 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWei
 // group streams its segment's rows (contiguous in the block): with one row per cell, in chunks of
 // L rows whose small codes and weights lane i loads for row i, four rows' loads in flight;
 // otherwise cell by cell over the cell's rows.
-// NSA: the small blocks summed (S.ns_acc when the small coordinates are accumulated, else 0).
+// NSA: the small blocks summed (S.ns_acc when the small coordinates are accumulated, else 0). cell_sums
+// (when given, cells of several rows): s_c, M x R.
 template <int L, int NSA>
 __global__ void __launch_bounds__(WPB * 32, 4) k_grhs(DevStruct S, DevWeights W, const u32* __restrict__ segs,
                                                       u32 nsegs, const double* __restrict__ rows, int R, int j0,
                                                       int Rc, double* __restrict__ b1, double* __restrict__ cta_part,
-                                                      double* __restrict__ cta_small) {
+                                                      double* __restrict__ cta_small, double* __restrict__ cell_sums) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int G = 32 / L;
     constexpr int U = 4;  // rows whose loads are in flight together (two columns each)
@@ -666,6 +660,11 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_grhs(DevStruct S, DevWeights W,
                         qa += v0 * a0;
                         qb += v1 * a1;
                     }
+                    if (cell_sums) {
+                        double* o = cell_sums + size_t(cb + i) * Ru + j0 + j;
+                        if (on0) o[0] = s0;
+                        if (on1) o[L] = s1;
+                    }
                     sum0 += s0;
                     sum1 += s1;
 #pragma unroll
@@ -726,20 +725,23 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_grhs(DevStruct S, DevWeights W,
 
 // Right-hand side pass 2 on short coordinate lists (k >= ms_acc): rhs[k] = sum over the cells c
 // of k of (s_c - W_c b1_{s(c)} / n1_{s(c)}). The rows are gathered with the default cache policy:
-// a row shares its sectors with the rows of neighbouring coordinates, which nearby warps read.
+// a row shares its sectors with the rows of neighbouring coordinates, which nearby warps read. cs (when
+// given): the cells' sums s_c from pass 1, read instead of the cells' rows (5 rows a cell, 3 columns,
+// 4e6 entries: 252 -> 61 us).
 template <int RCP>
 __global__ void __launch_bounds__(WPB * 32, 4) k_wpull_rhs(DevStruct S, DevWeights W, WarpTiles wt,
                                                            const double* __restrict__ rows,
                                                            const double* __restrict__ b1, int R, int j0, int Rc,
-                                                           double* __restrict__ Y) {
+                                                           double* __restrict__ Y, const double* __restrict__ cs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using L_t = Lanes<RCP>;
     constexpr int G = L_t::G;
     const PullStage st = pull_stage_at(smem_raw + size_t(wid_in_cta()) * pull_bytes());
     const L_t L(Rc);
     const u32 Ru = u32(R);
-    const bool trivial = S.cell_row == nullptr;
-    const double* vj = rows + j0 + L.j;
+    const bool trivial = cs || S.cell_row == nullptr;  // one value a cell
+    const double* vj = (cs ? cs : rows) + j0 + L.j;
+    const double* wr = cs ? nullptr : W.w_rows;
     const double* bj = b1 + j0 + L.j;
     const u32 wid = blockIdx.x * WPB + wid_in_cta(), nw = gridDim.x * WPB;
     uint4 tb = wid < wt.n ? wt.t[wid] : make_uint4(0, 0, 0, 0);
@@ -756,7 +758,7 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_wpull_rhs(DevStruct S, DevWeigh
                 for (u32 i = ib; i < ie; i += step) {
                     const u32 c = st.cell[i], s = st.seg[i];
                     const double x = __ldg(vj + size_t(c) * Ru);
-                    const double sc = W.w_rows ? W.w_rows[c] * x : x;
+                    const double sc = wr ? wr[c] * x : x;
                     acc += sc - cellw(W, c) * __ldcg(bj + size_t(s) * Ru) * W.n1inv[s];
                 }
             } else {

@@ -67,6 +67,7 @@ struct DevWeights {
     const double* cell_w;  // null: every cell weight is 1
     const double* n1inv;
     const double* nr;
+    const double* pl_w;    // the cells' weights in list order (null: every cell weight is 1)
 };
 
 __device__ __forceinline__ double cellw(const DevWeights& W, u32 c) { return W.cell_w ? W.cell_w[c] : 1.0; }
@@ -138,117 +139,33 @@ __device__ __forceinline__ void zero_cta_row(T* __restrict__ cta_small, u32 len)
 }
 
 // ---------------------------------------------------------------------------------------------
-// Operator pass 1 (operator.rs:894-948): t_s = sum_c W_c u_c / n1_s with u_c = sum_b P[coord_b(c)],
-// and the small coordinates' Y_k = sum over the cells c of k of W_c (u_c - t_s) into the CTA
-// rows of cta_small. Slices of long segments write partial W u sums (`part`). With
-// `slices_only` only the slices run (the W u partials of the residualize pass).
-template <class T>
-__global__ void __launch_bounds__(TB) k_seg_apply(DevStruct S, DevWeights W, const T* __restrict__ P, int R,
-                                                  T* __restrict__ t, T* __restrict__ part, bool slices_only,
-                                                  T* __restrict__ cta_small) {
-    __shared__ SegSmem<T> sm;
-    if (halted(S)) return;
+// The W u partials of the slices of long segments for the residualization (part, nparts x R), with
+// u_c = sum_b x[coord_b(c)]; k_fix_alpha turns them into the segments' alpha.
+__global__ void __launch_bounds__(TB) k_slice_wu(DevStruct S, DevWeights W, const double* __restrict__ x, int R,
+                                                 double* __restrict__ part) {
+    __shared__ double vals[TILE * RC_MAX];
     const TileSet& ts = S.seg;
-    const bool acc = cta_small && S.ms_acc > 0;
-    if (acc) zero_cta_row(cta_small, S.ms_acc * u32(R));
     for (u32 tile = blockIdx.x; tile < ts.n; tile += gridDim.x) {
-        const u32 s0 = ts.k0[tile], s1 = ts.k1[tile], c0 = ts.e0[tile], c1 = ts.e1[tile];
+        const u32 c0 = ts.e0[tile], c1 = ts.e1[tile];
         const int pslot = ts.part[tile];
-        if (slices_only && pslot < 0) continue;
-        __syncthreads();
-        if (acc && pslot < 0) seg_maps(S, s0, s1, c0, c1, sm.cellseg, sm.scode);
+        if (pslot < 0) continue;
         for (int j0 = 0; j0 < R; j0 += RC_MAX) {
             const ColMap cm = colmap(R, j0);
             if (cm.on) {
 #pragma unroll 4
                 for (u32 c = c0 + cm.slot; c < c1; c += cm.nslot) {
-                    T u = T(0);
-                    for (u32 b = 0; b < S.nb; b++) u += P[size_t(__ldcs(S.coord + size_t(b) * S.M + c)) * R + j0 + cm.col];
-                    sm.vals[(c - c0) * cm.Rc + cm.col] = T(cellw(W, c)) * u;
+                    double u = 0.0;
+                    for (u32 b = 0; b < S.nb; b++) u += x[size_t(__ldcs(S.coord + size_t(b) * S.M + c)) * R + j0 + cm.col];
+                    vals[(c - c0) * cm.Rc + cm.col] = cellw(W, c) * u;
                 }
             }
             __syncthreads();
-            const u32 nk = (s1 - s0) * u32(cm.Rc);
-            for (u32 idx = threadIdx.x; idx < nk; idx += TB) {
-                const u32 s = s0 + idx / cm.Rc;
-                const int col = int(idx % cm.Rc);
-                const u32 a = max(S.seg_off[s], c0), b = min(S.seg_off[s + 1], c1);
-                T sum = T(0);
-                for (u32 c = a; c < b; c++) sum += sm.vals[(c - c0) * cm.Rc + col];
-                if (pslot < 0) {
-                    const T ts_ = sum * T(W.n1inv[s]);
-                    t[size_t(s) * R + j0 + col] = ts_;
-                    sm.sval[(s - s0) * cm.Rc + col] = ts_;
-                } else {
-                    part[size_t(pslot) * R + j0 + col] = sum;
-                }
-            }
-            if (acc && pslot < 0) {
-                __syncthreads();
-                // z_c = W_c (u_c - t_s)
-                for (u32 i = threadIdx.x; i < (c1 - c0) * u32(cm.Rc); i += TB) {
-                    const u32 c = i / cm.Rc;
-                    const int col = int(i % cm.Rc);
-                    sm.vals[i] -= T(cellw(W, c0 + c)) * sm.sval[sm.cellseg[c] * cm.Rc + col];
-                }
-                __syncthreads();
-                small_accumulate(S, sm, c1 - c0, cm, j0, R, cta_small);
+            if (int(threadIdx.x) < cm.Rc) {
+                double sum = 0.0;
+                for (u32 c = 0; c < c1 - c0; c++) sum += vals[c * cm.Rc + threadIdx.x];
+                part[size_t(pslot) * R + j0 + threadIdx.x] = sum;
             }
             __syncthreads();
-        }
-    }
-}
-
-// Sum over the slots of a CTA of red[slot * Rc + col] into red[col] (slot 0), by a pairwise tree
-// over the slot indices: the same order every call. Every thread of the CTA calls it.
-template <class T>
-__device__ __forceinline__ void slot_tree(T* red, const ColMap& cm) {
-    for (int s = 1; s < cm.nslot; s *= 2) {
-        __syncthreads();
-        if (cm.on && cm.slot % (2 * s) == 0 && cm.slot + s < cm.nslot)
-            red[cm.slot * cm.Rc + cm.col] += red[(cm.slot + s) * cm.Rc + cm.col];
-    }
-    __syncthreads();
-}
-
-// Operator pass 2: Y[k] = nr_k P[k] + sum over the cells c of k of W_c (sum_{other b} P - t_{s(c)})
-// for the pulled coordinates. A tile holds whole lists or a slice of one long list (its partial
-// goes to k_fix); per list, thread (slot, column) sums the entries slot, slot + nslot, ... in a
-// register and the slots are combined by slot_tree.
-template <class T>
-__global__ void __launch_bounds__(TB) k_pull_apply(DevStruct S, DevWeights W, const T* __restrict__ P,
-                                                   const T* __restrict__ t, int R, T* __restrict__ Y,
-                                                   T* __restrict__ part) {
-    __shared__ T red[TB];
-    if (halted(S)) return;
-    const TileSet& ts = S.pull;
-    const u32 no = S.nb - 1;
-    for (u32 tile = blockIdx.x; tile < ts.n; tile += gridDim.x) {
-        const u32 k0 = ts.k0[tile], k1 = ts.k1[tile], e0 = ts.e0[tile], e1 = ts.e1[tile];
-        const int pslot = ts.part[tile];
-        for (int j0 = 0; j0 < R; j0 += RC_MAX) {
-            const ColMap cm = colmap(R, j0);
-            for (u32 k = k0; k < k1; k++) {
-                const u32 a = max(S.pl_off[k], e0), b = min(S.pl_off[k + 1], e1);
-                T acc = T(0);
-                if (cm.on) {
-#pragma unroll 4
-                    for (u32 e = a + cm.slot; e < b; e += cm.nslot) {
-                        T u = -__ldcg(t + size_t(__ldcs(S.pl_seg + e)) * R + j0 + cm.col);
-                        for (u32 o = 0; o < no; o++)
-                            u += P[size_t(__ldcs(S.pl_other + size_t(e) * no + o)) * R + j0 + cm.col];
-                        acc += W.cell_w ? T(W.cell_w[__ldcs(S.pl_cell + e)]) * u : u;
-                    }
-                    red[cm.slot * cm.Rc + cm.col] = acc;
-                }
-                slot_tree(red, cm);
-                if (cm.on && cm.slot == 0) {
-                    const size_t o = size_t(k) * R + j0 + cm.col;
-                    if (pslot < 0) Y[o] = T(W.nr[k]) * P[o] + red[cm.col];
-                    else part[size_t(pslot) * R + j0 + cm.col] = red[cm.col];
-                }
-                __syncthreads();
-            }
         }
     }
 }
@@ -313,7 +230,8 @@ __global__ void k_small_reduce(const T* __restrict__ a, int na, const T* __restr
 // coordinates' rhs_k = sum over the cells c of k of (s_c - W_c b1_s / n1_s) into cta_small.
 __global__ void __launch_bounds__(TB) k_seg_rhs(DevStruct S, DevWeights W, const double* __restrict__ rows, int R,
                                                 double* __restrict__ b1, double* __restrict__ part,
-                                                double* __restrict__ cta_part, double* __restrict__ cta_small) {
+                                                double* __restrict__ cta_part, double* __restrict__ cta_small,
+                                                double* __restrict__ cs) {
     __shared__ SegSmem<double> sm;
     __shared__ double red[2 * TB];
     const TileSet& ts = S.seg;
@@ -341,6 +259,7 @@ __global__ void __launch_bounds__(TB) k_seg_rhs(DevStruct S, DevWeights W, const
                         q += wv * v;
                     }
                     a1 += a;
+                    if (cs) cs[size_t(c) * R + j0 + cm.col] = a;
                     sm.vals[(c - c0) * cm.Rc + cm.col] = a;
                 }
             }
@@ -417,46 +336,6 @@ __global__ void __launch_bounds__(TB) k_rhs_small_slices(DevStruct S, DevWeights
     }
 }
 
-// Right-hand side pass 2: rhs[k] = sum over the cells c of k of (s_c - W_c b1_{s(c)} / n1_{s(c)})
-// for the pulled coordinates, with the tiles and the slot sums of k_pull_apply.
-__global__ void __launch_bounds__(TB) k_pull_rhs(DevStruct S, DevWeights W, const double* __restrict__ rows,
-                                                 const double* __restrict__ b1, int R, double* __restrict__ Y,
-                                                 double* __restrict__ part) {
-    __shared__ double red[TB];
-    const TileSet& ts = S.pull;
-    for (u32 tile = blockIdx.x; tile < ts.n; tile += gridDim.x) {
-        const u32 k0 = ts.k0[tile], k1 = ts.k1[tile], e0 = ts.e0[tile], e1 = ts.e1[tile];
-        const int pslot = ts.part[tile];
-        for (int j0 = 0; j0 < R; j0 += RC_MAX) {
-            const ColMap cm = colmap(R, j0);
-            for (u32 k = k0; k < k1; k++) {
-                const u32 a = max(S.pl_off[k], e0), b = min(S.pl_off[k + 1], e1);
-                double acc = 0.0;
-                if (cm.on) {
-#pragma unroll 4
-                    for (u32 e = a + cm.slot; e < b; e += cm.nslot) {
-                        const u32 c = __ldcs(S.pl_cell + e), s = __ldcs(S.pl_seg + e);
-                        double sc = 0.0;
-                        const u32 r1 = row1_of(S, c);
-                        for (u32 row = row0_of(S, c); row < r1; row++) {
-                            const double v = __ldcs(rows + size_t(row) * R + j0 + cm.col);
-                            sc += W.w_rows ? W.w_rows[row] * v : v;
-                        }
-                        acc += sc - cellw(W, c) * __ldcg(b1 + size_t(s) * R + j0 + cm.col) * W.n1inv[s];
-                    }
-                    red[cm.slot * cm.Rc + cm.col] = acc;
-                }
-                slot_tree(red, cm);
-                if (cm.on && cm.slot == 0) {
-                    if (pslot < 0) Y[size_t(k) * R + j0 + cm.col] = red[cm.col];
-                    else part[size_t(pslot) * R + j0 + cm.col] = red[cm.col];
-                }
-                __syncthreads();
-            }
-        }
-    }
-}
-
 // sum_s b1_s^2 / n1_s per column (solve.rs:648-658) as per-CTA partials (grid x R).
 __global__ void __launch_bounds__(TB) k_b1sq(u32 g1, const double* __restrict__ b1, const double* __restrict__ n1inv,
                                              int R, double* __restrict__ cta_part) {
@@ -491,90 +370,6 @@ __global__ void __launch_bounds__(TB) k_b1sq(u32 g1, const double* __restrict__ 
             cta_part[size_t(blockIdx.x) * R + j0 + threadIdx.x] = s;
         }
         __syncthreads();
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
-// Residualization (operator.rs:1107-1179): alpha_s = (b1_s - sum_c W_c u_c) / n1_s with
-// u_c = sum_b x[coord_b(c)], then every row of cell c loses alpha_s + u_c. Slices of long
-// segments take alpha from `along` (fix index x R), filled beforehand by k_seg_apply on x and
-// k_fix_alpha. With one row per cell, each thread's row elements are loaded first so their
-// latency overlaps the gathers of x.
-constexpr int PF = TILE / (TB / RC_MAX);  // row elements per thread and chunk (one row per cell)
-
-__global__ void __launch_bounds__(TB, 4) k_residualize(DevStruct S, DevWeights W, double* __restrict__ rows, int R,
-                                                    const double* __restrict__ x, const double* __restrict__ b1,
-                                                    const double* __restrict__ along, double* __restrict__ alpha) {
-    __shared__ double vals[TILE * RC_MAX];
-    __shared__ double aseg[TILE * RC_MAX];
-    __shared__ u32 cellseg[TILE];
-    const TileSet& ts = S.seg;
-    for (u32 tile = blockIdx.x; tile < ts.n; tile += gridDim.x) {
-        const u32 s0 = ts.k0[tile], s1 = ts.k1[tile], c0 = ts.e0[tile], c1 = ts.e1[tile];
-        const int fidx = ts.fixidx[tile];
-        __syncthreads();
-        for (u32 s = s0 + threadIdx.x; s < s1; s += TB) {
-            const u32 a = max(S.seg_off[s], c0), b = min(S.seg_off[s + 1], c1);
-            for (u32 c = a; c < b; c++) cellseg[c - c0] = s - s0;
-        }
-        for (int j0 = 0; j0 < R; j0 += RC_MAX) {
-            const ColMap cm = colmap(R, j0);
-            double rv[PF];
-            const bool pre = S.cell_row == nullptr;
-            if (pre && cm.on) {
-#pragma unroll
-                for (int k = 0; k < PF; k++) {
-                    const u32 c = c0 + cm.slot + u32(k * cm.nslot);
-                    rv[k] = c < c1 ? __ldcs(rows + size_t(c) * R + j0 + cm.col) : 0.0;
-                }
-            }
-            if (cm.on) {
-#pragma unroll 4
-                for (u32 c = c0 + cm.slot; c < c1; c += cm.nslot) {
-                    double u = 0.0;
-                    for (u32 b = 0; b < S.nb; b++) u += x[size_t(__ldcs(S.coord + size_t(b) * S.M + c)) * R + j0 + cm.col];
-                    vals[(c - c0) * cm.Rc + cm.col] = u;
-                }
-            }
-            __syncthreads();
-            const u32 nk = (s1 - s0) * u32(cm.Rc);
-            for (u32 idx = threadIdx.x; idx < nk; idx += TB) {
-                const u32 s = s0 + idx / cm.Rc;
-                const int col = int(idx % cm.Rc);
-                double a;
-                if (fidx < 0) {
-                    const u32 ca = S.seg_off[s], cb = S.seg_off[s + 1];
-                    double acc = 0.0;
-                    for (u32 c = ca; c < cb; c++) acc += cellw(W, c) * vals[(c - c0) * cm.Rc + col];
-                    a = (b1[size_t(s) * R + j0 + col] - acc) * W.n1inv[s];
-                    if (alpha) alpha[size_t(s) * R + j0 + col] = a;
-                } else {
-                    a = along[size_t(fidx) * R + j0 + col];
-                }
-                aseg[(s - s0) * cm.Rc + col] = a;
-            }
-            __syncthreads();
-            if (cm.on) {
-                if (pre) {
-#pragma unroll
-                    for (int k = 0; k < PF; k++) {
-                        const u32 c = c0 + cm.slot + u32(k * cm.nslot);
-                        if (c < c1) {
-                            const double f = aseg[cellseg[c - c0] * cm.Rc + cm.col] + vals[(c - c0) * cm.Rc + cm.col];
-                            __stcs(rows + size_t(c) * R + j0 + cm.col, rv[k] - f);
-                        }
-                    }
-                } else {
-#pragma unroll 4
-                    for (u32 c = c0 + cm.slot; c < c1; c += cm.nslot) {
-                        const double f = aseg[cellseg[c - c0] * cm.Rc + cm.col] + vals[(c - c0) * cm.Rc + cm.col];
-                        const u32 r1 = row1_of(S, c);
-                        for (u32 row = row0_of(S, c); row < r1; row++) rows[size_t(row) * R + j0 + cm.col] -= f;
-                    }
-                }
-            }
-            __syncthreads();
-        }
     }
 }
 

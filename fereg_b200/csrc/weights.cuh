@@ -38,6 +38,14 @@ __global__ void k_gather_rows_f64(const double* __restrict__ in, const u32* __re
         out[r] = in[pi[r]];
 }
 
+// pw[e] = the weight of list entry e's cell: the list passes of the operator then read the weights in
+// order (4e6 entries, 4 columns: 67 -> 53 us an apply with the direct reads they allow, 19 us per weight state).
+__global__ void k_list_weights(const double* __restrict__ cw, const u32* __restrict__ pl_cell, size_t E,
+                               double* __restrict__ pw) {
+    for (size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x; e < E; e += size_t(gridDim.x) * blockDim.x)
+        pw[e] = cw[pl_cell[e]];
+}
+
 // W_c = the number of rows of cell c (unit row weights).
 __global__ void k_cell_counts(const u32* __restrict__ cell_row, u32 M, double* __restrict__ cw) {
     for (u32 c = blockIdx.x * blockDim.x + threadIdx.x; c < M; c += gridDim.x * blockDim.x)
@@ -132,29 +140,43 @@ __global__ void k_coord_combine(const u32* __restrict__ list_chunk_off, u32 m, c
                                 uint8_t* __restrict__ red, double* __restrict__ inv_diag) {
     constexpr u32 NONE = 0xffffffffu;
     for (u32 k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-        double n_acc = 0.0, dq = 0.0, X = 0.0, Q = 0.0;
+        double n_acc = 0.0, dq = 0.0, X = 0.0, Q = 0.0, csn = 0.0;  // csn: 1 / n1 of segment cs
         u32 cs = NONE;
-        for (u32 c = list_chunk_off[k]; c < list_chunk_off[k + 1]; c++) {
-            const CwChunk h = ch[c];
-            n_acc += h.nr;
-            dq += h.dq;
-            if (h.sf == cs) {
-                X += h.xf;
-                Q += h.xf * h.xf;
-            } else {
-                if (cs != NONE) dq += (X * X - Q) * n1inv[cs];
-                cs = h.sf;
-                X = h.xf;
-                Q = h.xf * h.xf;
-            }
-            if (h.sl != h.sf) {  // the chunk holds more runs: the carried run ends at its first
-                dq += (X * X - Q) * n1inv[cs];
-                cs = h.sl;
-                X = h.xl;
-                Q = h.xl * h.xl;
+        const u32 cb = list_chunk_off[k], ce = list_chunk_off[k + 1];
+        for (u32 c0 = cb; c0 < ce; c0 += 4) {
+            CwChunk hh[4];  // four chunks' loads in flight (a list of 117 chunks took 83 us one by one)
+            double ni[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (c0 + u < ce) hh[u] = ch[c0 + u];
+#pragma unroll
+            for (int u = 0; u < 4; u++) ni[u] = c0 + u < ce ? n1inv[hh[u].sf] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (c0 + u >= ce) break;
+                const CwChunk& h = hh[u];
+                n_acc += h.nr;
+                dq += h.dq;
+                if (h.sf == cs) {
+                    X += h.xf;
+                    Q += h.xf * h.xf;
+                } else {
+                    if (cs != NONE) dq += (X * X - Q) * csn;
+                    cs = h.sf;
+                    csn = ni[u];
+                    X = h.xf;
+                    Q = h.xf * h.xf;
+                }
+                if (h.sl != h.sf) {  // the chunk holds more runs: the carried run ends at its first
+                    dq += (X * X - Q) * csn;
+                    cs = h.sl;
+                    csn = n1inv[h.sl];
+                    X = h.xl;
+                    Q = h.xl * h.xl;
+                }
             }
         }
-        if (cs != NONE) dq += (X * X - Q) * n1inv[cs];
+        if (cs != NONE) dq += (X * X - Q) * csn;
         const double dg = n_acc - dq;
         const bool r = dg <= 1e-12 * n_acc;
         nr[k] = n_acc;
