@@ -178,6 +178,8 @@ def _setup(L):
     L.fereg_drop_singletons.argtypes = [C.POINTER(u32p), u32p, C.c_int, C.c_size_t, f64p, f64p, C.c_int, C.c_int,
                                         u8p, u64p, u64p]
     L.fereg_restrict.argtypes = [u32p, C.c_uint32, u8p, C.c_size_t, u32p, u32p, u64p]
+    L.fereg_prepare.argtypes = [C.POINTER(f64p), C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.c_int, C.c_size_t,
+                                f64p, f64p, C.c_int, C.c_int, u8p, C.POINTER(u32p), u32p, u64p, u64p, u64p]
     L.fereg_server_create.argtypes = [C.POINTER(ServerConfig), C.POINTER(P)]
     L.fereg_server_submit.argtypes = [P, C.POINTER(Request), C.POINTER(C.c_uint64)]
     L.fereg_server_wait.argtypes = [P, C.c_uint64, C.POINTER(RequestResult), C.c_char_p, C.c_size_t]
@@ -779,6 +781,33 @@ def prepare(factors, absorb, fw=None, y=None, family=None, singletons=True):
     singletons (and, with a GLM family and its outcome, fe-separated rows) cyclically, and
     renumber each term's codes over the kept rows. Returns alive, the drop counts and the kept
     terms as (codes, levels)."""
+    cols = [np.ascontiguousarray(f, dtype=np.float64) for f in factors]
+    n = len(cols[0])
+    parts = [[int(i) if i >= 0 else len(cols) + int(i) for i in t] for t in absorb]
+    if (not parts or n == 0 or any(len(c) != n for c in cols)
+            or any(not t or any(not 0 <= i < len(cols) for i in t) for t in parts)):
+        return _prepare_steps(cols, absorb, fw, y, family, singletons)
+    off = np.cumsum([0] + [len(t) for t in parts]).astype(np.int32)
+    flat = np.array([i for t in parts for i in t], dtype=np.int32)
+    ip = C.POINTER(C.c_int)
+    colp = (f64p * len(cols))(*[_p(c, f64p) for c in cols])
+    codes = [np.empty(n, dtype=np.uint32) for _ in parts]
+    codep = (u32p * len(parts))(*[_p(c, u32p) for c in codes])
+    levels = np.zeros(len(parts), dtype=np.uint32)
+    alive = np.empty(n, dtype=np.uint8)
+    fwa = None if fw is None else np.ascontiguousarray(fw, dtype=np.float64)
+    ya = None if y is None else np.ascontiguousarray(y, dtype=np.float64)
+    kept, s, f = C.c_uint64(), C.c_uint64(), C.c_uint64()
+    _check(lib().fereg_prepare(colp, len(cols), _p(off, ip), _p(flat, ip), len(parts), n, _p(fwa, f64p), _p(ya, f64p),
+                               FAMILY_CODE[family], int(singletons), _p(alive, u8p), codep, _p(levels, u32p),
+                               C.byref(kept), C.byref(s), C.byref(f)))
+    k = int(kept.value)
+    return dict(alive=alive.view(bool), num_singletons=int(s.value), fe_separated=int(f.value),
+                terms=[(c[:k], int(g)) for c, g in zip(codes, levels)])
+
+
+def _prepare_steps(factors, absorb, fw, y, family, singletons):
+    """prepare() by the steps' own calls (no terms, no rows, columns or terms that these refuse)."""
     fac = [factorize(f) for f in factors]
     terms = [combine([fac[i][0] for i in t], [fac[i][1] for i in t]) for t in absorb]
     if terms:

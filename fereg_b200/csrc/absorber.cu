@@ -357,8 +357,23 @@ struct Scratch {
     }
 };
 
+cudaStream_t GpuAbsorber::make_stream(const Ctx& ctx) {
+    cudaStream_t st = nullptr;
+    if (ctx.priority_level < 0) {
+        CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    } else {
+        int least = 0, greatest = 0;
+        CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        const int prio = std::min(std::max(greatest, least - 1), greatest + ctx.priority_level);
+        CK(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, prio));
+    }
+    return st;
+}
+
+const u32* GpuAbsorber::row_order_device() const { return d_->pi.p; }
+
 GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector<u32>& g, const double* w, size_t n,
-                         const Ctx& ctx, const std::vector<const u32*>* dev_codes)
+                         const Ctx& ctx, const std::vector<const u32*>* dev_codes, cudaStream_t own)
     : g_(g), ctx_(ctx) {
     check_codes_host(codes, g, n);
     if (w) check_weights_host(w, n);
@@ -366,14 +381,7 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
     norm_fe1_ = fe1_index(g);
     ctx_.check();
     keep_pool_mapped();
-    if (ctx_.priority_level < 0) {
-        CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    } else {
-        int least = 0, greatest = 0;
-        CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        const int prio = std::min(std::max(greatest, least - 1), greatest + ctx_.priority_level);
-        CK(cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, prio));
-    }
+    stream_ = own ? own : make_stream(ctx_);
     AllocScope alloc_scope(stream_);
     d_ = std::make_unique<Scratch>();
     CK(cudaHostAlloc(&d_->h_nactive, 16 * sizeof(int), cudaHostAllocDefault));

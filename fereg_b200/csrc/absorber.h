@@ -59,6 +59,8 @@ class DeviceAbsorber {
     // Values term_values writes: sum over terms of levels x (intercept + slopes).
     virtual size_t term_values_len() const = 0;
     virtual const std::vector<u32>& row_order() const = 0;
+    // row_order() in device memory, or null where the absorber keeps it on the host only
+    virtual const u32* row_order_device() const { return nullptr; }
     virtual bool weights(double* out) const = 0;
     virtual void set_weights(const double* w_rows) = 0;
     virtual void set_weights_device(const double* w_rows_dev) = 0;
@@ -98,9 +100,12 @@ class GpuAbsorber : public DeviceAbsorber {
    public:
     // `codes[q]` are the kept-order codes of term q (< g[q]); `w` kept-order weights or null.
     // The cell structure is built on the device; `dev_codes`, when given, are device copies of
-    // `codes` (the caller's session keeps them), otherwise the codes are uploaded for the build.
+    // `codes` (the caller's session keeps them, queued on `own`), otherwise the codes are uploaded for
+    // the build. `own`: a stream of make_stream() that the absorber works on and owns from its
+    // construction on (null: it makes one).
+    static cudaStream_t make_stream(const Ctx& ctx);
     GpuAbsorber(const std::vector<const u32*>& codes, const std::vector<u32>& g, const double* w, size_t n, const Ctx& ctx,
-                const std::vector<const u32*>* dev_codes = nullptr);
+                const std::vector<const u32*>* dev_codes = nullptr, cudaStream_t own = nullptr);
     ~GpuAbsorber() override;
 
     size_t n() const override { return hs_.n; }
@@ -109,6 +114,7 @@ class GpuAbsorber : public DeviceAbsorber {
     size_t coefs_len() const override { return hs_.m + hs_.g1; }
     size_t term_values_len() const override;
     const std::vector<u32>& row_order() const override { return hs_.pi; }
+    const u32* row_order_device() const override;
     const HostStructure& structure() const { return hs_; }
     // Row-order weights (false: all ones).
     bool weights(double* out) const override;

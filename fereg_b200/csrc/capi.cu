@@ -784,6 +784,35 @@ int fereg_restrict(const uint32_t* codes, uint32_t g, const uint8_t* alive, size
     });
 }
 
+int fereg_prepare(const double* const* factors, int nf, const int* term_off, const int* term_fac, int nterms, size_t n,
+                  const double* fw, const double* y, int family, int singletons, uint8_t* alive, uint32_t* const* codes,
+                  uint32_t* levels, uint64_t* kept, uint64_t* dropped_singletons, uint64_t* dropped_separated) {
+    return guard([&] {
+        if (!factors || nf < 1 || !term_off || !term_fac || nterms < 1 || n == 0 || !alive || !codes || !levels || !kept)
+            throw Error(RC_INVALID_INPUT, "fereg_prepare: NULL or empty argument");
+        if (n > size_t(0xffffffffu)) throw Error(RC_INVALID_INPUT, "fereg_prepare: more than 2^32 - 1 rows");
+        if (family < 0 || family > 2 || (family && !y))
+            throw Error(RC_INVALID_INPUT, "fereg_prepare: family 1 / 2 needs the outcome");
+        for (int f = 0; f < nf; f++)
+            if (!factors[f]) throw Error(RC_INVALID_INPUT, "fereg_prepare: NULL factor");
+        std::vector<std::vector<int>> terms(static_cast<size_t>(nterms));
+        std::vector<u32*> out(codes, codes + nterms);
+        for (int t = 0; t < nterms; t++) {
+            if (!codes[t] || term_off[t + 1] <= term_off[t]) throw Error(RC_INVALID_INPUT, "fereg_prepare: empty term");
+            for (int i = term_off[t]; i < term_off[t + 1]; i++) {
+                if (term_fac[i] < 0 || term_fac[i] >= nf) throw Error(RC_INVALID_INPUT, "fereg_prepare: factor index out of range");
+                terms[size_t(t)].push_back(term_fac[i]);
+            }
+        }
+        u64 k = 0;
+        const DropCounts d = prep_sample(std::vector<const double*>(factors, factors + nf), terms, n, fw, y, family,
+                                         singletons != 0, alive, out, levels, &k);
+        *kept = k;
+        if (dropped_singletons) *dropped_singletons = d.singletons;
+        if (dropped_separated) *dropped_separated = d.separated;
+    });
+}
+
 int fereg_structure_digest(const uint32_t* const* codes, const uint32_t* g, int nterms, size_t n, uint64_t* out) {
     return guard([&] {
         if (!codes || !g || nterms < 1 || !out) throw Error(RC_INVALID_INPUT, "fereg_structure_digest: NULL argument");

@@ -193,4 +193,41 @@ void build_structure_device(const std::vector<const u32*>& dcodes, const std::ve
     CK(cudaStreamSynchronize(st));
 }
 
+void check_codes_device(const u32* codes, size_t n, u32 g, const char* what, cudaStream_t st) {
+    if (!n) return;
+    DBuf<int> flag;
+    flag.alloc(1);
+    CK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
+    k_ds_check<<<ds_grid(n), DS_TB, 0, st>>>(codes, n, g, flag.p);
+    int bad = 0;
+    CK(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (bad) throw Error(RC_INVALID_INPUT, what);
+}
+
+void group_rows_device(const u32* codes, const u32* pi, size_t n, u32 G, u32* perm, u32* coff, cudaStream_t st) {
+    if (!n) {
+        CK(cudaMemsetAsync(coff, 0, (size_t(G) + 1) * sizeof(u32), st));
+        return;
+    }
+    check_codes_device(codes, n, G, "cluster code out of range of its level count", st);
+    DBuf<u64> k1, k2;
+    DBuf<u32> v1, v2, cnt;
+    k1.alloc(n);
+    k2.alloc(n);
+    v1.alloc(n);
+    v2.alloc(n);
+    cnt.alloc(size_t(G) + 1);
+    k_ds_gather_key<<<ds_grid(n), DS_TB, 0, st>>>(codes, pi, n, k1.p);
+    k_ds_iota<<<ds_grid(n), DS_TB, 0, st>>>(v1.p, n);
+    u64* keys = k1.p;
+    u32* vals = v1.p;
+    device_sort_pairs(keys, vals, k2.p, v2.p, n, bits_for(G - 1), st);
+    CK(cudaMemcpyAsync(perm, vals, n * sizeof(u32), cudaMemcpyDeviceToDevice, st));
+    CK(cudaMemsetAsync(cnt.p, 0, (size_t(G) + 1) * sizeof(u32), st));
+    k_ds_count<<<ds_grid(n), DS_TB, 0, st>>>(codes, n, cnt.p);
+    device_excl_scan(cnt.p, size_t(G) + 1, coff, st);
+    CK(cudaGetLastError());
+}
+
 }  // namespace fereg

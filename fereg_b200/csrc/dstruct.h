@@ -30,4 +30,12 @@ void build_structure_device(const std::vector<const u32*>& dcodes, const std::ve
                             DeviceStructure& ds, std::vector<u32>& pl_off_host, std::vector<u32>& pl_seg_host,
                             cudaStream_t st);
 
+// Throws 198 when one of n device codes is not below g.
+void check_codes_device(const u32* codes, size_t n, u32 g, const char* what, cudaStream_t st);
+
+// The rows grouped by a kept-order code (device arrays, n codes below G, checked here): perm (n) holds
+// the rows r of code 0, then 1, ... in row order, coff (G + 1) the groups' first positions; row r
+// is kept observation pi[r].
+void group_rows_device(const u32* codes, const u32* pi, size_t n, u32 G, u32* perm, u32* coff, cudaStream_t st);
+
 }  // namespace fereg

@@ -22,6 +22,16 @@ struct DropCounts {
 // (1 Poisson, 2 logit) and its outcome y, the `fe` rule drops levels without variation.
 DropCounts prep_drop(const std::vector<const u32*>& codes, const std::vector<u32>& g, size_t n, const double* fw,
                      const double* y, int family, bool singletons, uint8_t* alive);
+// Session::prepare's steps in one call (n > 0 rows, at least one term): the factors factorized, each
+// term the interaction of its factors, the drops, and the terms' codes of the kept rows renumbered
+// (codes_out[t]: room for n; levels[t]); *kept: the kept rows.
+DropCounts prep_sample(const std::vector<const double*>& factors, const std::vector<std::vector<int>>& terms, size_t n,
+                       const double* fw, const double* y, int family, bool singletons, uint8_t* alive,
+                       const std::vector<u32*>& codes_out, u32* levels, u64* kept);
+// factor.rs:255 combine of device columns (n > 0, every code below its level count) into codes
+// (device); returns the level count.
+u32 device_combine(const std::vector<const u32*>& parts, const std::vector<u32>& nl, size_t n, u32* codes,
+                   cudaStream_t st);
 // Exclusive scan of n device u32 values into out (device) on `st`; returns the total (the host
 // waits for it).
 u32 device_excl_scan(const u32* in, size_t n, u32* out, cudaStream_t st);

@@ -15,7 +15,9 @@
 #include <numeric>
 #include <sstream>
 
+#include "dstruct.h"
 #include "linalg.h"
+#include "prep.h"
 #include "session.h"
 #include "slopes.h"
 #include "boot.cuh"
@@ -104,8 +106,6 @@ GpuSession::GpuSession(const std::vector<const u32*>& codes, const std::vector<u
     }
     tg_ = tg;
     cg_ = cl_g;
-    for (size_t q = 0; q < tptr.size(); q++) tcodes_.emplace_back(tptr[q], tptr[q] + n);
-    for (size_t c = 0; c < cl_codes.size(); c++) ccodes_.emplace_back(cl_codes[c], cl_codes[c] + n);
     if (w) {
         wk_.assign(w, w + n);
         sumw_ = 0.0;
@@ -113,17 +113,8 @@ GpuSession::GpuSession(const std::vector<const u32*>& codes, const std::vector<u
     } else {
         sumw_ = double(n);
     }
-    // the term codes on the device: the session's copies, from which the absorber also builds its
-    // cell structure
     d_ = std::make_unique<SessionDev>();
     SessionDev& d = *d_;
-    std::vector<const u32*> dcodes;
-    for (auto& c : tcodes_) {
-        d.tcodes.emplace_back();
-        d.tcodes.back().upload(c, nullptr);
-        dcodes.push_back(d.tcodes.back().p);
-    }
-    CK(cudaStreamSynchronize(nullptr));
     bool slopes = false;
     for (size_t q = 0; q < tptr.size(); q++) {
         const bool icpt = shapes ? (*shapes)[q].intercept : true;
@@ -145,54 +136,87 @@ GpuSession::GpuSession(const std::vector<const u32*>& codes, const std::vector<u
             st[q].slopes = (*shapes)[q].slopes;
         }
         ab_ = std::make_unique<GpuSlopeSolver>(st, w, n, ctx);
+        AllocScope alloc_scope(ab_->stream());
+        for (const u32* c : tptr) {
+            d.tcodes.emplace_back();
+            d.tcodes.back().upload(c, n, ab_->stream());
+        }
     } else {
-        ab_ = std::make_unique<GpuAbsorber>(tptr, tg, w, n, ctx, &dcodes);
+        // the term codes go up once, in the order of the absorber's stream: the session's copies, from
+        // which the absorber also builds its cell structure
+        const cudaStream_t own = GpuAbsorber::make_stream(ctx);
+        try {
+            AllocScope alloc_scope(own);
+            std::vector<const u32*> dcodes;
+            for (const u32* c : tptr) {
+                d.tcodes.emplace_back();
+                d.tcodes.back().upload(c, n, own);
+                dcodes.push_back(d.tcodes.back().p);
+            }
+            ab_ = std::make_unique<GpuAbsorber>(tptr, tg, w, n, ctx, &dcodes, own);
+        } catch (...) {
+            d.tcodes.clear();
+            cudaStreamSynchronize(own);
+            cudaStreamDestroy(own);
+            throw;
+        }
     }
     d.st = ab_->stream();
     AllocScope alloc_scope(d.st);
-    for (auto& c : ccodes_) {
+    for (const u32* c : cl_codes) {
         d.ccodes.emplace_back();
-        d.ccodes.back().upload(c, d.st);
+        d.ccodes.back().upload(c, n, d.st);
     }
-    const std::vector<u32>& pi = ab_->row_order();
     if (w) {
-        std::vector<double> raw(n), wv(n);
-        for (size_t i = 0; i < n; i++) raw[i] = wk_[pi[i]];
         // ols.rs:77-108 Weights: aweights and pweights normalized to sum n, fweights as given
         const double f = (kind_ == 1 || kind_ == 3) ? double(n) / sumw_ : 1.0;
-        for (size_t i = 0; i < n; i++) wv[i] = raw[i] * f;
-        d.w_raw.upload(raw, d.st);
-        d.wv.upload(wv, d.st);
+        DBuf<double> wk;
+        wk.upload(w, n, d.st);
+        d.w_raw.alloc(n);
+        d.wv.alloc(n);
+        k_row_weights<<<blocks_for(n, 256), 256, 0, d.st>>>(wk.p, pi_device(), n, f, d.w_raw.p, d.wv.p);
+        CK(cudaGetLastError());
     }
     // cluster subsets (inclusion-exclusion of vcov.rs:480-560): every non-empty subset of the
     // dimensions, its rows grouped by the combined code
-    const size_t q = ccodes_.size();
+    const size_t q = cg_.size();
     for (u32 mask = 1; mask < (1u << q); mask++) {
-        std::vector<const std::vector<u32>*> dims;
+        std::vector<const u32*> dims;
         std::vector<u32> gs;
         for (size_t c = 0; c < q; c++)
             if (mask & (1u << c)) {
-                dims.push_back(&ccodes_[c]);
+                dims.push_back(d.ccodes[c].p);
                 gs.push_back(cg_[c]);
             }
-        std::vector<u32> kc;
-        u32 G = 0;
-        combine_codes(dims, gs, n, kc, G);
-        std::vector<u32> coff(size_t(G) + 1, 0);
-        for (size_t i = 0; i < n; i++) coff[kc[pi[i]] + 1]++;
-        for (u32 k = 0; k < G; k++) coff[k + 1] += coff[k];
-        std::vector<int> perm(n);
-        std::vector<u32> pos(coff.begin(), coff.end() - 1);
-        for (size_t i = 0; i < n; i++) perm[pos[kc[pi[i]]]++] = int(i);
+        // the combined code, its levels numbered in ascending order of the tuple (factor.rs:255)
+        const u32* kc = dims[0];
+        u32 G = gs[0];
+        DBuf<u32> comb;
+        if (dims.size() > 1) {
+            for (size_t i = 0; i < dims.size(); i++)
+                check_codes_device(dims[i], n, gs[i], "cluster code out of range of its level count", d.st);
+            comb.alloc(n);
+            G = device_combine(dims, gs, n, comb.p, d.st);
+            kc = comb.p;
+        }
         d.subsets.emplace_back();
         auto& s = d.subsets.back();
-        s.perm.upload(perm, d.st);
-        s.coff.upload(coff, d.st);
+        s.perm.alloc(n);
+        s.coff.alloc(size_t(G) + 1);
+        group_rows_device(kc, pi_device(), n, G, reinterpret_cast<u32*>(s.perm.p), s.coff.p, d.st);
         s.G = G;
         s.sign = dims.size() % 2 == 1 ? 1.0 : -1.0;
-        s.kc = std::move(kc);
+        s.mask = mask;
     }
     CK(cudaStreamSynchronize(d.st));
+}
+
+// The row order in device memory: the absorber's, or a copy of the host's.
+const u32* GpuSession::pi_device() {
+    if (const u32* p = ab_->row_order_device()) return p;
+    SessionDev& d = *d_;
+    if (!d.pi.p) d.pi.upload(ab_->row_order(), d.st);
+    return d.pi.p;
 }
 
 GpuSession::~GpuSession() {
@@ -380,7 +404,7 @@ GpuSession::Dof GpuSession::dof_pass(bool clusters, bool firstpair, bool want_gr
     std::vector<bool> live(ns);
     for (size_t i = 0; i < ns; i++) live[i] = icpt_term[i] >= 0;
     if (clusters && !firstpair)
-        for (size_t c = 0; c < ccodes_.size(); c++) {
+        for (size_t c = 0; c < cg_.size(); c++) {
             std::vector<size_t> at, qs;  // the live intercept slots and their terms
             for (size_t i = 0; i < ns; i++)
                 if (live[i] && !dof.slots[i].exact) {
@@ -554,12 +578,11 @@ double* GpuSession::gather_columns(const double* const* cols, size_t R) {
     if (R == 0 || R + 1 > size_t(OP_MAXM)) throw Error(RC_INVALID_INPUT, "fereg gather: 1 to 62 columns");
     for (size_t j = 0; j < R; j++)
         if (!cols[j]) throw Error(RC_INVALID_INPUT, "fereg gather: NULL column");
-    if (!d.pi.p) d.pi.upload(ab_->row_order(), st);
     d.colbuf.alloc(n * R);
     for (size_t j = 0; j < R; j++)
         CK(cudaMemcpyAsync(d.colbuf.p + j * n, cols[j], n * 8, cudaMemcpyHostToDevice, st));
     d.rows.alloc(n * R);
-    k_gather_cols<<<blocks_for(n, 256), 256, 0, st>>>(d.colbuf.p, d.pi.p, n, int(R), d.rows.p);
+    k_gather_cols<<<blocks_for(n, 256), 256, 0, st>>>(d.colbuf.p, pi_device(), n, int(R), d.rows.p);
     d.launches++;
     CK(cudaGetLastError());
     return d.rows.p;
@@ -680,7 +703,7 @@ void GpuSession::ols(double* rows_in, bool on_device, size_t nx, const OlsSpec& 
     if (vce < 0 || vce > 5) throw Error(RC_INVALID_INPUT, "fereg ols: unknown variance");
     if (vce == 5 && kind == 3) throw Error(RC_INVALID_INPUT, "pweights not allowed with option vce(hc3)");  // ols.rs:251
     const bool clustered = vce == 2 || vce == 3;
-    if (clustered && ccodes_.empty()) throw Error(RC_INVALID_INPUT, "fereg ols: cluster variance without clusters");
+    if (clustered && cg_.empty()) throw Error(RC_INVALID_INPUT, "fereg ols: cluster variance without clusters");
     if (vce == 3 && (kind == 2 || !dynamic_cast<GpuAbsorber*>(ab_.get())))
         throw Error(RC_INVALID_INPUT, "fereg ols: CRV3 needs intercept-only terms and no fweights");
     const bool has_intercept = true;  // intercept-only terms (or noabsorb) contain the constant
@@ -929,7 +952,7 @@ void GpuSession::ols(double* rows_in, bool on_device, size_t nx, const OlsSpec& 
             fit_.crv1_scale = q_cluster;
             fit_.ok = true;
             v_s = la::sandwich(bread, meat, msz, q_cluster);
-            if (ccodes_.size() > 1) la::fix_psd(v_s, msz, report_constant);
+            if (cg_.size() > 1) la::fix_psd(v_s, msz, report_constant);
         } else {
             const la::Mat meat = crv3_meat(rows, raw_h, R, kept, beta, wmean, report_constant, g);
             const double nested_adj = dof.df_a_nested > 0 ? 1.0 : 0.0;
@@ -937,7 +960,7 @@ void GpuSession::ols(double* rows_in, bool on_device, size_t nx, const OlsSpec& 
             for (size_t a = 0; a < msz; a++)
                 for (size_t b = 0; b < msz; b++)
                     v_s[a * msz + b] = q_cluster * meat[a * msz + b] * sc[a] * sc[b] / (sd_y * sd_y);
-            if (ccodes_.size() > 1) la::fix_psd(v_s, msz, report_constant);
+            if (cg_.size() > 1) la::fix_psd(v_s, msz, report_constant);
         }
     }
     d.end(ph);
@@ -998,7 +1021,7 @@ void GpuSession::ols(double* rows_in, bool on_device, size_t nx, const OlsSpec& 
     out.df_a_redundant = double(dof.df_a_redundant);
     out.df_a_nested = double(dof.df_a_nested);
     out.N_clust = clustered ? g_min : nanv();
-    out.N_clustervars = clustered ? double(ccodes_.size()) : nanv();
+    out.N_clustervars = clustered ? double(cg_.size()) : nanv();
     out.N_clust1 = clustered && !cg_.empty() ? double(cg_[0]) : nanv();
     out.N_clust2 = clustered && cg_.size() > 1 ? double(cg_[1]) : nanv();
     out.num_singletons = double(nsing_);
@@ -1094,7 +1117,7 @@ void GpuSession::iv(double* rows_in, bool on_device, size_t nx, size_t ne, size_
     const double bigN = kind == 2 ? sumw_ : double(n);
     int vce = spec.vce;
     if (vce == 0 && kind == 3) vce = 1;  // pweights imply robust
-    if (vce == 2 && ccodes_.empty()) throw Error(RC_INVALID_INPUT, "fereg iv: cluster variance without clusters");
+    if (vce == 2 && cg_.empty()) throw Error(RC_INVALID_INPUT, "fereg iv: cluster variance without clusters");
 
     std::future<Dof> dof_job = dof_begin(vce == 2, false, false);
     int ph = d.begin(S_COLSTATS);
@@ -1282,7 +1305,7 @@ void GpuSession::wildboot(double* rows, bool on_device, size_t nx, const OlsSpec
                           BootOut& out) {
     AllocScope alloc_scope(ab_->stream());
     restore_weights();
-    if (ccodes_.empty()) throw Error(RC_INVALID_INPUT, "fereg wildboot: the session has no cluster dimension");
+    if (cg_.empty()) throw Error(RC_INVALID_INPUT, "fereg wildboot: the session has no cluster dimension");
     if (bs.coef >= nx) throw Error(RC_INVALID_INPUT, "fereg wildboot: coefficient index out of range");
     if (bs.reps == 0 || bs.tile == 0) throw Error(RC_INVALID_INPUT, "fereg wildboot: reps and tile must be positive");
     if (d_->subsets.size() > size_t(BOOT_MAX_SUB)) throw Error(RC_INVALID_INPUT, "fereg wildboot: at most 3 cluster dimensions");
@@ -1372,11 +1395,10 @@ void GpuSession::wildboot(double* rows, bool on_device, size_t nx, const OlsSpec
     out.reps = reps;
     out.full_enum = full;
     const u32 nwords = (G0 + 63) / 64;
-    const std::vector<u32>& pi = ab_->row_order();
-    std::vector<u32> bcode(n);
-    for (size_t i = 0; i < n; i++) bcode[i] = ccodes_[0][pi[i]];
     DBuf<u32> bcode_d;
-    bcode_d.upload(bcode, st);
+    bcode_d.alloc(n);
+    k_gather_codes<<<blocks_for(n, 256), 256, 0, st>>>(d.ccodes[0].p, pi_device(), n, bcode_d.p);
+    d.launches++;
     DBuf<double> Adev, U, D, Z, tb;
     Adev.upload(A, st);
     const size_t tile = std::min(bs.tile, reps);
@@ -1497,7 +1519,7 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
     if (!wk_.empty()) throw Error(RC_INVALID_INPUT, "fereg glm: weighted sessions are not supported");
     if (gs.family != 0 && gs.family != 1) throw Error(RC_INVALID_INPUT, "fereg glm: family is 0 (Poisson) or 1 (logit)");
     const int fam = gs.family;
-    if (gs.vce == 2 && ccodes_.empty()) throw Error(RC_INVALID_INPUT, "fereg glm: cluster variance without clusters");
+    if (gs.vce == 2 && cg_.empty()) throw Error(RC_INVALID_INPUT, "fereg glm: cluster variance without clusters");
     if (1 + nx + 1 > size_t(OP_MAXM)) throw Error(RC_INVALID_INPUT, "fereg glm: at most 62 regressors");
     SessionDev& d = *d_;
     cudaStream_t st = d.st;
@@ -1671,7 +1693,7 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
             }
             const double gmin = double(*std::min_element(cg_.begin(), cg_.end()));
             V = la::sandwich(inv, meat, k, gmin > 1.0 ? gmin / (gmin - 1.0) : 0.0);
-            if (ccodes_.size() > 1) la::fix_psd(V, k, false);
+            if (cg_.size() > 1) la::fix_psd(V, k, false);
             out.N_clust = gmin;
         } else if (gs.vce == 1) {
             k_glm_score<<<blocks, 256, 0, st>>>(e.p, w.p, n, 1, om.p);
@@ -1971,20 +1993,43 @@ std::vector<double> GpuSession::crv3_meat(const double* rows, const std::vector<
             for (size_t c = 0; c < k; c++) b[a] += inv[a * k + c] * C[(1 + c) * k1];
         return b;
     };
+    // the codes back on the host, kept order (the refits renumber them there)
+    auto host_codes = [&](const std::vector<DBuf<u32>>& dev) {
+        std::vector<std::vector<u32>> h(dev.size());
+        for (size_t i = 0; i < dev.size(); i++) {
+            h[i].resize(n);
+            CK(cudaMemcpyAsync(h[i].data(), dev[i].p, n * sizeof(u32), cudaMemcpyDeviceToHost, st));
+        }
+        CK(cudaStreamSynchronize(st));
+        return h;
+    };
+    const std::vector<std::vector<u32>> tcodes = host_codes(d.tcodes), ccodes = host_codes(d.ccodes);
     std::vector<double> meat(kt * kt, 0.0);
     DBuf<int> dcol;
     dcol.upload(cols, st);
     for (auto& sub : d.subsets) {
         const u32 G = sub.G;
+        std::vector<u32> kc;  // the combined cluster code of every kept observation
+        {
+            std::vector<const std::vector<u32>*> dims;
+            std::vector<u32> gs;
+            for (size_t c = 0; c < cg_.size(); c++)
+                if (sub.mask & (1u << c)) {
+                    dims.push_back(&ccodes[c]);
+                    gs.push_back(cg_[c]);
+                }
+            u32 levels = 0;
+            combine_codes(dims, gs, n, kc, levels);
+        }
         std::vector<u32> cl(n);  // cluster of every row (row order)
-        for (size_t i = 0; i < n; i++) cl[i] = sub.kc[pi[i]];
+        for (size_t i = 0; i < n; i++) cl[i] = kc[pi[i]];
         bool nested_all = true;
-        for (size_t q = 0; q < tcodes_.size() && nested_all; q++) {
+        for (size_t q = 0; q < tcodes.size() && nested_all; q++) {
             std::vector<u32> map(tg_[q], UINT32_MAX);
             for (size_t i = 0; i < n && nested_all; i++) {
-                u32& m = map[tcodes_[q][i]];
-                if (m == UINT32_MAX) m = sub.kc[i];
-                else nested_all = m == sub.kc[i];
+                u32& m = map[tcodes[q][i]];
+                if (m == UINT32_MAX) m = kc[i];
+                else nested_all = m == kc[i];
             }
         }
         std::vector<double> betas(size_t(G) * k);
@@ -2012,17 +2057,17 @@ std::vector<double> GpuSession::crv3_meat(const double* rows, const std::vector<
                 for (size_t i = 0; i < n; i++)
                     if (cl[i] != gg) idx.push_back(u32(i));
                 const size_t m = idx.size();
-                std::vector<std::vector<u32>> sc(tcodes_.size());
+                std::vector<std::vector<u32>> sc(tcodes.size());
                 std::vector<const u32*> sp;
                 std::vector<u32> sg;
-                for (size_t q = 0; q < tcodes_.size(); q++) {
+                for (size_t q = 0; q < tcodes.size(); q++) {
                     std::vector<u32> map(tg_[q], UINT32_MAX);
-                    for (u32 i : idx) map[tcodes_[q][pi[i]]] = 0;
+                    for (u32 i : idx) map[tcodes[q][pi[i]]] = 0;
                     u32 next = 0;
                     for (auto& v : map)
                         if (v == 0) v = next++;
                     sc[q].resize(m);
-                    for (size_t j = 0; j < m; j++) sc[q][j] = map[tcodes_[q][pi[idx[j]]]];
+                    for (size_t j = 0; j < m; j++) sc[q][j] = map[tcodes[q][pi[idx[j]]]];
                     sp.push_back(sc[q].data());
                     sg.push_back(next);
                 }

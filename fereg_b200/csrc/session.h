@@ -163,7 +163,6 @@ class GpuSession {
     int kind_ = 0;
     u64 nsing_ = 0;
     std::vector<u32> tg_, cg_;
-    std::vector<std::vector<u32>> tcodes_, ccodes_;  // kept order (host)
     std::vector<double> wk_;                         // raw kept-order weights
     double sumw_ = 0;
     std::unique_ptr<DeviceAbsorber> ab_;
@@ -218,6 +217,7 @@ class GpuSession {
     };
     FitState fit_;
     void mobility_groups(size_t qa, size_t qb, bool save, u32* out, DofScratch& s);
+    const u32* pi_device();
     std::vector<uint8_t> nested_within(const std::vector<size_t>& qs, size_t c, DofScratch& s);
 };
 

@@ -63,7 +63,7 @@ struct SessionDev {
         DBuf<u32> coff;  // G + 1
         u32 G = 0;
         double sign = 1.0;
-        std::vector<u32> kc;  // host: the combined cluster code of every kept observation
+        u32 mask = 0;    // its cluster dimensions
     };
     std::vector<Subset> subsets;
     DBuf<double> w_raw, wv;  // row order

@@ -827,6 +827,22 @@ __global__ void k_uf_label(const u32* __restrict__ a, size_t n, const u32* __res
         gv[i] = scan[parent[a[i]]] + 1u;
 }
 
+// Kept-order weights in row order: raw as given, wv scaled by f.
+__global__ void k_row_weights(const double* __restrict__ w, const u32* __restrict__ pi, size_t n, double f,
+                              double* __restrict__ raw, double* __restrict__ wv) {
+    for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += size_t(gridDim.x) * blockDim.x) {
+        const double x = w[pi[r]];
+        raw[r] = x;
+        wv[r] = x * f;
+    }
+}
+
+// Kept-order codes in row order.
+__global__ void k_gather_codes(const u32* __restrict__ c, const u32* __restrict__ pi, size_t n, u32* __restrict__ out) {
+    for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += size_t(gridDim.x) * blockDim.x)
+        out[r] = c[pi[r]];
+}
+
 // Nested within (dof.rs:184): map[level] takes the first cluster value seen; any other value
 // marks the term as not nested (flag = 1). Rows in any order give the same verdict. A row reads its
 // level's entry before it tries the CAS (an entry never changes once set), and a warp leaves as

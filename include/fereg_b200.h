@@ -363,7 +363,13 @@ int fereg_drop_singletons(const uint32_t* const* codes, const uint32_t* g, int n
                           uint64_t* dropped_separated);
 int fereg_restrict(const uint32_t* codes, uint32_t g, const uint8_t* alive, size_t n, uint32_t* out,
                    uint32_t* nlevels, uint64_t* kept);
-
+/* Session::prepare's steps in one call (the codes stay on the device between them): nf factor columns
+ * of n values; term t the interaction of the factors term_fac[term_off[t]] .. term_fac[term_off[t + 1]
+ * - 1]; the drops of fereg_drop_singletons from all rows alive; codes[t] (room for n values) receives
+ * the kept rows' codes of term t, levels[t] its levels, *kept the kept rows. n and nterms positive. */
+int fereg_prepare(const double* const* factors, int nf, const int* term_off, const int* term_fac, int nterms, size_t n,
+                  const double* fw, const double* y, int family, int singletons, uint8_t* alive, uint32_t* const* codes,
+                  uint32_t* levels, uint64_t* kept, uint64_t* dropped_singletons, uint64_t* dropped_separated);
 /* Serving: a request loop over independent regressions on one GPU. Requests are admitted in
  * arrival order while their estimated device memory fits the budget (hbm_budget bytes; 0 = 80%
  * of the free memory at creation); `workers` requests run at once, each on its own session and
