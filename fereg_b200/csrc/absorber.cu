@@ -2190,6 +2190,20 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
         }
         d.launches++;
     }
+    else if (d.wseg.n && !S.cell_row && R % 4 == 0 && reinterpret_cast<uintptr_t>(rows) % 16 == 0) {  // wide rows, 16-byte aligned
+        for (int j0 = 0; j0 < R; j0 += VCOLS) {
+            const int Rc = std::min(VCOLS, R - j0);
+            auto go = [&](auto lc, auto nbk) {
+                constexpr int L = decltype(lc)::value, NBK = decltype(nbk)::value;
+                allow_smem(k_vresid<L, NBK>, VR_SMEM);
+                k_vresid<L, NBK><<<148 * 5, VR_WPB * 32, VR_SMEM, st>>>(S, W, d.wseg_segs.p, u32(d.wseg_segs.n), rows, R,
+                                                                       j0, Rc, x, d.b1.p, alpha);
+            };
+            if (S.nb == 0) go(std::integral_constant<int, 32>{}, std::integral_constant<int, 0>{});
+            else with_vlanes(Rc, S.nb, go);
+            d.launches++;
+        }
+    }
     else if (d.wseg.n)
         for (int j0 = 0; j0 < R; j0 += WCOLS) {
             const int Rc = std::min(WCOLS, R - j0);

@@ -42,30 +42,71 @@ __global__ void k_boot_words(u64 seed, u64 b0, u32 bt, u32 nwords, int full_enum
     }
 }
 
-__device__ __forceinline__ double boot_sign(const u64* W, u32 nwords, u32 col, u32 g) {
-    return (W[size_t(col) * nwords + (g >> 6)] >> (g & 63)) & 1ull ? -1.0 : 1.0;
-}
-
-// Z[i][col] = v_{g(i), b0 + col} e_r[i] (row order, n x bt row-major).
-__global__ void k_boot_gen(size_t n, u32 bt, const double* __restrict__ er, const u32* __restrict__ bcode,
-                           const u64* __restrict__ W, u32 nwords, double* __restrict__ Z) {
-    for (size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < n * bt; idx += size_t(gridDim.x) * blockDim.x) {
-        const size_t i = idx / bt;
-        const u32 col = u32(idx % bt);
-        Z[idx] = boot_sign(W, nwords, col, bcode[i]) * er[i];
+// The tile's signs by cluster: bit j of B[g * cw + q] is the sign bit of draw 32 q + j for cluster g
+// (cw = ceil(bt / 32) words; 0 past bt), so that a row's draws are a few consecutive words.
+__global__ void k_boot_bits(const u64* __restrict__ W, u32 nwords, u32 bt, u32 G, u32 cw, u32* __restrict__ B) {
+    const size_t total = size_t(G) * cw;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
+        const u32 g = u32(i % G), q = u32(i / G);  // neighbouring threads read the same words of W
+        u32 bits = 0;
+#pragma unroll 8
+        for (u32 j = 0; j < 32; j++)
+            if (32 * q + j < bt) bits |= u32((W[size_t(32 * q + j) * nwords + (g >> 6)] >> (g & 63)) & 1ull) << j;
+        B[size_t(g) * cw + q] = bits;
     }
 }
 
-// U[col][p] = sum_g v_{g,col} Phi[g][p] (g in order); one thread per (col, p).
-__global__ void k_boot_u(u32 bt, u32 G, int k, const u64* __restrict__ W, u32 nwords, const double* __restrict__ Phi,
-                         double* __restrict__ U) {
-    for (size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < size_t(bt) * k;
-         idx += size_t(gridDim.x) * blockDim.x) {
-        const u32 col = u32(idx / k);
-        const int p = int(idx % k);
-        double s = 0.0;
-        for (u32 g = 0; g < G; g++) s += boot_sign(W, nwords, col, g) * Phi[size_t(g) * k + p];
-        U[idx] = s;
+// Z[i][col] = v_{g(i), b0 + col} e_r[i] (row order, n x btp row-major, btp = bt rounded up to 4, the
+// padding 0): a thread writes four columns. The write of the block bounds it (1e6 x 512: 2.2 ms with a
+// sign word per element, 1.26 ms here, 0.63 of bytes).
+__global__ void __launch_bounds__(BOOT_TB) k_boot_gen(size_t n, u32 bt, u32 btp, const double* __restrict__ er,
+                                                      const u32* __restrict__ bcode, const u32* __restrict__ B, u32 cw,
+                                                      double* __restrict__ Z) {
+    const u32 Q = btp / 4;
+    const size_t total = n * Q, step = size_t(gridDim.x) * BOOT_TB;
+    size_t idx = size_t(blockIdx.x) * BOOT_TB + threadIdx.x;
+    size_t i = idx / Q;
+    u32 q = u32(idx % Q);
+    const size_t di = step / Q;
+    const u32 dq = u32(step % Q);
+    for (; idx < total; idx += step) {
+        const double e = er[i];
+        const u32 bits = B[size_t(bcode[i]) * cw + q / 8] >> (4 * (q % 8));
+        const u32 left = bt - 4 * q;  // columns of this quad within bt
+        double2* o = reinterpret_cast<double2*>(Z + i * btp + 4 * q);
+        __stcs(o, make_double2(bits & 1 ? -e : e, left > 1 ? (bits & 2 ? -e : e) : 0.0));
+        __stcs(o + 1, make_double2(left > 2 ? (bits & 4 ? -e : e) : 0.0, left > 3 ? (bits & 8 ? -e : e) : 0.0));
+        i += di;
+        q += dq;
+        if (q >= Q) {
+            q -= Q;
+            i++;
+        }
+    }
+}
+
+// U[col][p] = sum_g v_{g,col} Phi[g][p]: a CTA per (32 draws, p), lane = draw, the warps taking equal
+// runs of the clusters in order, their sums added in order (one thread per (draw, p) over all clusters
+// took 1.5 ms at 2e4 clusters, 256 threads a CTA 0.32, here 0.10).
+constexpr int BU_TB = 1024;
+__global__ void __launch_bounds__(BU_TB) k_boot_u(u32 bt, u32 G, int k, const u32* __restrict__ B, u32 cw,
+                                                    const double* __restrict__ Phi, double* __restrict__ U) {
+    __shared__ double red[BU_TB];
+    const u32 q = blockIdx.x, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const int p = int(blockIdx.y);
+    const u32 run = (G + BU_TB / 32 - 1) / (BU_TB / 32), g0 = min(G, w * run), g1 = min(G, g0 + run);
+    double s = 0.0;
+#pragma unroll 8
+    for (u32 g = g0; g < g1; g++) {
+        const double x = Phi[size_t(g) * k + p];
+        s += (B[size_t(g) * cw + q] >> lane) & 1u ? -x : x;
+    }
+    red[threadIdx.x] = s;
+    __syncthreads();
+    if (w == 0 && 32 * q + lane < bt) {
+        double t = 0.0;
+        for (u32 i = 0; i < BU_TB / 32; i++) t += red[i * 32 + lane];
+        U[size_t(32 * q + lane) * k + p] = t;
     }
 }
 
@@ -83,8 +124,8 @@ __global__ void k_boot_delta(u32 bt, int k, const double* __restrict__ A, const 
 }
 
 // T1[g][col] = sum over the rows of cluster g (perm[coff[g] .. coff[g+1]], in order) of
-// cw[row] Z[row][col]; a warp per (cluster, 32 columns), lane = column.
-__global__ void k_boot_t1(const double* __restrict__ Z, u32 bt, const double* __restrict__ cw,
+// cw[row] Z[row][col] (Z: row stride ldz); a warp per (cluster, 32 columns), lane = column.
+__global__ void k_boot_t1(const double* __restrict__ Z, u32 bt, u32 ldz, const double* __restrict__ cw,
                           const int* __restrict__ perm, const u32* __restrict__ coff, u32 G, double* __restrict__ T1) {
     const u32 chunks = (bt + 31) / 32;
     const u32 lane = threadIdx.x & 31;
@@ -95,7 +136,7 @@ __global__ void k_boot_t1(const double* __restrict__ Z, u32 bt, const double* __
         double s = 0.0;
         for (u32 q = coff[g]; q < coff[g + 1]; q++) {
             const size_t row = size_t(perm[q]);
-            s += cw[row] * Z[row * bt + col];
+            s += cw[row] * Z[row * ldz + col];
         }
         T1[size_t(g) * bt + col] = s;
     }

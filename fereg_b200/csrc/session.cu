@@ -1404,9 +1404,12 @@ void GpuSession::wildboot(double* rows, bool on_device, size_t nx, const OlsSpec
     const size_t tile = std::min(bs.tile, reps);
     DBuf<u64> Wd;
     Wd.alloc(tile * nwords);
+    const size_t ldz = (tile + 3) / 4 * 4;  // the block's columns rounded up to 4: 16-byte rows
+    DBuf<u32> Bd;
+    Bd.alloc(size_t(G0) * ((tile + 31) / 32));
     U.alloc(tile * k + 1);
     D.alloc(tile * k + 1);
-    Z.alloc(n * tile);
+    Z.alloc(n * ldz);
     tb.alloc(tile);
     for (size_t si = 0; si < d.subsets.size(); si++) T1[si].alloc(size_t(d.subsets[si].G) * tile);
     std::vector<double> t_host(reps);
@@ -1415,13 +1418,14 @@ void GpuSession::wildboot(double* rows, bool on_device, size_t nx, const OlsSpec
         const u32 bt = u32(std::min(tile, reps - b0));
         k_boot_words<<<std::max(1, int((size_t(bt) * nwords + 255) / 256)), 256, 0, st>>>(bs.seed, b0, bt, nwords,
                                                                                          full ? 1 : 0, Wd.p);
-        k_boot_gen<<<int(std::min<size_t>((n * bt + 255) / 256, 148 * 32)), 256, 0, st>>>(n, bt, er.p, bcode_d.p, Wd.p,
-                                                                                          nwords, Z.p);
-        d.launches += 2;
-        ab_->residualize_device(Z.p, bt, bs.tol, bs.maxiter, false, nullptr, nullptr, bs.prec);
+        const u32 btp = (bt + 3) / 4 * 4, cw32 = (bt + 31) / 32;
+        k_boot_bits<<<blocks_for(size_t(G0) * cw32, 256), 256, 0, st>>>(Wd.p, nwords, bt, G0, cw32, Bd.p);
+        k_boot_gen<<<int(std::min<size_t>((n * (btp / 4) + BOOT_TB - 1) / BOOT_TB, 148 * 16)), BOOT_TB, 0, st>>>(
+            n, bt, btp, er.p, bcode_d.p, Bd.p, cw32, Z.p);
+        d.launches += 3;
+        ab_->residualize_device(Z.p, btp, bs.tol, bs.maxiter, false, nullptr, nullptr, bs.prec);
         if (k) {
-            k_boot_u<<<std::max(1, int((size_t(bt) * k + 127) / 128)), 128, 0, st>>>(bt, G0, int(k), Wd.p, nwords, Phi.p,
-                                                                                    U.p);
+            k_boot_u<<<dim3(cw32, u32(k)), BU_TB, 0, st>>>(bt, G0, int(k), Bd.p, cw32, Phi.p, U.p);
             k_boot_delta<<<std::max(1, int((size_t(bt) * k + 127) / 128)), 128, 0, st>>>(bt, int(k), Adev.p, U.p, D.p);
             d.launches += 2;
         }
@@ -1430,7 +1434,7 @@ void GpuSession::wildboot(double* rows, bool on_device, size_t nx, const OlsSpec
         for (size_t si = 0; si < d.subsets.size(); si++) {
             const auto& sub = d.subsets[si];
             const size_t warps = size_t(sub.G) * ((bt + 31) / 32);
-            k_boot_t1<<<int(std::min<size_t>((warps * 32 + 255) / 256, 148 * 32)), 256, 0, st>>>(Z.p, bt, cw.p, sub.perm.p,
+            k_boot_t1<<<int(std::min<size_t>((warps * 32 + 255) / 256, 148 * 32)), 256, 0, st>>>(Z.p, bt, btp, cw.p, sub.perm.p,
                                                                                                sub.coff.p, sub.G, T1[si].p);
             d.launches++;
             subs.T1[si] = T1[si].p;

@@ -1063,4 +1063,61 @@ __global__ void __launch_bounds__(FR_WPB * 32, 5) k_fresid(DevStruct S, DevWeigh
     cp_async_wait_all();
 }
 
+// Residualization of the short segments with one row per cell and wide rows (R a multiple of 4, 16-byte
+// aligned): a lane group of L lanes per segment and VCOLS-column chunk, lane j holding four columns.
+// The cells' u = sum_b x[coord_b(c)] are formed once, a segment's first VR_KEEP of them kept in
+// shared memory for the second walk, which reads and writes the rows along the row. What bounds it is
+// the rows' way through memory and the gathers of x through L2: 1e6 rows x 512 columns 3.7 ms by the
+// warp tiles of k_wresid (32 columns a launch), 2.2 ms here (1.25 of bytes).
+constexpr u32 VR_KEEP = 10;  // five CTAs an SM (16: three, 2.8 ms; 6: 2.4 ms)
+constexpr int VR_WPB = 4;
+constexpr size_t VR_SMEM = size_t(VR_WPB) * 32 * VR_KEEP * 32;
+template <int L, int NBK>
+__global__ void __launch_bounds__(VR_WPB * 32) k_vresid(DevStruct S, DevWeights W, const u32* __restrict__ segs, u32 nsegs,
+                                                        double* __restrict__ rows, int R, int j0, int Rc,
+                                                        const double* __restrict__ x, const double* __restrict__ b1,
+                                                        double* __restrict__ alpha) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int G = 32 / L;
+    constexpr int NL = NBK < WNB ? NBK : WNB;
+    const u32 lane = wlane(), g = lane / L, j = lane % L;
+    if (int(4 * j) >= Rc) return;  // no step below needs the whole warp
+    double* keep = reinterpret_cast<double*>(smem_raw) + size_t(threadIdx.x) * 4;  // + cell * VR_WPB * 128
+    const size_t Ru = size_t(R), cj = size_t(j0) + 4 * j;
+    const double* xj = x + cj;
+    const u32 groups = gridDim.x * VR_WPB * G;
+    auto u_of = [&](u32 c) {
+        V4<double> u{0.0, 0.0, 0.0, 0.0};
+        if constexpr (NBK > 0) {
+            u32 k[NL];
+#pragma unroll
+            for (int b = 0; b < NL; b++) k[b] = __ldg(S.coord + size_t(b) * S.M + c);
+            u = gather4<NBK>(S, k, xj, Ru, c, static_cast<const double*>(nullptr), 0, 0);
+        }
+        return u;
+    };
+    for (u32 q = (blockIdx.x * VR_WPB + wid_in_cta()) * G + g; q < nsegs; q += groups) {
+        const u32 s = segs[q], c0 = S.seg_off[s], c1 = S.seg_off[s + 1];
+        const V4<double> b = ld4(b1 + size_t(s) * Ru + cj);
+        V4<double> a{0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+        for (u32 c = c0; c < c1; c++) {
+            const V4<double> u = u_of(c);
+            if (c - c0 < VR_KEEP) st4(keep + size_t(c - c0) * (VR_WPB * 128), u);
+            fma4(a, cellw(W, c), u);
+        }
+        const double n = W.n1inv[s];
+        a = V4<double>{(b.a - a.a) * n, (b.b - a.b) * n, (b.c - a.c) * n, (b.d - a.d) * n};
+        if (alpha) st4(alpha + size_t(s) * Ru + cj, a);
+#pragma unroll 4
+        for (u32 c = c0; c < c1; c++) {
+            double2* o = reinterpret_cast<double2*>(rows + size_t(c) * Ru + cj);
+            const double2 v0 = __ldcs(o), v1 = __ldcs(o + 1);
+            const V4<double> u = c - c0 < VR_KEEP ? ld4s(keep + size_t(c - c0) * (VR_WPB * 128)) : u_of(c);
+            __stcs(o, make_double2(v0.x - (a.a + u.a), v0.y - (a.b + u.b)));
+            __stcs(o + 1, make_double2(v1.x - (a.c + u.c), v1.y - (a.d + u.d)));
+        }
+    }
+}
+
 }  // namespace fereg
