@@ -511,20 +511,28 @@ std::vector<double> GpuSession::outer_products(const double* src, size_t nrows, 
         if (bulk) {
             CK(cudaMemsetAsync(d.err.p, 0, sizeof(int), st));
             const size_t shm = size_t(CS_STAGES) * CS_ROWS * size_t(srcR) * sizeof(double);
-            auto run = [&](auto kernel) {
+            auto run = [&](auto kernel, int threads) {
                 if (shm > size_t(smem_limit(kernel)))  // static + dynamic can pass 48 KB: always raise it
                     throw Error(RC_INTERNAL, "fereg: the outer-product ring does not fit shared memory");
                 // one wave: the CTAs resident at once (registers or the ring bound them), so that no
                 // second, partial wave runs the last chunks at a fraction of the occupancy
-                parts = std::max(1, std::min(ST_GRID, 148 * resident_ctas(kernel, ST_TB, shm)));
-                kernel<<<parts, ST_TB, shm, st>>>(sp, d.part.p, d.err.p);
+                parts = std::max(1, std::min(ST_GRID, 148 * resident_ctas(kernel, threads, shm)));
+                kernel<<<parts, threads, shm, st>>>(sp, d.part.p, d.err.p);
             };
-            switch ((msz + 7) / 8) {
-                case 1: run(k_outer_mma_bulk<1>); break;
-                case 2: run(k_outer_mma_bulk<2>); break;
-                case 3: run(k_outer_mma_bulk<3>); break;
-                default: run(k_outer_mma_bulk<4>); break;
-            }
+            auto rows_of = [&](auto kc) {
+                constexpr int K = decltype(kc)::value;
+                if (ssq) run(k_gram_rows<K, true>, GR_TB);
+                else run(k_gram_rows<K, false>, GR_TB);
+            };
+            using std::integral_constant;
+            if (msz <= 2) rows_of(integral_constant<int, 2>{});
+            else if (msz <= 4) rows_of(integral_constant<int, 4>{});
+            else if (msz <= 6) rows_of(integral_constant<int, 6>{});
+            else if (msz <= 8) rows_of(integral_constant<int, 8>{});
+            else if (msz <= GR_MAX) rows_of(integral_constant<int, GR_MAX>{});
+            else if (msz <= 16) run(k_outer_mma_bulk<2>, ST_TB);
+            else if (msz <= 24) run(k_outer_mma_bulk<3>, ST_TB);
+            else run(k_outer_mma_bulk<4>, ST_TB);
         } else {
             switch ((msz + 7) / 8) {
                 case 1: k_outer_mma<1><<<ST_GRID, ST_TB, 0, st>>>(sp, d.part.p); break;

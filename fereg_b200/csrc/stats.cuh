@@ -508,6 +508,118 @@ __global__ void __launch_bounds__(ST_TB, NB <= 2 ? 3 : 2) k_outer_mma_bulk(OpSpe
         part[size_t(blockIdx.x) * len + i] = i < mm ? red[(i / s.msz) * W + i % s.msz] : red[W * W + (i - mm)];
 }
 
+// The outer products of at most GR_MAX entries a row (msz <= K, the rest 0) with a row per thread: the
+// rows stream through the bulk-copy ring, a thread takes its row's entries into registers and adds the
+// K (K + 1) / 2 products to sums of its own. The matrix instruction works on blocks of 8 x 8: at 3
+// entries it spends 64 products a row on the 6 that differ, at 9 it spends 192 on 45, in fragment loads
+// and FP64 issue beside the stream. 1e7 weighted rows of 3 entries: 140 us with it, 85 here (49 of
+// bytes); 8.1e5 rows of 9 entries 25 and 18, of 8 entries 14 and 13. The line lies at 10: at 11 entries
+// the 66 products a row bind this kernel too and the sums take most of a thread's registers (1e7 rows:
+// 239 us by the matrix instruction, 248 by rows). SSQ: also the plain sums of squares. Per-thread sums
+// in row order, a butterfly in the warp, the warps in order.
+constexpr int GR_TB = CS_ROWS, GR_MAX = 10;
+template <int K, bool SSQ>
+__global__ void __launch_bounds__(GR_TB) k_gram_rows(OpSpec s, double* __restrict__ part, int* __restrict__ err) {
+    constexpr int NP = K * (K + 1) / 2, NA = NP + (SSQ ? K : 0), NWARP = GR_TB / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(8) u64 bar[CS_STAGES];
+    __shared__ double red[NWARP][NA], shift[K];
+    __shared__ int col[K];
+    double* buf = reinterpret_cast<double*>(smem_raw);  // CS_STAGES x CS_ROWS x R
+    const int R = s.R;
+    const u32 chunk = u32(CS_ROWS) * u32(R);
+    const size_t nchunks = s.n / CS_ROWS;
+    if (threadIdx.x < K) {  // -1: the constant, -2: nothing
+        const int c = int(threadIdx.x);
+        col[c] = c < s.k ? s.col[c] : (c < s.msz ? -1 : -2);
+        shift[c] = (c < s.k && s.shift) ? s.shift[c] : 0.0;
+    }
+    double acc[NA];
+#pragma unroll
+    for (int i = 0; i < NA; i++) acc[i] = 0.0;
+    auto add_row = [&](const double* row, double om) {
+        double x[K];
+#pragma unroll
+        for (int c = 0; c < K; c++) {
+            const int cc = col[c];
+            x[c] = cc >= 0 ? row[cc] : 0.0;
+            if constexpr (SSQ) acc[NP + c] += x[c] * x[c];
+            x[c] = cc == -1 ? 1.0 : x[c] + shift[c];
+        }
+        int p = 0;
+#pragma unroll
+        for (int a = 0; a < K; a++) {
+            const double w = om * x[a];
+#pragma unroll
+            for (int b = a; b < K; b++, p++) acc[p] += w * x[b];
+        }
+    };
+    const size_t mine = blockIdx.x < nchunks ? (nchunks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    auto issue = [&](size_t i) {  // thread 0: chunk i of this CTA into buffer i mod CS_STAGES
+        const int sb = int(i % CS_STAGES);
+        const size_t q = blockIdx.x + i * gridDim.x;
+        mbar_expect_tx(&bar[sb], chunk * 8u);
+        bulk_load(buf + size_t(sb) * chunk, s.rows + q * chunk, chunk * 8u, &bar[sb]);
+    };
+    if (threadIdx.x == 0) {
+        for (int sb = 0; sb < CS_STAGES; sb++) mbar_init(&bar[sb], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (size_t i = 0; i < mine && i < size_t(CS_STAGES); i++) issue(i);
+    size_t failed = mine;
+    double om = (s.om && mine) ? s.om[size_t(blockIdx.x) * CS_ROWS + threadIdx.x] : 1.0;
+    for (size_t i = 0; i < mine; i++) {
+        const int sb = int(i % CS_STAGES);
+        double om_next = 1.0;  // the next chunk's weight, in flight beside this one's products
+        if (s.om && i + 1 < mine) om_next = s.om[(blockIdx.x + (i + 1) * gridDim.x) * CS_ROWS + threadIdx.x];
+        const bool late = !mbar_wait(&bar[sb], u32((i / CS_STAGES) & 1), MBAR_WAIT_LIMIT);
+        if (__syncthreads_or(late)) {
+            failed = i;
+            break;
+        }
+        add_row(buf + size_t(sb) * chunk + size_t(threadIdx.x) * R, om);
+        om = om_next;
+        __syncthreads();  // every thread is done with buffer sb
+        if (threadIdx.x == 0 && i + CS_STAGES < mine) issue(i + CS_STAGES);
+    }
+    if (failed < mine) {
+        if (threadIdx.x == 0) {
+            atomicExch(err, 1);
+            for (size_t i = failed; i < mine && i < failed + CS_STAGES; i++)
+                mbar_wait(&bar[i % CS_STAGES], u32((i / CS_STAGES) & 1), MBAR_WAIT_LIMIT);
+        }
+        __syncthreads();
+        return;
+    }
+    if (blockIdx.x == 0) {  // the rows past the last whole chunk
+        const size_t r = nchunks * CS_ROWS + threadIdx.x;
+        if (r < s.n) add_row(s.rows + r * R, s.om ? s.om[r] : 1.0);
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < NA; i++) {
+        double t = acc[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+        if (lane == 0) red[warp][i] = t;
+    }
+    __syncthreads();
+    const int mm = s.msz * s.msz;
+    const int len = mm + (s.ssq ? s.k : 0);
+    for (int i = threadIdx.x; i < len; i += GR_TB) {
+        int p = NP + (i - mm);
+        if (i < mm) {
+            const int a = min(i / s.msz, i % s.msz), b = max(i / s.msz, i % s.msz);
+            p = a * K - a * (a - 1) / 2 + (b - a);
+        }
+        double t = 0.0;
+        for (int w = 0; w < NWARP; w++) t += red[w][p];
+        part[size_t(blockIdx.x) * len + i] = t;
+    }
+}
+
 // Column statistics in one pass, about a shift c per column (the column's first value):
 // [sum (x-c), sum (x-c)^2, sum w (x-c), sum w (x-c)^2, sum x^2, sum w x^2] per column; the means
 // and the sums of squares about them follow exactly up to rounding (m2 = S2 - S1^2 / n).
