@@ -2190,7 +2190,7 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
         }
         d.launches++;
     }
-    else if (d.wseg.n && !S.cell_row && R % 4 == 0 && reinterpret_cast<uintptr_t>(rows) % 16 == 0) {  // wide rows, 16-byte aligned
+    else if (d.wseg.n && !S.cell_row && R % 4 == 0 && reinterpret_cast<uintptr_t>(rows) % 32 == 0) {  // wide rows, 32-byte aligned
         for (int j0 = 0; j0 < R; j0 += VCOLS) {
             const int Rc = std::min(VCOLS, R - j0);
             auto go = [&](auto lc, auto nbk) {

@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(LT_WPB * 32, 4) k_ltile_pull(DevStruct S, DevW
             acc.b = total(acc.b);
             acc.c = total(acc.c);
             acc.d = total(acc.d);
-            if (g == 0) st4(&red[par][w][4 * j], acc);
+            if (g == 0) st4s(&red[par][w][4 * j], acc);
             __syncthreads();  // two buffers: the next list's warps write the other one
             if (threadIdx.x < u32(Rc)) {
                 const u32 c = threadIdx.x;

@@ -148,9 +148,9 @@ __device__ __forceinline__ bool tile_sums(double* part, int W, size_t stride, un
 }
 
 __device__ __forceinline__ V4<double> ldv(const double* p) {
-    const double2 x = reinterpret_cast<const double2*>(p)[0];
-    const double2 y = reinterpret_cast<const double2*>(p)[1];
-    return V4<double>{x.x, x.y, y.x, y.y};
+    V4<double> v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ V4<float> ldv(const float* p) {
     const float4 x = *reinterpret_cast<const float4*>(p);

@@ -3,7 +3,7 @@
 //
 // The operator's passes (k_vseg_apply, k_vpull_apply) run on the PCG's padded vectors (a row
 // stride that is a multiple of 4): lane j of a group of L lanes holds 4 consecutive columns,
-// gathered with 16-byte loads. The segment pass gives each group one segment at a time and the
+// gathered with one load. The segment pass gives each group one segment at a time and the
 // group walks its cells in order; the list pass deals a list's entries to the groups and adds
 // their sums in group order.
 //
@@ -226,9 +226,12 @@ __device__ __forceinline__ void flush_pairs(const T* wacc_all, u32 ms_acc, int R
 }
 
 // ---------------------------------------------------------------------------------------------
-// The operator's passes on the PCG's padded vectors (row stride Rv, a multiple of 4, 16-byte
-// aligned rows): lane j of a group of L lanes holds the 4 consecutive columns j0 + 4j .. j0 + 4j + 3
-// of the launch's chunk, gathered with 16-byte loads (two per row in FP64, one in FP32).
+// The operator's passes on the PCG's padded vectors (row stride Rv, a multiple of 4; every vector is an
+// allocation of its own, so that four columns start on a 32-byte boundary in FP64, on a 16-byte one in
+// FP32): lane j of a group of L lanes holds the 4 consecutive columns j0 + 4j .. j0 + 4j + 3 of the
+// launch's chunk, gathered with one load per row (256 bits in FP64: two of 128 bits a lane touch
+// every sector twice, and the L1, which bounds these passes, counts each. 1e7 rows, 13 columns: the
+// segment pass 177 us with two, 128 with one, the list pass 230 and 165).
 constexpr int VCOLS = 128;  // columns per launch of the padded-vector passes (32 lanes x 4)
 
 template <class T>
@@ -236,9 +239,9 @@ struct V4 {
     T a, b, c, d;
 };
 __device__ __forceinline__ V4<double> ld4(const double* p) {
-    const double2 x = __ldg(reinterpret_cast<const double2*>(p));
-    const double2 y = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    return V4<double>{x.x, x.y, y.x, y.y};
+    V4<double> v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ V4<float> ld4(const float* p) {
     const float4 x = __ldg(reinterpret_cast<const float4*>(p));
@@ -246,17 +249,16 @@ __device__ __forceinline__ V4<float> ld4(const float* p) {
 }
 // L2-coherent load of values written earlier in the same pass sequence (t)
 __device__ __forceinline__ V4<double> ld4cg(const double* p) {
-    const double2 x = __ldcg(reinterpret_cast<const double2*>(p));
-    const double2 y = __ldcg(reinterpret_cast<const double2*>(p) + 1);
-    return V4<double>{x.x, x.y, y.x, y.y};
+    V4<double> v;
+    asm("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ V4<float> ld4cg(const float* p) {
     const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
     return V4<float>{x.x, x.y, x.z, x.w};
 }
 __device__ __forceinline__ void st4(double* p, const V4<double>& v) {
-    reinterpret_cast<double2*>(p)[0] = make_double2(v.a, v.b);
-    reinterpret_cast<double2*>(p)[1] = make_double2(v.c, v.d);
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.a), "d"(v.b), "d"(v.c), "d"(v.d) : "memory");
 }
 __device__ __forceinline__ void st4(float* p, const V4<float>& v) {
     *reinterpret_cast<float4*>(p) = make_float4(v.a, v.b, v.c, v.d);
@@ -299,6 +301,13 @@ __device__ __forceinline__ V4<double> ld4s(const double* p) {
 __device__ __forceinline__ V4<float> ld4s(const float* p) {
     const float4 x = *reinterpret_cast<const float4*>(p);
     return V4<float>{x.x, x.y, x.z, x.w};
+}
+__device__ __forceinline__ void st4s(double* p, const V4<double>& v) {
+    reinterpret_cast<double2*>(p)[0] = make_double2(v.a, v.b);
+    reinterpret_cast<double2*>(p)[1] = make_double2(v.c, v.d);
+}
+__device__ __forceinline__ void st4s(float* p, const V4<float>& v) {
+    *reinterpret_cast<float4*>(p) = make_float4(v.a, v.b, v.c, v.d);
 }
 // Shared memory of the staged small rows for an Rc-column chunk (0: none staged).
 template <class T>
@@ -1063,15 +1072,26 @@ __global__ void __launch_bounds__(FR_WPB * 32, 5) k_fresid(DevStruct S, DevWeigh
     cp_async_wait_all();
 }
 
-// Residualization of the short segments with one row per cell and wide rows (R a multiple of 4, 16-byte
+// Residualization of the short segments with one row per cell and wide rows (R a multiple of 4, 32-byte
 // aligned): a lane group of L lanes per segment and VCOLS-column chunk, lane j holding four columns.
 // The cells' u = sum_b x[coord_b(c)] are formed once, a segment's first VR_KEEP of them kept in
 // shared memory for the second walk, which reads and writes the rows along the row. What bounds it is
 // the rows' way through memory and the gathers of x through L2: 1e6 rows x 512 columns 3.7 ms by the
-// warp tiles of k_wresid (32 columns a launch), 2.2 ms here (1.25 of bytes).
+// warp tiles of k_wresid (32 columns a launch), 2.2 ms here (1.25 of bytes) with 16-byte accesses to
+// the rows, 2.18 with 32-byte ones.
 constexpr u32 VR_KEEP = 10;  // five CTAs an SM (16: three, 2.8 ms; 6: 2.4 ms)
 constexpr int VR_WPB = 4;
 constexpr size_t VR_SMEM = size_t(VR_WPB) * 32 * VR_KEEP * 32;
+// rows read and written once
+__device__ __forceinline__ V4<double> ld4cs(const double* p) {
+    V4<double> v;
+    asm volatile("ld.global.cs.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st4cs(double* p, const V4<double>& v) {
+    asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.a), "d"(v.b), "d"(v.c), "d"(v.d)
+                 : "memory");
+}
 template <int L, int NBK>
 __global__ void __launch_bounds__(VR_WPB * 32) k_vresid(DevStruct S, DevWeights W, const u32* __restrict__ segs, u32 nsegs,
                                                         double* __restrict__ rows, int R, int j0, int Rc,
@@ -1103,7 +1123,7 @@ __global__ void __launch_bounds__(VR_WPB * 32) k_vresid(DevStruct S, DevWeights 
 #pragma unroll 4
         for (u32 c = c0; c < c1; c++) {
             const V4<double> u = u_of(c);
-            if (c - c0 < VR_KEEP) st4(keep + size_t(c - c0) * (VR_WPB * 128), u);
+            if (c - c0 < VR_KEEP) st4s(keep + size_t(c - c0) * (VR_WPB * 128), u);
             fma4(a, cellw(W, c), u);
         }
         const double n = W.n1inv[s];
@@ -1111,11 +1131,10 @@ __global__ void __launch_bounds__(VR_WPB * 32) k_vresid(DevStruct S, DevWeights 
         if (alpha) st4(alpha + size_t(s) * Ru + cj, a);
 #pragma unroll 4
         for (u32 c = c0; c < c1; c++) {
-            double2* o = reinterpret_cast<double2*>(rows + size_t(c) * Ru + cj);
-            const double2 v0 = __ldcs(o), v1 = __ldcs(o + 1);
+            double* o = rows + size_t(c) * Ru + cj;
+            const V4<double> v = ld4cs(o);
             const V4<double> u = c - c0 < VR_KEEP ? ld4s(keep + size_t(c - c0) * (VR_WPB * 128)) : u_of(c);
-            __stcs(o, make_double2(v0.x - (a.a + u.a), v0.y - (a.b + u.b)));
-            __stcs(o + 1, make_double2(v1.x - (a.c + u.c), v1.y - (a.d + u.d)));
+            st4cs(o, V4<double>{v.a - (a.a + u.a), v.b - (a.b + u.b), v.c - (a.c + u.c), v.d - (a.d + u.d)});
         }
     }
 }
