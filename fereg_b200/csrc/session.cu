@@ -1589,6 +1589,7 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
     la::Mat inv;
     std::vector<double> beta;
     u64 iters = 0, pcg = 0;
+    irls_weights_ = true;  // the absorber holds IRLS weights from here on, also after an error
     for (size_t it = 1; it <= gs.maxiter; it++) {
         ab_->ctx().check();
         iters = it;
@@ -1749,11 +1750,10 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
     out.converged = converged;
     d.collect();
     CK(cudaGetLastError());
-    irls_weights_ = true;  // the absorber holds the last IRLS weights
 }
 
-// The absorber back on the session's weights after a GLM call left its IRLS weights there (the
-// GLM runs on unweighted sessions only).
+// The absorber back on the session's weights after a GLM call (ended or failed) left its IRLS weights
+// there (the GLM runs on unweighted sessions only).
 void GpuSession::restore_weights() {
     if (!irls_weights_) return;
     ab_->set_weights(nullptr);
@@ -1842,6 +1842,7 @@ void GpuSession::relu_separation(double* rows_in, bool on_device, size_t nx, con
         ratio = nb / bd;
         ratio = std::isfinite(ratio) ? std::max(ratio, 1.0) : 1.0;
     }
+    irls_weights_ = true;  // until the end of the check, also after an error
     ab_->set_weights_device(w.p);
     std::vector<int> all(r);
     std::iota(all.begin(), all.end(), 0);
@@ -1934,7 +1935,7 @@ void GpuSession::relu_separation(double* rows_in, bool on_device, size_t nx, con
         k_relu_update<<<blocks, 256, 0, st>>>(raw.p, n, R, xbd.p, u.p);
         d.launches++;
     }
-    ab_->set_weights(nullptr);
+    restore_weights();
     out.iterations = iter;
     out.pcg_iterations = pcg;
     out.complete = found;

@@ -171,7 +171,7 @@ class GpuSession {
     // (dof.rs:165-176, reghdfe dof_update_cvars), fixed by the session's data
     std::vector<bool> t_icpt_;
     std::vector<std::vector<u64>> slope_red_;
-    bool irls_weights_ = false;  // a GLM call left its IRLS weights on the absorber
+    bool irls_weights_ = false;  // a GLM call or a separation check left its weights on the absorber
     void restore_weights();
     // CRV3 (crv3.rs, ols/stata_vce.rs:516-545): the jackknife meat of [b, _cons] over the cluster
     // subsets; rows: the residualized block (device), raw_h: the raw rows (host, row order),
