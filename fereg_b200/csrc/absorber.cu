@@ -736,6 +736,12 @@ bool GpuAbsorber::weights(double* out) const {
     return true;
 }
 
+double* GpuAbsorber::weights_buffer() {
+    AllocScope alloc_scope(stream_);
+    d_->w_rows.alloc(hs_.n);
+    return d_->w_rows.p;
+}
+
 // Device form of refresh_weights for row-order weights already in device memory: every array
 // of the weight state is computed on the device (weights.cuh); the host mirrors are copied back
 // only when a host-side reader needs them.
@@ -747,16 +753,27 @@ void GpuAbsorber::set_weights_device(const double* w_dev) {
     Scratch& d = *d_;
     d.wflag.alloc(1);
     CK(cudaMemsetAsync(d.wflag.p, 0, sizeof(int), stream_));
-    k_check_weights<<<grid_for(n), THREADS, 0, stream_>>>(w_dev, n, d.wflag.p);
     int bad = 0;
-    CK(cudaMemcpyAsync(&bad, d.wflag.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
-    CK(cudaStreamSynchronize(stream_));
-    if (bad) throw Error(RC_INVALID_INPUT, "weights must be positive and finite");
-    d.w_rows.alloc(n);
-    CK(cudaMemcpyAsync(d.w_rows.p, w_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
+    auto refuse_bad = [&]() {  // the stream has passed the copy of the flag
+        if (bad) throw Error(RC_INVALID_INPUT, "weights must be positive and finite");
+    };
+    // weights of the caller's are checked before they replace anything; those written in place
+    // (weights_buffer) in the pass that sums them by cell, and the flag is read with the sums below
+    const bool in_place = w_dev == d.w_rows.p;
+    const bool check_first = !in_place || st.trivial();
+    if (check_first) k_check_weights<<<grid_for(n), THREADS, 0, stream_>>>(w_dev, n, d.wflag.p);
+    if (!in_place) {
+        CK(cudaMemcpyAsync(&bad, d.wflag.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaStreamSynchronize(stream_));
+        refuse_bad();
+        d.w_rows.alloc(n);
+        CK(cudaMemcpyAsync(d.w_rows.p, w_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
+    }
     d.cell_w.alloc(M);
     if (st.trivial()) CK(cudaMemcpyAsync(d.cell_w.p, w_dev, M * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
-    else k_cell_weights<<<grid_for(M), THREADS, 0, stream_>>>(w_dev, d.cell_row.p, u32(M), d.cell_w.p);
+    else
+        k_cell_weights<<<grid_for(M), THREADS, 0, stream_>>>(w_dev, d.cell_row.p, u32(M), d.cell_w.p,
+                                                             check_first ? nullptr : d.wflag.p);
     d.n1.alloc(g1);
     d.n1inv.alloc(g1);
     k_seg_weights<<<grid_for(g1), THREADS, 0, stream_>>>(d.cell_w.p, d.seg_off.p, u32(g1), d.n1.p, d.n1inv.p);
@@ -765,8 +782,10 @@ void GpuAbsorber::set_weights_device(const double* w_dev) {
     d.launches += 4;
     std::vector<double> part(GRID_V);
     CK(cudaMemcpyAsync(part.data(), d.wpart.p, GRID_V * sizeof(double), cudaMemcpyDeviceToHost, stream_));
+    if (in_place) CK(cudaMemcpyAsync(&bad, d.wflag.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
     CK(cudaGetLastError());
+    refuse_bad();
     sw_ = 0.0;
     for (double v : part) sw_ += v;
     weighted_ = true;

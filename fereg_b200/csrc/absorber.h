@@ -64,6 +64,10 @@ class DeviceAbsorber {
     virtual bool weights(double* out) const = 0;
     virtual void set_weights(const double* w_rows) = 0;
     virtual void set_weights_device(const double* w_rows_dev) = 0;
+    // The n row-order weights in device memory, for a caller that writes them in place and passes the
+    // pointer to set_weights_device (no copy then); null where they are kept on the host. Once it is
+    // asked for, the weights are the caller's to set or restore, also after a refused set.
+    virtual double* weights_buffer() { return nullptr; }
     virtual SolveInfo residualize(double* z, size_t r, double tol, size_t maxiter, bool want_coefs, const double* warm,
                                   double* coefs, Precision prec = Precision::F64) = 0;
     virtual SolveInfo residualize_device(double* z_dev, size_t r, double tol, size_t maxiter, bool want_coefs,
@@ -123,6 +127,7 @@ class GpuAbsorber : public DeviceAbsorber {
     // The same for row-order weights in device memory; the weight state is computed on the
     // device (the host mirrors follow when a host-side reader needs them).
     void set_weights_device(const double* w_rows_dev) override;
+    double* weights_buffer() override;
 
     // Residualizes the N x R row-major block `z` in place (rows in row order). `z` is host
     // memory for `residualize`, device memory for `residualize_device`. `warm` and `coefs` are

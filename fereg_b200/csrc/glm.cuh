@@ -8,6 +8,7 @@
 namespace fereg {
 
 constexpr int GLM_TB = 256;
+constexpr int GLM_GRID = 148 * 4;  // CTAs of the passes (1e7 rows: 256 CTAs left k_glm_ll at 188 us, 116 here)
 
 __device__ __forceinline__ double glm_block_sum(double v, double* red) {
     red[threadIdx.x] = v;
@@ -19,15 +20,17 @@ __device__ __forceinline__ double glm_block_sum(double v, double* red) {
     return red[0];
 }
 
-// Partials of sum y; flag = 1 when a y is out of the family's range (Poisson: y >= 0; logit:
-// y in {0, 1}).
+// Partials of sum y and the column y (null: not wanted), so that the later passes read 8 bytes of a row
+// and not the sectors of the whole of it; flag = 1 when a y is out of the family's range (Poisson:
+// y >= 0; logit: y in {0, 1}).
 __global__ void __launch_bounds__(GLM_TB) k_glm_ysum(const double* __restrict__ raw, size_t n, int R, int fam,
-                                                     double* __restrict__ part, int* flag) {
+                                                     double* __restrict__ yc, double* __restrict__ part, int* flag) {
     __shared__ double red[GLM_TB];
     double s = 0.0;
     for (size_t i = size_t(blockIdx.x) * GLM_TB + threadIdx.x; i < n; i += size_t(gridDim.x) * GLM_TB) {
         const double y = raw[i * R];
         if (fam == 0 ? !(y >= 0.0) : !(y == 0.0 || y == 1.0)) atomicExch(flag, 1);
+        if (yc) yc[i] = y;
         s += y;
     }
     const double t = glm_block_sum(s, red);
@@ -59,10 +62,10 @@ __device__ __forceinline__ double glm_mu_dev(int fam, double et, double y, doubl
 
 // Start: Poisson (the `simple` guess) mu = (y + mean y) / 2, logit mu = (y + 1/2) / 2
 // (glm/mod.rs:816-820); `center` is mean y or 1/2. eta = link(mu).
-__global__ void k_glm_start(const double* __restrict__ raw, size_t n, int R, double center, int fam,
-                            double* __restrict__ mu, double* __restrict__ eta) {
+__global__ void k_glm_start(const double* __restrict__ yc, size_t n, double center, int fam, double* __restrict__ mu,
+                            double* __restrict__ eta) {
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const double m = 0.5 * (raw[i * R] + center);
+        const double m = 0.5 * (yc[i] + center);
         mu[i] = m;
         eta[i] = glm_link(fam, m);
     }
@@ -85,19 +88,33 @@ __global__ void k_glm_work(const double* __restrict__ raw, size_t n, int R, int 
     }
 }
 
+// Row i's residual of the weighted regression, e = z~ - sum_p beta[p] x~[col[p]] on the residualized
+// block B = [z~, X~].
+__device__ __forceinline__ double glm_resid(const double* __restrict__ B, size_t i, int R, const int* __restrict__ col,
+                                            const double* __restrict__ beta, int k) {
+    const double* row = B + i * R;
+    double v = row[0];
+    for (int p = 0; p < k; p++) v -= beta[p] * row[col[p]];
+    return v;
+}
+
 // eta = z - e (the fitted linear predictor of the weighted regression), mu from eta, and partials
-// of the deviance / 2 (glm_mu_dev); `old` (non-null) saves the previous eta first.
-__global__ void __launch_bounds__(GLM_TB) k_glm_update(const double* __restrict__ raw, size_t n, int R, int fam,
-                                                       const double* __restrict__ z, const double* __restrict__ e,
-                                                       double* __restrict__ eta, double* __restrict__ old,
-                                                       double* __restrict__ mu, double* __restrict__ part) {
+// of the deviance / 2 (glm_mu_dev); `old` (non-null) saves the previous eta first. The rows' way
+// through memory bounds it (56 bytes a row with 2 regressors): 1e7 rows 212 us with the residuals
+// written by a pass of their own and y read from the block, 115 here (85 of bytes).
+__global__ void __launch_bounds__(GLM_TB, 4) k_glm_update(const double* __restrict__ B, size_t n, int R, int fam,
+                                                          const int* __restrict__ col, const double* __restrict__ beta,
+                                                          int k, const double* __restrict__ yc,
+                                                          const double* __restrict__ z, double* __restrict__ eta,
+                                                          double* __restrict__ old, double* __restrict__ mu,
+                                                          double* __restrict__ part) {
     __shared__ double red[GLM_TB];
     double dev = 0.0;
     for (size_t i = size_t(blockIdx.x) * GLM_TB + threadIdx.x; i < n; i += size_t(gridDim.x) * GLM_TB) {
-        const double et = z[i] - e[i];
+        const double et = z[i] - glm_resid(B, i, R, col, beta, k);
         if (old) old[i] = eta[i];
         double m;
-        dev += glm_mu_dev(fam, et, raw[i * R], m);
+        dev += glm_mu_dev(fam, et, yc[i], m);
         eta[i] = et;
         mu[i] = m;
     }
@@ -107,7 +124,7 @@ __global__ void __launch_bounds__(GLM_TB) k_glm_update(const double* __restrict_
 
 // One step halving toward the previous eta (irls.rs:739-748): eta = (eta + old) / 2, mu and the
 // deviance partials again.
-__global__ void __launch_bounds__(GLM_TB) k_glm_halve(const double* __restrict__ raw, size_t n, int R, int fam,
+__global__ void __launch_bounds__(GLM_TB) k_glm_halve(const double* __restrict__ yc, size_t n, int fam,
                                                       const double* __restrict__ old, double* __restrict__ eta,
                                                       double* __restrict__ mu, double* __restrict__ part) {
     __shared__ double red[GLM_TB];
@@ -115,7 +132,7 @@ __global__ void __launch_bounds__(GLM_TB) k_glm_halve(const double* __restrict__
     for (size_t i = size_t(blockIdx.x) * GLM_TB + threadIdx.x; i < n; i += size_t(gridDim.x) * GLM_TB) {
         const double et = 0.5 * (eta[i] + old[i]);
         double m;
-        dev += glm_mu_dev(fam, et, raw[i * R], m);
+        dev += glm_mu_dev(fam, et, yc[i], m);
         eta[i] = et;
         mu[i] = m;
     }
@@ -125,13 +142,13 @@ __global__ void __launch_bounds__(GLM_TB) k_glm_halve(const double* __restrict__
 
 // Partials of the log-likelihood: Poisson sum [y eta - mu - lgamma(y + 1)], logit
 // sum [y eta - softplus(eta)] (family.rs:143-147).
-__global__ void __launch_bounds__(GLM_TB) k_glm_ll(const double* __restrict__ raw, size_t n, int R, int fam,
+__global__ void __launch_bounds__(GLM_TB) k_glm_ll(const double* __restrict__ yc, size_t n, int fam,
                                                    const double* __restrict__ eta, const double* __restrict__ mu,
                                                    double* __restrict__ part) {
     __shared__ double red[GLM_TB];
     double ll = 0.0;
     for (size_t i = size_t(blockIdx.x) * GLM_TB + threadIdx.x; i < n; i += size_t(gridDim.x) * GLM_TB) {
-        const double y = raw[i * R];
+        const double y = yc[i];
         if (fam == 0) ll += y * eta[i] - mu[i] - lgamma(y + 1.0);
         else ll += y * eta[i] - glm_softplus(eta[i]);
     }
@@ -139,11 +156,12 @@ __global__ void __launch_bounds__(GLM_TB) k_glm_ll(const double* __restrict__ ra
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// Score weights of the sandwich: om = (e w)^2 (robust) or e w (cluster scores).
-__global__ void k_glm_score(const double* __restrict__ e, const double* __restrict__ w, size_t n, int squared,
+// Score weights of the sandwich: om = (e w)^2 (robust) or e w (cluster scores), e as in k_glm_update.
+__global__ void k_glm_score(const double* __restrict__ B, int R, const int* __restrict__ col,
+                            const double* __restrict__ beta, int k, const double* __restrict__ w, size_t n, int squared,
                             double* __restrict__ om) {
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const double s = e[i] * w[i];
+        const double s = glm_resid(B, i, R, col, beta, k) * w[i];
         om[i] = squared ? s * s : s;
     }
 }

@@ -1538,22 +1538,26 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
     const size_t n = n_, r = 1 + nx;
     const int R = int(r);
     const int blocks = int(std::min<size_t>((n + 255) / 256, 148 * 16));
-    DBuf<double> raw, B, mu, eta, eta_old, z, w, e, part, om;
+    DBuf<double> raw_copy, y, B, mu, eta, eta_old, z, own_w, part, om;
     DBuf<int> flag;
-    raw.alloc(n * r);
-    CK(cudaMemcpyAsync(raw.p, rows_in, n * r * 8, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+    // a device block is read where it is (unless the bulk copies could not: a 16-byte boundary)
+    const double* raw = rows_in;
+    if (!on_device || reinterpret_cast<uintptr_t>(rows_in) % 16 != 0) {
+        raw_copy.alloc(n * r);
+        CK(cudaMemcpyAsync(raw_copy.p, rows_in, n * r * 8, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                           st));
+        raw = raw_copy.p;
+    }
+    y.alloc(n);
     B.alloc(n * r);
     mu.alloc(n);
     eta.alloc(n);
     if (fam == 1) eta_old.alloc(n);
     z.alloc(n);
-    w.alloc(n);
-    e.alloc(n);
-    om.alloc(n);
-    part.alloc(GLM_TB * 8);
+    part.alloc(GLM_GRID);
     flag.alloc(1);
     CK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
-    k_glm_ysum<<<GLM_TB, GLM_TB, 0, st>>>(raw.p, n, R, fam, part.p, flag.p);
+    k_glm_ysum<<<GLM_GRID, GLM_TB, 0, st>>>(raw, n, R, fam, y.p, part.p, flag.p);
     auto host_sum = [&](int parts) {
         std::vector<double> h(static_cast<size_t>(parts));
         CK(cudaMemcpyAsync(h.data(), part.p, size_t(parts) * 8, cudaMemcpyDeviceToHost, st));
@@ -1562,7 +1566,7 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
         for (double x : h) t += x;
         return t;
     };
-    const double ysum = host_sum(GLM_TB);
+    const double ysum = host_sum(GLM_GRID);
     int neg = 0;
     CK(cudaMemcpyAsync(&neg, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1571,14 +1575,14 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
                                                : "fereg glm: the logit outcome must be 0 or 1");
     if (!(ysum > 0.0)) throw Error(RC_TOO_FEW_OBS, "insufficient observations (the dependent variable is all zero)");
     if (fam == 1 && !(ysum < double(n))) throw Error(RC_TOO_FEW_OBS, "insufficient observations (the outcome never varies)");
-    k_glm_start<<<blocks, 256, 0, st>>>(raw.p, n, R, fam == 0 ? ysum / double(n) : 0.5, fam, mu.p, eta.p);
+    k_glm_start<<<blocks, 256, 0, st>>>(y.p, n, fam == 0 ? ysum / double(n) : 0.5, fam, mu.p, eta.p);
     d.launches += 2;
 
     // unweighted sums of squares of the raw regressors (stage-1 collinearity, ols.rs:38)
     std::vector<int> all(r);
     std::iota(all.begin(), all.end(), 0);
     std::vector<double> sumsq;
-    outer_products(raw.p, n, R, all, nullptr, false, nullptr, nullptr, true, &sumsq);
+    outer_products(raw, n, R, all, nullptr, false, nullptr, nullptr, true, &sumsq);
     const double highest = std::max(1e-12, std::min(gs.itol, 0.1 * gs.tol));  // glm/mod.rs:826
     double tol_in = std::max(1e-4, gs.tol);
     double dev_old = nanv(), dev = nanv(), eps = nanv(), alt_tol = nanv();
@@ -1590,14 +1594,19 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
     std::vector<double> beta;
     u64 iters = 0, pcg = 0;
     irls_weights_ = true;  // the absorber holds IRLS weights from here on, also after an error
+    double* w = ab_->weights_buffer();  // written in place where the absorber keeps them on the device
+    if (!w) {
+        own_w.alloc(n);
+        w = own_w.p;
+    }
     for (size_t it = 1; it <= gs.maxiter; it++) {
         ab_->ctx().check();
         iters = it;
         const double predicted = hist.predict(eps);
         int ph = d.begin(S_WEIGHTS);
-        k_glm_work<<<blocks, 256, 0, st>>>(raw.p, n, R, fam, mu.p, eta.p, B.p, z.p, w.p);
+        k_glm_work<<<blocks, 256, 0, st>>>(raw, n, R, fam, mu.p, eta.p, B.p, z.p, w);
         d.launches++;
-        ab_->set_weights_device(w.p);
+        ab_->set_weights_device(w);
         d.end(ph);
         // warm start: the previous iteration's reduced solution, left on the device
         const SolveInfo si = have_warm ? ab_->residualize_device_warm_last(B.p, r, tol_in, gs.inner_maxiter, gs.prec)
@@ -1606,7 +1615,7 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
         pcg += si.iterations;
         std::vector<double> ss_res;
         ph = d.begin(S_GRAM);
-        const std::vector<double> G = outer_products(B.p, n, R, all, nullptr, false, w.p, nullptr, true, &ss_res);
+        const std::vector<double> G = outer_products(B.p, n, R, all, nullptr, false, w, nullptr, true, &ss_res);
         d.end(ph);
         ph = d.begin(S_VARIANCE);
         if (it == 1) {  // columns absorbed by the FE, then collinear ones
@@ -1643,18 +1652,17 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
             CK(cudaMemcpyAsync(d.col.p, kc.data(), k * sizeof(int), cudaMemcpyHostToDevice, st));
             CK(cudaMemcpyAsync(d.beta.p, beta.data(), k * 8, cudaMemcpyHostToDevice, st));
         }
-        k_resid_e<<<ST_GRID, ST_TB, 0, st>>>(B.p, n, R, d.col.p, d.beta.p, int(k), 0, nullptr, e.p, part.p);
-        k_glm_update<<<GLM_TB, GLM_TB, 0, st>>>(raw.p, n, R, fam, z.p, e.p, eta.p, fam == 1 ? eta_old.p : nullptr,
-                                                mu.p, part.p);
-        d.launches += 2;
-        dev = 2.0 * host_sum(GLM_TB);
+        k_glm_update<<<GLM_GRID, GLM_TB, 0, st>>>(B.p, n, R, fam, d.col.p, d.beta.p, int(k), y.p, z.p, eta.p,
+                                                  fam == 1 ? eta_old.p : nullptr, mu.p, part.p);
+        d.launches++;
+        dev = 2.0 * host_sum(GLM_GRID);
         // logit step halving while the deviance rose (irls.rs:739-748, at most 25 halvings)
         if (fam == 1 && it > 1) {
             for (int h = 0; h < 25 && (std::isnan(dev) || dev > dev_old + 1e-9 * std::max(std::fabs(dev_old), 1.0));
                  h++) {
-                k_glm_halve<<<GLM_TB, GLM_TB, 0, st>>>(raw.p, n, R, fam, eta_old.p, eta.p, mu.p, part.p);
+                k_glm_halve<<<GLM_GRID, GLM_TB, 0, st>>>(y.p, n, fam, eta_old.p, eta.p, mu.p, part.p);
                 d.launches++;
-                dev = 2.0 * host_sum(GLM_TB);
+                dev = 2.0 * host_sum(GLM_GRID);
             }
         }
         d.end(ph);
@@ -1682,14 +1690,15 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
     }
     if (!converged) throw Error(RC_CONVERGENCE, "fereg glm: IRLS did not converge");
 
-    // variance on the last iteration's weights (w, e and the residualized block B)
+    // variance on the last iteration's weights (w, beta and the residualized block B)
     const size_t k = kept.size();
     std::vector<int> kc(kept.begin(), kept.end());
     la::Mat V(k * k, 0.0);
     const double bigN = double(n);
     if (k) {
+        if (gs.vce != 0) om.alloc(n);
         if (gs.vce == 2) {
-            k_glm_score<<<blocks, 256, 0, st>>>(e.p, w.p, n, 0, om.p);
+            k_glm_score<<<blocks, 256, 0, st>>>(B.p, R, d.col.p, d.beta.p, int(k), w, n, 0, om.p);
             d.launches++;
             la::Mat meat(k * k, 0.0);
             for (auto& sub : d.subsets) {
@@ -1709,7 +1718,7 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
             if (cg_.size() > 1) la::fix_psd(V, k, false);
             out.N_clust = gmin;
         } else if (gs.vce == 1) {
-            k_glm_score<<<blocks, 256, 0, st>>>(e.p, w.p, n, 1, om.p);
+            k_glm_score<<<blocks, 256, 0, st>>>(B.p, R, d.col.p, d.beta.p, int(k), w, n, 1, om.p);
             d.launches++;
             const la::Mat meat = outer_products(B.p, n, R, kc, nullptr, false, om.p, nullptr, false, nullptr);
             V = la::sandwich(inv, meat, k, bigN / (bigN - 1.0));
@@ -1729,9 +1738,9 @@ void GpuSession::glm(double* rows_in, bool on_device, size_t nx, const GlmSpec& 
             chi2 = finite_or_nan(q);
         }
     }
-    k_glm_ll<<<GLM_TB, GLM_TB, 0, st>>>(raw.p, n, R, fam, eta.p, mu.p, part.p);
+    k_glm_ll<<<GLM_GRID, GLM_TB, 0, st>>>(y.p, n, fam, eta.p, mu.p, part.p);
     d.launches++;
-    const double ll = host_sum(GLM_TB);
+    const double ll = host_sum(GLM_GRID);
     if (out.b) std::fill(out.b, out.b + nx, 0.0);
     if (out.V) std::fill(out.V, out.V + nx * nx, 0.0);
     for (size_t a = 0; a < k; a++) {
@@ -1801,7 +1810,7 @@ void GpuSession::relu_separation(double* rows_in, bool on_device, size_t nx, con
     DBuf<int> flag;
     flag.alloc(1);
     CK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
-    k_glm_ysum<<<blocks, GLM_TB, 0, st>>>(raw.p, n, R, 0, part.p, flag.p);
+    k_glm_ysum<<<blocks, GLM_TB, 0, st>>>(raw.p, n, R, 0, nullptr, part.p, flag.p);
     int neg = 0;
     CK(cudaMemcpyAsync(&neg, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

@@ -21,12 +21,19 @@ __global__ void k_check_weights(const double* __restrict__ w, size_t n, int* fla
     }
 }
 
-// W_c = sum of the row weights of cell c (rows cell_row[c] .. cell_row[c+1]).
+// W_c = sum of the row weights of cell c (rows cell_row[c] .. cell_row[c+1]); flag (non-null): as
+// k_check_weights.
 __global__ void k_cell_weights(const double* __restrict__ w, const u32* __restrict__ cell_row, u32 M,
-                               double* __restrict__ cw) {
+                               double* __restrict__ cw, int* __restrict__ flag) {
     for (u32 c = blockIdx.x * blockDim.x + threadIdx.x; c < M; c += gridDim.x * blockDim.x) {
         double s = 0.0;
-        for (u32 r = cell_row[c]; r < cell_row[c + 1]; r++) s += w[r];
+        bool bad = false;
+        for (u32 r = cell_row[c]; r < cell_row[c + 1]; r++) {
+            const double x = w[r];
+            bad |= !(x > 0.0 && x <= 1.7976931348623157e308);
+            s += x;
+        }
+        if (flag && bad) atomicExch(flag, 1);
         cw[c] = s;
     }
 }
