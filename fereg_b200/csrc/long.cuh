@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(LT_WPB * 32, 4) k_ltile_apply(DevStruct S, Dev
                     u32 k[NL];
 #pragma unroll
                     for (int q = 0; q < NL; q++) k[q] = __ldg(S.coord + size_t(q) * S.M + c);
-                    const V4<T> u = gather4<NBK>(S, k, Pj, Ru, c, spj, nsm, Rc);
+                    const V4<T> u = gather4<NBK, L>(S, k, Pj, Ru, c, spj, nsm, Rc);
                     if constexpr (WEIGHTED) fma4(acc, T(W.cell_w[c]), u);
                     else add4(acc, u);
                 }

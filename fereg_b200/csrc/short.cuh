@@ -293,11 +293,25 @@ __device__ __forceinline__ void stage_small(T* sp, const T* __restrict__ P, size
         sp[i] = P[size_t(i / u32(Rc)) * Ru + j0 + i % u32(Rc)];
     __syncthreads();
 }
+// Shared-memory rows in FP64, 16 bytes at a time. Eight lanes go to a pass over the banks: where they read
+// one row (groups of 8 lanes and more), every other four take its upper half first, as in the order of
+// the halves all eight meet in the same 16 banks (1e6 cells, 128 columns: the segment pass 112 us in
+// order, 104 so). Smaller groups read rows of their own, often the same one, which a pass serves at
+// once in order (1e7 cells, 13 columns:
+// 128 us in order, 149 with the halves swapped).
+template <int L>
 __device__ __forceinline__ V4<double> ld4s(const double* p) {
-    const double2 x = reinterpret_cast<const double2*>(p)[0];
-    const double2 y = reinterpret_cast<const double2*>(p)[1];
-    return V4<double>{x.x, x.y, y.x, y.y};
+    const double2* h = reinterpret_cast<const double2*>(p);
+    if constexpr (L >= 8) {
+        const bool up = threadIdx.x & 4;
+        const double2 x = h[up], y = h[!up];
+        return up ? V4<double>{y.x, y.y, x.x, x.y} : V4<double>{x.x, x.y, y.x, y.y};
+    } else {
+        const double2 x = h[0], y = h[1];
+        return V4<double>{x.x, x.y, y.x, y.y};
+    }
 }
+template <int L>
 __device__ __forceinline__ V4<float> ld4s(const float* p) {
     const float4 x = *reinterpret_cast<const float4*>(p);
     return V4<float>{x.x, x.y, x.z, x.w};
@@ -320,14 +334,14 @@ __host__ __device__ constexpr int vlanes_of(int Rc) { return rcp_of((Rc + 3) / 4
 
 // Sum over the blocks of the rows P[coord_b(c)] (this lane's 4 columns): the first NL blocks'
 // coordinates in `code`, the ones past WNB (NBK == WNB) read from the structure.
-template <int NBK, class T>
+template <int NBK, int L, class T>
 __device__ __forceinline__ V4<T> gather4(const DevStruct& S, const u32* code, const T* __restrict__ Pj, size_t Ru,
                                          u32 c, const T* spj, int nsm, int Rc) {
     constexpr int NL = NBK < WNB ? NBK : WNB;
     // the first nsm blocks are small, their rows staged at spj (stride Rc)
-    V4<T> u = nsm > 0 ? ld4s(spj + size_t(code[0]) * Rc) : ld4(Pj + size_t(code[0]) * Ru);
+    V4<T> u = nsm > 0 ? ld4s<L>(spj + size_t(code[0]) * Rc) : ld4(Pj + size_t(code[0]) * Ru);
 #pragma unroll
-    for (int b = 1; b < NL; b++) add4(u, b < nsm ? ld4s(spj + size_t(code[b]) * Rc) : ld4(Pj + size_t(code[b]) * Ru));
+    for (int b = 1; b < NL; b++) add4(u, b < nsm ? ld4s<L>(spj + size_t(code[b]) * Rc) : ld4(Pj + size_t(code[b]) * Ru));
     if constexpr (NBK == WNB)
         for (u32 b = WNB; b < S.nb; b++) add4(u, ld4(Pj + size_t(__ldg(S.coord + size_t(b) * S.M + c)) * Ru));
     return u;
@@ -367,8 +381,8 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vseg_apply(DevStruct S, DevWeig
                     k0[b] = __ldg(S.coord + size_t(b) * S.M + c);
                     k1[b] = __ldg(S.coord + size_t(b) * S.M + c + 1);
                 }
-                const V4<T> u0 = gather4<NBK>(S, k0, Pj, Ru, c, spj, nsm, Rc);
-                const V4<T> u1 = gather4<NBK>(S, k1, Pj, Ru, c + 1, spj, nsm, Rc);
+                const V4<T> u0 = gather4<NBK, L>(S, k0, Pj, Ru, c, spj, nsm, Rc);
+                const V4<T> u1 = gather4<NBK, L>(S, k1, Pj, Ru, c + 1, spj, nsm, Rc);
                 if constexpr (WEIGHTED) {
                     fma4(acc, T(W.cell_w[c]), u0);
                     fma4(acc, T(W.cell_w[c + 1]), u1);
@@ -381,7 +395,7 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vseg_apply(DevStruct S, DevWeig
                 u32 k0[NL];
 #pragma unroll
                 for (int b = 0; b < NL; b++) k0[b] = __ldg(S.coord + size_t(b) * S.M + c);
-                const V4<T> u0 = gather4<NBK>(S, k0, Pj, Ru, c, spj, nsm, Rc);
+                const V4<T> u0 = gather4<NBK, L>(S, k0, Pj, Ru, c, spj, nsm, Rc);
                 if constexpr (WEIGHTED) fma4(acc, T(W.cell_w[c]), u0);
                 else add4(acc, u0);
             }
@@ -522,7 +536,7 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWei
 #pragma unroll
                     for (int o = 0; o < NO; o++) {
                         const u32 x = WEIGHTED ? __ldcs(S.pl_other + size_t(e0 + i) * no + o) : oth[o * PULL_WARP_MAX + i];
-                        add4(v, o < nsm ? ld4s(spj + size_t(x) * Rc) : ld4(Pj + size_t(x) * Ru));
+                        add4(v, o < nsm ? ld4s<L>(spj + size_t(x) * Rc) : ld4(Pj + size_t(x) * Ru));
                     }
                     if constexpr (NBK == WNB)
                         for (u32 o = WNO; o < no; o++)
@@ -1112,7 +1126,7 @@ __global__ void __launch_bounds__(VR_WPB * 32) k_vresid(DevStruct S, DevWeights 
             u32 k[NL];
 #pragma unroll
             for (int b = 0; b < NL; b++) k[b] = __ldg(S.coord + size_t(b) * S.M + c);
-            u = gather4<NBK>(S, k, xj, Ru, c, static_cast<const double*>(nullptr), 0, 0);
+            u = gather4<NBK, L>(S, k, xj, Ru, c, static_cast<const double*>(nullptr), 0, 0);
         }
         return u;
     };
@@ -1133,7 +1147,7 @@ __global__ void __launch_bounds__(VR_WPB * 32) k_vresid(DevStruct S, DevWeights 
         for (u32 c = c0; c < c1; c++) {
             double* o = rows + size_t(c) * Ru + cj;
             const V4<double> v = ld4cs(o);
-            const V4<double> u = c - c0 < VR_KEEP ? ld4s(keep + size_t(c - c0) * (VR_WPB * 128)) : u_of(c);
+            const V4<double> u = c - c0 < VR_KEEP ? ld4s<L>(keep + size_t(c - c0) * (VR_WPB * 128)) : u_of(c);
             st4cs(o, V4<double>{v.a - (a.a + u.a), v.b - (a.b + u.b), v.c - (a.c + u.c), v.d - (a.d + u.d)});
         }
     }
