@@ -2428,7 +2428,13 @@ u64 PcgDriver::run(DevOperator& op, double* x, const double* b, int R, const std
 }
 
 void PcgDriver::col_sums(const double* part, int nparts, int ncols, double* out, cudaStream_t st) {
-    reduce_cols(*d_, part, nparts, ncols, out, st);
+    if (nparts <= TALL_PARTS) {
+        reduce_cols(*d_, part, nparts, ncols, out, st);
+        return;
+    }
+    k_reduce_tall<<<std::max(1, std::min(GRID_V, ncols)), TALL_TB, 0, st>>>(part, nparts, ncols, out);
+    d_->launches++;
+    CK(cudaGetLastError());
 }
 
 u64 PcgDriver::launches() const { return d_->launches; }

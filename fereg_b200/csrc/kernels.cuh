@@ -64,6 +64,28 @@ __global__ void k_reduce_cols(const double* __restrict__ part, int nparts, const
     }
 }
 
+// The same sums of one array of many parts (a part per level of a term): a CTA per column, so that a
+// column's chain of loads is short. 2e4 parts of 9 columns: 168 us by warps, 8 here.
+constexpr int TALL_TB = 1024, TALL_PARTS = 4096;
+__global__ void __launch_bounds__(TALL_TB) k_reduce_tall(const double* __restrict__ part, int nparts, int ncols,
+                                                         double* __restrict__ out) {
+    __shared__ double red[TALL_TB / 32];
+    for (int col = blockIdx.x; col < ncols; col += gridDim.x) {
+        double acc = 0.0;
+#pragma unroll 8
+        for (int p = threadIdx.x; p < nparts; p += TALL_TB) acc += part[size_t(p) * ncols + col];
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+        if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0.0;
+            for (int w = 0; w < TALL_TB / 32; w++) t += red[w];
+            out[col] = t;
+        }
+        __syncthreads();
+    }
+}
+
 // Per-column PCG state (cg.rs:132-292), kept on the device. active: 1 iterating, 0 stopped by
 // the reference's rules, 2 stopped at the FP32 precision floor of a refinement round.
 struct CgState {

@@ -30,6 +30,7 @@
 
 #include "bulk.cuh"
 #include "tiles.cuh"
+#include "vec4.cuh"
 
 namespace fereg {
 
@@ -234,56 +235,6 @@ __device__ __forceinline__ void flush_pairs(const T* wacc_all, u32 ms_acc, int R
 // segment pass 177 us with two, 128 with one, the list pass 230 and 165).
 constexpr int VCOLS = 128;  // columns per launch of the padded-vector passes (32 lanes x 4)
 
-template <class T>
-struct V4 {
-    T a, b, c, d;
-};
-__device__ __forceinline__ V4<double> ld4(const double* p) {
-    V4<double> v;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ V4<float> ld4(const float* p) {
-    const float4 x = __ldg(reinterpret_cast<const float4*>(p));
-    return V4<float>{x.x, x.y, x.z, x.w};
-}
-// L2-coherent load of values written earlier in the same pass sequence (t)
-__device__ __forceinline__ V4<double> ld4cg(const double* p) {
-    V4<double> v;
-    asm("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ V4<float> ld4cg(const float* p) {
-    const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
-    return V4<float>{x.x, x.y, x.z, x.w};
-}
-__device__ __forceinline__ void st4(double* p, const V4<double>& v) {
-    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.a), "d"(v.b), "d"(v.c), "d"(v.d) : "memory");
-}
-__device__ __forceinline__ void st4(float* p, const V4<float>& v) {
-    *reinterpret_cast<float4*>(p) = make_float4(v.a, v.b, v.c, v.d);
-}
-template <class T>
-__device__ __forceinline__ void add4(V4<T>& s, const V4<T>& v) {
-    s.a += v.a;
-    s.b += v.b;
-    s.c += v.c;
-    s.d += v.d;
-}
-template <class T>
-__device__ __forceinline__ void sub4(V4<T>& s, const V4<T>& v) {
-    s.a -= v.a;
-    s.b -= v.b;
-    s.c -= v.c;
-    s.d -= v.d;
-}
-template <class T>
-__device__ __forceinline__ void fma4(V4<T>& s, T w, const V4<T>& v) {
-    s.a += w * v.a;
-    s.b += w * v.b;
-    s.c += w * v.c;
-    s.d += w * v.d;
-}
 // The rows of the small coordinates (0 .. ms_acc - 1, the first blocks) of the launch's column
 // chunk, staged in shared memory once per CTA: every cell holds one of them per small block, and a
 // gather from shared memory spares the L1 the tag and line work of a global gather.
@@ -315,13 +266,6 @@ template <int L>
 __device__ __forceinline__ V4<float> ld4s(const float* p) {
     const float4 x = *reinterpret_cast<const float4*>(p);
     return V4<float>{x.x, x.y, x.z, x.w};
-}
-__device__ __forceinline__ void st4s(double* p, const V4<double>& v) {
-    reinterpret_cast<double2*>(p)[0] = make_double2(v.a, v.b);
-    reinterpret_cast<double2*>(p)[1] = make_double2(v.c, v.d);
-}
-__device__ __forceinline__ void st4s(float* p, const V4<float>& v) {
-    *reinterpret_cast<float4*>(p) = make_float4(v.a, v.b, v.c, v.d);
 }
 // Shared memory of the staged small rows for an Rc-column chunk (0: none staged).
 template <class T>

@@ -227,6 +227,19 @@ struct SlopeDevBufs {
 
 namespace {
 
+// Y (m x C, stride ldy) from Z (stride ldz, a multiple of 4).
+void launch_pull(const SlopeHost& h, SlopeDevBufs& d, int C, int ldz, double* Y, int ldy, const int* halt,
+                 cudaStream_t st) {
+    const size_t work = size_t(h.m) * size_t((C + 3) / 4);
+    if (h.n * size_t(h.k) > size_t(SL_LONG) * h.m)
+        k_sl_pull<SL_TB><<<sl_grid(work * SL_TB), SL_TB, 0, st>>>(h.m, C, d.pl_off.p, d.pl_row.p, d.pl_val.p, d.Z.p, ldz,
+                                                                  Y, ldy, halt);
+    else
+        k_sl_pull<32><<<sl_grid(work * 32), SL_TB, 0, st>>>(h.m, C, d.pl_off.p, d.pl_row.p, d.pl_val.p, d.Z.p, ldz, Y, ldy,
+                                                            halt);
+    d.launches++;
+}
+
 // The slope operator seen by PcgDriver: S p by the segment and coordinate passes, z = J r.
 struct SlopeOp final : DevOperator {
     const SlopeHost& h;
@@ -235,12 +248,26 @@ struct SlopeOp final : DevOperator {
     SlopeOp(const SlopeHost& h_, SlopeDevBufs& d_, const SlopeDev& D_) : h(h_), d(d_), D(D_) {}
     u32 m() const override { return h.m; }
     void apply(double* p, int R, double* q, cudaStream_t st) override {
+        if (R % 4 != 0) throw Error(RC_INTERNAL, "fereg: the slope operator takes padded vectors (a multiple of 4 columns)");
         d.Z.alloc(std::max<size_t>(1, h.n * size_t(R)));
-        k_sl_seg<SL_APPLY><<<sl_grid(size_t(h.ge) * R), SL_TB, 0, st>>>(D, p, R, R, nullptr, 0, d.Z.p, R, nullptr,
-                                                                        nullptr, 0, nullptr, halt);
-        k_sl_pull<<<sl_grid(size_t(h.m) * R), SL_TB, 0, st>>>(h.m, R, d.pl_off.p, d.pl_row.p, d.pl_val.p, d.Z.p, R, q,
-                                                               R, halt);
-        d.launches += 2;
+        // lanes per level: the average level's rows, in one step where they are at most a warp's
+        const size_t work = size_t(h.ge) * size_t(R / 4), rows = h.n / std::max<u32>(h.ge, 1);
+        auto go = [&](auto bc, auto gc) {
+            constexpr int BE = decltype(bc)::value, GL = decltype(gc)::value;
+            k_sl_apply<BE, GL><<<sl_grid(work * GL), SL_TB, 0, st>>>(D, p, R, d.Z.p, halt);
+        };
+        using std::integral_constant;
+        auto by_level = [&](auto bc) {
+            if (rows <= 4) go(bc, integral_constant<int, 4>{});
+            else if (rows <= 8) go(bc, integral_constant<int, 8>{});
+            else if (rows <= 16) go(bc, integral_constant<int, 16>{});
+            else go(bc, integral_constant<int, 32>{});
+        };
+        if (h.be <= 2) by_level(integral_constant<int, 2>{});
+        else if (h.be <= 4) by_level(integral_constant<int, 4>{});
+        else by_level(integral_constant<int, SL_BE_MAX>{});
+        launch_pull(h, d, R, R, q, R, halt, st);
+        d.launches++;
     }
     void precond(double* r, double* z, int R, cudaStream_t st) override {
         const u32 nu = u32(h.un_c0.size());
@@ -524,8 +551,8 @@ SolveInfo GpuSlopeSolver::solve(double* z, size_t r, double tol, size_t maxiter,
         CK(cudaMemsetAsync(d.rhs.p, 0, m * rv * 8, st));
         k_sl_seg<SL_RHS><<<sl_grid(size_t(h.ge) * r), SL_TB, 0, st>>>(D, z, R, R, nullptr, 0, d.Z.p, RV, nullptr,
                                                                       nullptr, 0, d.part.p);
-        k_sl_pull<<<sl_grid(m * r), SL_TB, 0, st>>>(h.m, R, d.pl_off.p, d.pl_row.p, d.pl_val.p, d.Z.p, RV, d.rhs.p, RV);
-        d.launches += 2;
+        launch_pull(h, d, R, RV, d.rhs.p, RV, nullptr, st);
+        d.launches++;
         d.pcg.col_sums(d.part.p, int(h.ge), 3 * R, d.stats.p, st);
         std::vector<double> ex(3 * r);
         CK(cudaMemcpyAsync(ex.data(), d.stats.p, 3 * r * 8, cudaMemcpyDeviceToHost, st));
@@ -668,13 +695,15 @@ void GpuSlopeSolver::apply_host(const double* p, size_t r, double* y) {
     SlopeDevBufs& d = *d_;
     const size_t m = hs_.m;
     if (m == 0 || r == 0) return;
-    d.pin.alloc(m * r);
-    d.pout.alloc(m * r);
-    CK(cudaMemcpyAsync(d.pin.p, p, m * r * 8, cudaMemcpyHostToDevice, stream_));
+    const size_t rv = (r + 3) / 4 * 4;
+    d.pin.alloc(m * rv);
+    d.pout.alloc(m * rv);
+    CK(cudaMemsetAsync(d.pin.p, 0, m * rv * 8, stream_));
+    CK(cudaMemcpy2DAsync(d.pin.p, rv * 8, p, r * 8, r * 8, m, cudaMemcpyHostToDevice, stream_));
     SlopeOp op(hs_, d, d.dev(hs_, !w_rows_.empty()));
-    op.apply(d.pin.p, int(r), d.pout.p, stream_);
+    op.apply(d.pin.p, int(rv), d.pout.p, stream_);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(y, d.pout.p, m * r * 8, cudaMemcpyDeviceToHost, stream_));
+    CK(cudaMemcpy2DAsync(y, r * 8, d.pout.p, rv * 8, r * 8, m, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
 }
 
@@ -701,16 +730,16 @@ void GpuSlopeSolver::rhs_host(const double* rows, size_t r, double* y, double* s
     if (r == 0) return;
     const SlopeDev D = d.dev(h, !w_rows_.empty());
     d.zbuf.alloc(std::max<size_t>(1, n * r));
-    d.Z.alloc(std::max<size_t>(1, n * r));
+    const size_t rv = (r + 3) / 4 * 4;
+    d.Z.alloc(std::max<size_t>(1, n * rv));
     d.rhs.alloc(std::max<size_t>(1, m * r));
     d.part.alloc(std::max<size_t>(1, size_t(h.ge) * 3 * r));
     d.stats.alloc(3 * r);
     const int R = int(r);
     CK(cudaMemcpyAsync(d.zbuf.p, rows, n * r * 8, cudaMemcpyHostToDevice, stream_));
-    k_sl_seg<SL_RHS><<<sl_grid(size_t(h.ge) * r), SL_TB, 0, stream_>>>(D, d.zbuf.p, R, R, nullptr, 0, d.Z.p, R,
+    k_sl_seg<SL_RHS><<<sl_grid(size_t(h.ge) * r), SL_TB, 0, stream_>>>(D, d.zbuf.p, R, R, nullptr, 0, d.Z.p, int(rv),
                                                                        nullptr, nullptr, 0, d.part.p);
-    if (m) k_sl_pull<<<sl_grid(m * r), SL_TB, 0, stream_>>>(h.m, R, d.pl_off.p, d.pl_row.p, d.pl_val.p, d.Z.p, R,
-                                                            d.rhs.p, R);
+    if (m) launch_pull(h, d, R, int(rv), d.rhs.p, R, nullptr, stream_);
     d.pcg.col_sums(d.part.p, int(h.ge), 3 * R, d.stats.p, stream_);
     CK(cudaGetLastError());
     if (m) CK(cudaMemcpyAsync(y, d.rhs.p, m * r * 8, cudaMemcpyDeviceToHost, stream_));
