@@ -37,7 +37,8 @@ struct RowLanes {
 
 // Operator pass 1 on segments of more than LONG_SEG cells: t_s = n1inv_s sum_c W_c u_c, a warp per
 // tile, a segment's cells dealt to the lane groups; slices of longer segments write partials.
-// 4e4 segments of 50 weighted cells, 4 columns: 43 us with one lane group a segment, 25 here.
+// 4e4 segments of 50 weighted cells, 4 columns: 43 us with one lane group a segment, 25 by
+// tiles, 19 with 256-bit gathers.
 template <class T, int L, int NBK, bool WEIGHTED>
 __global__ void __launch_bounds__(LT_WPB * 32, 4) k_ltile_apply(DevStruct S, DevWeights W, const T* __restrict__ P,
                                                                 int Rv, int j0, int Rc, T* __restrict__ t,
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(LT_WPB * 32, 4) k_ltile_apply(DevStruct S, Dev
 // Operator pass 2 on long coordinate lists: Y[k] = nr_k P[k] + sum over the cells c of k of
 // W_c (sum_{other b} P[coord_b(c)] - t_{s(c)}); slices write partials. A CTA per tile, the entries
 // dealt to the lane groups of its warps in turn, the groups' sums added by a butterfly and the warps'
-// in order. 1.6e6 entries in 110 lists, 12 columns: 104 us by (slot, column) threads, 56 here
+// in order. 1.6e6 entries in 110 lists, 12 columns: 104 us by (slot, column) threads, 41 here
 // (466 MB of gathered rows through L2).
 template <class T, int L, int NBK, bool WEIGHTED>
 __global__ void __launch_bounds__(LT_WPB * 32, 4) k_ltile_pull(DevStruct S, DevWeights W, const T* __restrict__ P,

@@ -434,7 +434,8 @@ __device__ __forceinline__ void vpull_prefetch(const DevStruct& S, const uint4& 
 // the 1e6-row bootstrap panel's list pass 8% faster). Weighted cells read the indices and the
 // weights (in list order, W.pl_w) straight from memory: on the gravity panel's lists of 200 entries,
 // one entry a lane, staging and its barriers cost more than they hid (4e6 entries, 4 columns: 67 us
-// staged with the weights gathered by cell, 65 staged with them in order, 53 here).
+// staged with the weights gathered by cell, 65 staged with them in order, 53 direct; 36 with
+// 256-bit gathers).
 template <class T, int L, int NBK, bool WEIGHTED>
 __global__ void __launch_bounds__(WPB * 32, 4) k_vpull_apply(DevStruct S, DevWeights W, WarpTiles wt,
                                                              const T* __restrict__ P, const T* __restrict__ t, int Rv,
@@ -873,7 +874,9 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_wresid(DevStruct S, DevWeights 
 // to lane e mod 32), so the row copies and stores and the gathers of x run along the rows on all
 // 32 lanes. Software pipelined: while a warp works on one tile, cp.async copies bring the next
 // tile's rows, block coordinates, cell weights, segment offsets and 1/n1 into the other of two
-// shared buffers. For a tile:
+// shared buffers. A tile's chain of loads bounds it (1e7 rows, 11 columns: 543 us with b1 loaded in
+// step 2, 510 with it in flight beside the gathers; 270 of bytes. The next tile's gathers a step ahead
+// 634, the rows straight to registers 1060). For a tile:
 //  1. u(c, j) = sum_b x[coord_b(c), j] (blocks in order), every element's gathers in flight
 //     together, into the warp's shared memory U[e];
 //  2. alpha(s, j) = (b1(s, j) - sum_c W_c u(c, j)) / n1_s, one (segment, column) pair per lane,
@@ -950,6 +953,7 @@ __global__ void __launch_bounds__(FR_WPB * 32, 5) k_fresid(DevStruct S, DevWeigh
                                                            const double* __restrict__ b1, double* __restrict__ alpha) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int NC = NBK < WNB ? NBK : WNB;  // blocks whose coordinates are staged
+    constexpr int NP = (int(WSEG) * NE + int(WT) - 1) / int(WT);  // (segment, column) pairs per lane at most
     const u32 uR = u32(R);
     unsigned char* mine = smem_raw + size_t(threadIdx.x >> 5) * fresid_bytes(R);
     const u32 bbytes = u32(fr_buf_bytes(R));
@@ -982,6 +986,13 @@ __global__ void __launch_bounds__(FR_WPB * 32, 5) k_fresid(DevStruct S, DevWeigh
             while (cur.soff[sl + 1] - c0 <= lane) sl++;
             segl[lane] = sl;
         }
+        // b1 of the tile's (segment, column) pairs, pair pr in slot pr / 32 of lane pr mod 32
+        double bs[NP];
+#pragma unroll
+        for (int k = 0; k < NP; k++) {
+            const u32 pr = lane + 32u * u32(k);
+            bs[k] = pr < ns * uR ? __ldg(b1 + size_t(s0) * Ru + pr) : 0.0;
+        }
         // 1. u of every element, all the lane's gathers in flight together
         {
             double g[NE];
@@ -1006,12 +1017,15 @@ __global__ void __launch_bounds__(FR_WPB * 32, 5) k_fresid(DevStruct S, DevWeigh
         }
         __syncwarp();
         // 2. alpha of every (segment, column) pair
-        for (u32 pr = lane; pr < ns * uR; pr += 32) {
+#pragma unroll
+        for (int k = 0; k < NP; k++) {
+            const u32 pr = lane + 32u * u32(k);
+            if (pr >= ns * uR) break;
             const u32 sl = pr / uR, c = pr % uR;
             const u32 i0 = cur.soff[sl] - c0, i1 = cur.soff[sl + 1] - c0;
             double a = 0.0;
             for (u32 i = i0; i < i1; i++) a += (W.cell_w ? cur.cw[i] : 1.0) * U[i * uR + c];
-            const double al = (b1[size_t(s0 + sl) * Ru + c] - a) * cur.n1i[sl];
+            const double al = (bs[k] - a) * cur.n1i[sl];
             A[sl * uR + c] = al;
             if (alpha) alpha[size_t(s0 + sl) * Ru + c] = al;
         }

@@ -46,7 +46,8 @@ __global__ void k_gather_rows_f64(const double* __restrict__ in, const u32* __re
 }
 
 // pw[e] = the weight of list entry e's cell: the list passes of the operator then read the weights in
-// order (4e6 entries, 4 columns: 67 -> 53 us an apply with the direct reads they allow, 19 us per weight state).
+// order (4e6 entries, 4 columns: 67 -> 53 us an apply with the direct reads they allow
+// (36 since the gathers are of 256 bits), 19 us per weight state).
 __global__ void k_list_weights(const double* __restrict__ cw, const u32* __restrict__ pl_cell, size_t E,
                                double* __restrict__ pw) {
     for (size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x; e < E; e += size_t(gridDim.x) * blockDim.x)
