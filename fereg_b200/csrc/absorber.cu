@@ -58,7 +58,7 @@ inline int grid_for(size_t total) {
 struct DevTiles {
     DBuf<u32> k0, k1, e0, e1, fix_k, fix_p0, fix_np;
     DBuf<int> part, fixidx;
-    u32 n = 0, nfix = 0, nparts = 0;
+    u32 n = 0, nfix = 0, nparts = 0, nheavy = 0;
     void upload(const TileList& t, cudaStream_t s) {
         k0.upload(t.k0, s);
         k1.upload(t.k1, s);
@@ -72,8 +72,11 @@ struct DevTiles {
         n = u32(t.k0.size());
         nfix = u32(t.fix_k.size());
         nparts = t.nparts;
+        nheavy = t.nheavy;
     }
-    TileSet set() const { return TileSet{n, k0.p, k1.p, e0.p, e1.p, part.p, fixidx.p, nfix, fix_k.p, fix_p0.p, fix_np.p, nparts}; }
+    TileSet set() const {
+        return TileSet{n, k0.p, k1.p, e0.p, e1.p, part.p, fixidx.p, nfix, fix_k.p, fix_p0.p, fix_np.p, nparts, nheavy};
+    }
 };
 
 // Warp tiles packed as (k0, k1, e0, e1) in one 16-byte load.
@@ -412,7 +415,9 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
         CK(cudaStreamSynchronize(stream_));  // the uploaded codes die here
     }
     {
-        // segments weigh max(cells, rows): short ones go to warp tiles, the others to CTA tiles
+        // segments weigh max(cells, rows): short ones go to warp tiles, the others to tiles of at most
+        // TILE cells and LT_ROWS rows (or one segment); a tile of more rows than its share of the
+        // long segments' goes to a CTA, the others to a warp each
         std::vector<u32> wgt(hs_.g1);
         for (u32 s = 0; s < hs_.g1; s++) {
             const u32 c0 = hs_.seg_off[s], c1 = hs_.seg_off[s + 1];
@@ -421,8 +426,12 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
         }
         WarpTileList wt;
         TileList ct;
-        split_tiles(hs_.seg_off, &wgt, 0, hs_.g1, WT, WT, WSEG, TILE, wt, ct);
-            d_->nrows = n;
+        split_tiles(hs_.seg_off, &wgt, 0, hs_.g1, WT, WT, WSEG, TILE, LT_ROWS, wt, ct);
+        u64 long_rows = 0;
+        for (u32 s = 0; s < hs_.g1; s++)
+            if (wgt[s] > WT) long_rows += wgt[s];
+        heavy_first(ct, hs_.cell_row, long_rows / LT_SHARE);
+        d_->nrows = n;
         d_->wseg.upload(wt, stream_);
         std::vector<u32> segs;  // the short segments in order (one per lane group in k_vseg_apply)
         for (size_t i = 0; i < wt.k0.size(); i++)
@@ -514,7 +523,7 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
         for (u32 k = d_->ms_acc; k < u32(hs_.m); k++)
             if (pl_off[k + 1] - pl_off[k] > PULL_WARP_MAX) el += pl_off[k + 1] - pl_off[k];
         const u32 slice = u32(std::min<u64>(PULL_SLICE, (el / 444 + 255) / 256 * 256 + 256));
-        split_tiles(pl_off, nullptr, d_->ms_acc, u32(hs_.m), PULL_WARP_MAX, PULL_WARP_MAX, WLIST, slice, wt, ct);
+        split_tiles(pl_off, nullptr, d_->ms_acc, u32(hs_.m), PULL_WARP_MAX, PULL_WARP_MAX, WLIST, slice, UINT64_MAX, wt, ct);
         d_->wpull.upload(wt, stream_);
         d_->pull_tiles.upload(ct, stream_);
         CK(cudaStreamSynchronize(stream_));  // host tables die here
@@ -2242,13 +2251,14 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
         d.launches += 2;
     }
     if (S.seg.n) {
+        const u32 ctas = std::min<u32>(148 * 8, S.seg.nheavy + (S.seg.n - S.seg.nheavy + LR_WPB - 1) / LR_WPB);
         for (int j0 = 0; j0 < R; j0 += LR_COLS) {
             const int Rc = std::min(LR_COLS, R - j0);
             const size_t shm = LR_WPB * ltile_resid_bytes(Rc);
             with_nbk<1, 0>(S.nb, [&](auto, auto nbk) {
                 constexpr int NBK = decltype(nbk)::value;
                 allow_smem(k_ltile_resid<NBK>, shm);
-                k_ltile_resid<NBK><<<148 * 8, LR_WPB * 32, shm, st>>>(S, W, rows, R, j0, Rc, x, d.b1.p, d.along.p, alpha);
+                k_ltile_resid<NBK><<<int(ctas), LR_WPB * 32, shm, st>>>(S, W, rows, R, j0, Rc, x, d.b1.p, d.along.p, alpha);
             });
             d.launches++;
         }

@@ -97,6 +97,7 @@ struct TileList {
     std::vector<u32> fix_k;            // lists completed from partials
     std::vector<u32> fix_p0, fix_np;   // first partial slot and count per long list
     u32 nparts = 0;
+    u32 nheavy = 0;                    // the first tiles are heavy (heavy_first)
 };
 TileList build_tiles(const std::vector<u32>& off, u32 k_begin, u32 k_end, u32 cap, u32 min_len);
 
@@ -107,9 +108,14 @@ struct WarpTileList {
 
 // Splits the lists [k_begin, k_end) of a CSR-like array by weight (`weight[k]`, or the entry
 // count when null): lists of weight <= warp_max go to warp tiles, packed consecutively while the
-// summed weight stays <= pack and the tile holds at most max_lists lists; the others go to CTA
-// tiles of at most cta_cap entries (slices of longer lists write partials).
+// summed weight stays <= pack and the tile holds at most max_lists lists; the others go to tiles of
+// at most cta_cap entries (slices of longer lists write partials) and, where they hold more than
+// one list, a summed weight of at most cta_weight.
 void split_tiles(const std::vector<u32>& off, const std::vector<u32>* weight, u32 k_begin, u32 k_end, u32 warp_max,
-                 u32 pack, u32 max_lists, u32 cta_cap, WarpTileList& wt, TileList& ct);
+                 u32 pack, u32 max_lists, u32 cta_cap, u64 cta_weight, WarpTileList& wt, TileList& ct);
+
+// Moves the tiles of more than `limit` rows to the front of the list (order kept) and counts them;
+// entry e starts at row first_row[e] (empty: row e).
+void heavy_first(TileList& t, const std::vector<u32>& first_row, u64 limit);
 
 }  // namespace fereg

@@ -2,8 +2,9 @@
 // operator) and coordinate lists of more than PULL_WARP_MAX entries, cut into the tiles of
 // tiles.cuh. Every pass is bound by the latency of its gathers, so what these kernels do is keep
 // many of them in flight: a warp walks a segment tile on its own, with no barrier of the CTA, and
-// reads rows along the row (lane = (row group, column) over floor(32 / columns) groups); a list
-// tile is shared by the warps of a CTA, which meet once per list. The operator's kernels use the
+// reads rows along the row (lane = (row group, column) over floor(32 / columns) groups); a heavy
+// segment tile (one that would keep its warp busy when the others are done) and every list tile are
+// shared by the warps of a CTA, which meet once per segment or list. The operator's kernels use the
 // padded vectors and lane groups of short.cuh. All sums have a fixed order.
 #pragma once
 
@@ -15,6 +16,17 @@ constexpr u32 LONG_SEG = 32;  // cells of the longest segment one lane group of 
 constexpr int LT_WPB = 8;     // warps per CTA
 constexpr int LR_WPB = 4;     // of k_ltile_resid (its cells' values take up to 16 KB a warp)
 constexpr int LR_COLS = 16;   // columns per launch of k_ltile_resid
+// Rows of a segment tile of several segments. Tiles are cut by rows as well as cells: a tile of TILE
+// cells holds any number of rows, and a sample of few levels makes few tiles (1e7 rows, 11 columns, a
+// warp per tile cut by cells alone: one term of 50 levels, one tile, 1960 ms; a CTA per such tile 449;
+// cut by rows, the heavy ones to CTAs, 29. 1e3 levels: 253, 47 and 3.1 ms; 1e5: 3.06, 1.57 and 1.00).
+// 128 to 2048 rows measure the same, but for fewer, longer segments (60 of 1,000 rows, 12 columns:
+// 138, 142 and 170 us at 128, 512 and 2048); 512 leaves two segments of 250 rows a tile.
+constexpr u64 LT_ROWS = 512;
+// A tile of more than 1 / LT_SHARE of the long segments' rows is heavy: with fewer such tiles than
+// that the chip's warps are not all at work. 1e3 tiles of 5,000 rows: 197 us as heavy ones, 325 as light;
+// 4e3 tiles of 100 rows: 138 and 109; 2e3 tiles of 100 rows in eight IRLS steps: 3.54 and 3.46 ms.
+constexpr u64 LT_SHARE = 1184;
 
 // Lane = (group g, column c) over a chunk of Rc <= 32 columns.
 struct RowLanes {
@@ -167,38 +179,41 @@ __global__ void __launch_bounds__(LT_WPB * 32, 4) k_ltile_pull(DevStruct S, DevW
 
 // Right-hand side pass 1 on the long segments (no small coordinates summed): b1_s = sum over the rows
 // of w v (partials for slices), the CTAs' [sum w v^2, sum w v] per column (cta_part, grid x 2R), and
-// the cells' sums (cs, M x R) where the list pass reads those instead of the rows. A warp per tile,
-// cells dealt to the lane groups, the rows of a cell in order.
+// the cells' sums (cs, M x R) where the list pass reads those instead of the rows. A warp per tile
+// (heavy ones: a CTA), cells dealt to the lane groups, the rows of a cell in order.
 // 4e4 segments of 50 cells of 5 rows, 3 columns: 300 us by CTA tiles, 102 here (49 us of
 // bytes).
 __global__ void __launch_bounds__(LT_WPB * 32) k_ltile_rhs(DevStruct S, DevWeights W, const double* __restrict__ rows,
                                                            int R, int j0, int Rc, double* __restrict__ b1,
                                                            double* __restrict__ part, double* __restrict__ cta_part,
                                                            double* __restrict__ cs) {
-    __shared__ double red[2][LT_WPB * 32];
+    __shared__ double red[2][LT_WPB * 32], team[2][LT_WPB][32];
     constexpr int U = 8;
     const RowLanes L(Rc);
     const size_t Ru = size_t(R);
     const TileSet& ts = S.seg;
     const double* vj = rows + j0 + L.c;
     double q = 0.0, ws = 0.0;
-    for (u32 tile = blockIdx.x * LT_WPB + wid_in_cta(); tile < ts.n; tile += gridDim.x * LT_WPB) {
+    int par = 0;
+    auto take = [&](u32 tile, u32 w, auto warps) {  // warp w of the tile's warps
+        constexpr u32 NW = decltype(warps)::value;
         const u32 s0 = ts.k0[tile], s1 = ts.k1[tile], c0 = ts.e0[tile], c1 = ts.e1[tile];
         const int pslot = ts.part[tile];
+        const u32 first = w * u32(L.G) + u32(L.g), step = NW * u32(L.G);
         for (u32 s = s0; s < s1; s++) {
             const u32 a = max(S.seg_off[s], c0), b = min(S.seg_off[s + 1], c1);
             double sum = 0.0;
             if (L.on) {
                 if (!S.cell_row) {
 #pragma unroll 8
-                    for (u32 c = a + u32(L.g); c < b; c += u32(L.G)) {
+                    for (u32 c = a + first; c < b; c += step) {
                         const double v = __ldcs(vj + size_t(c) * Ru);
                         const double wv = W.w_rows ? W.w_rows[c] * v : v;
                         sum += wv;
                         q += wv * v;
                     }
                 } else {
-                    for (u32 c = a + u32(L.g); c < b; c += u32(L.G)) {
+                    for (u32 c = a + first; c < b; c += step) {
                         const u32 r0 = S.cell_row[c], r1 = S.cell_row[c + 1];
                         double sc = 0.0;
                         for (u32 r = r0; r < r1; r += U) {
@@ -221,12 +236,25 @@ __global__ void __launch_bounds__(LT_WPB * 32) k_ltile_rhs(DevStruct S, DevWeigh
             }
             ws += sum;
             sum = L.total(sum, Rc);
-            if (L.on && L.g == 0) {
+            if constexpr (NW > 1) {  // the warps in order; two buffers, as in k_ltile_pull
+                if (L.on && L.g == 0) team[par][w][L.c] = sum;
+                __syncthreads();
+                sum = 0.0;
+#pragma unroll
+                for (u32 i = 0; i < NW; i++) sum += team[par][i][L.c];
+                par ^= 1;
+            }
+            if (w == 0 && L.on && L.g == 0) {
                 if (pslot < 0) b1[size_t(s) * Ru + j0 + L.c] = sum;
                 else part[size_t(pslot) * Ru + j0 + L.c] = sum;
             }
         }
-    }
+    };
+    using std::integral_constant;
+    for (u32 tile = blockIdx.x; tile < ts.nheavy; tile += gridDim.x)
+        take(tile, wid_in_cta(), integral_constant<u32, LT_WPB>{});
+    for (u32 tile = ts.nheavy + blockIdx.x * LT_WPB + wid_in_cta(); tile < ts.n; tile += gridDim.x * LT_WPB)
+        take(tile, 0u, integral_constant<u32, 1>{});
     red[0][threadIdx.x] = q;
     red[1][threadIdx.x] = ws;
     __syncthreads();
@@ -302,8 +330,8 @@ __global__ void __launch_bounds__(LT_WPB * 32) k_ltile_pull_rhs(DevStruct S, Dev
 }
 
 // Residualization of the long segments (operator.rs:1107-1179): alpha_s = (b1_s - sum_c W_c u_c) / n1_s
-// with u_c = sum_b x[coord_b(c)], then every row of cell c loses alpha_s + u_c. A warp per tile: the
-// cells' u and first rows into shared memory, alpha of each segment (slices of long segments take it
+// with u_c = sum_b x[coord_b(c)], then every row of cell c loses alpha_s + u_c. A warp per tile (heavy
+// ones: a CTA): the cells' u and first rows into shared memory, alpha of each segment (slices of long segments take it
 // from `along`, index fixidx, filled beforehand), then the segment's rows, 8 of them in flight a
 // lane. 4e4 segments of 50 cells of 5 rows, 3 columns: 558 us by CTA tiles, 133 here (73 us of
 // bytes).
@@ -317,23 +345,30 @@ __global__ void __launch_bounds__(LR_WPB * 32) k_ltile_resid(DevStruct S, DevWei
                                                              const double* __restrict__ along,
                                                              double* __restrict__ alpha) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double team[2][LR_WPB][LR_COLS];
     constexpr int NL = NBK < WNB ? NBK : WNB;
     constexpr int U = 8;
-    unsigned char* mine = smem_raw + size_t(wid_in_cta()) * ltile_resid_bytes(Rc);
-    double* us = reinterpret_cast<double*>(mine);
-    u32* cr = reinterpret_cast<u32*>(mine + al16(size_t(TILE) * Rc * 8));
     const RowLanes L(Rc);
     const size_t Ru = size_t(R);
     const u32 lane = wlane(), uRc = u32(Rc);
     const TileSet& ts = S.seg;
     double* vj = rows + j0 + L.c;
-    for (u32 tile = blockIdx.x * LR_WPB + wid_in_cta(); tile < ts.n; tile += gridDim.x * LR_WPB) {
+    int par = 0;
+    auto take = [&](u32 tile, u32 w, unsigned char* mine, auto warps) {  // warp w of the tile's warps
+        constexpr u32 NW = decltype(warps)::value;
+        auto meet = [&]() {
+            if constexpr (NW > 1) __syncthreads();
+            else __syncwarp();
+        };
+        double* us = reinterpret_cast<double*>(mine);
+        u32* cr = reinterpret_cast<u32*>(mine + al16(size_t(TILE) * Rc * 8));
         const u32 s0 = ts.k0[tile], s1 = ts.k1[tile], c0 = ts.e0[tile], c1 = ts.e1[tile], nc = c1 - c0;
         const int fidx = ts.fixidx[tile];
+        const u32 me = w * 32u + lane, first = w * u32(L.G) + u32(L.g), step = NW * u32(L.G);
         if (S.cell_row)
-            for (u32 i = lane; i <= nc; i += 32) cr[i] = S.cell_row[c0 + i];
+            for (u32 i = me; i <= nc; i += NW * 32u) cr[i] = S.cell_row[c0 + i];
 #pragma unroll 4
-        for (u32 e = lane; e < nc * uRc; e += 32) {
+        for (u32 e = me; e < nc * uRc; e += NW * 32u) {
             const u32 i = e / uRc, c = e % uRc;
             double u = 0.0;
 #pragma unroll
@@ -342,33 +377,41 @@ __global__ void __launch_bounds__(LR_WPB * 32) k_ltile_resid(DevStruct S, DevWei
                 for (u32 q = WNB; q < S.nb; q++) u += __ldg(x + size_t(S.coord[size_t(q) * S.M + c0 + i]) * Ru + j0 + c);
             us[e] = u;
         }
-        __syncwarp();
+        meet();
         for (u32 s = s0; s < s1; s++) {
             const u32 a = max(S.seg_off[s], c0) - c0, b = min(S.seg_off[s + 1], c1) - c0;
             double al = 0.0;
             if (fidx < 0) {
                 double tot = 0.0;
                 if (L.on)
-                    for (u32 i = a + u32(L.g); i < b; i += u32(L.G)) tot += cellw(W, c0 + i) * us[i * uRc + L.c];
+                    for (u32 i = a + first; i < b; i += step) tot += cellw(W, c0 + i) * us[i * uRc + L.c];
                 tot = L.total(tot, Rc);
+                if constexpr (NW > 1) {  // the warps in order; two buffers, as in k_ltile_pull
+                    if (L.on && L.g == 0) team[par][w][L.c] = tot;
+                    __syncthreads();
+                    tot = 0.0;
+#pragma unroll
+                    for (u32 i = 0; i < NW; i++) tot += team[par][i][L.c];
+                    par ^= 1;
+                }
                 al = (b1[size_t(s) * Ru + j0 + L.c] - tot) * W.n1inv[s];
-                if (alpha && L.on && L.g == 0) alpha[size_t(s) * Ru + j0 + L.c] = al;
+                if (alpha && w == 0 && L.on && L.g == 0) alpha[size_t(s) * Ru + j0 + L.c] = al;
             } else {
                 al = along[size_t(fidx) * Ru + j0 + L.c];
             }
             if (L.on) {
                 const u32 r0 = S.cell_row ? cr[a] : c0 + a, r1 = S.cell_row ? cr[b] : c0 + b;
                 u32 i = a;
-                for (u32 r = r0 + u32(L.g); r < r1; r += U * u32(L.G)) {
+                for (u32 r = r0 + first; r < r1; r += U * step) {
                     double v[U];
 #pragma unroll
                     for (int k = 0; k < U; k++) {
-                        const u32 rr = r + u32(k * L.G);
+                        const u32 rr = r + u32(k) * step;
                         v[k] = rr < r1 ? __ldcs(vj + size_t(rr) * Ru) : 0.0;
                     }
 #pragma unroll
                     for (int k = 0; k < U; k++) {
-                        const u32 rr = r + u32(k * L.G);
+                        const u32 rr = r + u32(k) * step;
                         if (rr < r1) {
                             if (S.cell_row)
                                 while (cr[i + 1] <= rr) i++;
@@ -379,8 +422,14 @@ __global__ void __launch_bounds__(LR_WPB * 32) k_ltile_resid(DevStruct S, DevWei
                 }
             }
         }
-        __syncwarp();  // the next tile's values replace these
-    }
+        meet();  // the next tile's values replace these
+    };
+    using std::integral_constant;
+    for (u32 tile = blockIdx.x; tile < ts.nheavy; tile += gridDim.x)
+        take(tile, wid_in_cta(), smem_raw, integral_constant<u32, LR_WPB>{});
+    unsigned char* own = smem_raw + size_t(wid_in_cta()) * ltile_resid_bytes(Rc);
+    for (u32 tile = ts.nheavy + blockIdx.x * LR_WPB + wid_in_cta(); tile < ts.n; tile += gridDim.x * LR_WPB)
+        take(tile, 0u, own, integral_constant<u32, 1>{});
 }
 
 }  // namespace fereg

@@ -380,7 +380,7 @@ TileList build_tiles(const std::vector<u32>& off, u32 k_begin, u32 k_end, u32 ca
 namespace fereg {
 
 void split_tiles(const std::vector<u32>& off, const std::vector<u32>* weight, u32 k_begin, u32 k_end, u32 warp_max,
-                 u32 pack, u32 max_lists, u32 cta_cap, WarpTileList& wt, TileList& ct) {
+                 u32 pack, u32 max_lists, u32 cta_cap, u64 cta_weight, WarpTileList& wt, TileList& ct) {
     auto wgt = [&](u32 k) { return weight ? (*weight)[k] : off[k + 1] - off[k]; };
     // warp tiles: consecutive lists of weight <= warp_max, packed while the total stays <= pack
     u32 k = k_begin;
@@ -402,7 +402,7 @@ void split_tiles(const std::vector<u32>& off, const std::vector<u32>* weight, u3
         wt.e1.push_back(off[k1]);
         k = k1;
     }
-    // CTA tiles over the others (lists longer than warp_max by weight)
+    // tiles over the others (lists longer than warp_max by weight)
     k = k_begin;
     while (k < k_end) {
         if (wgt(k) <= warp_max) {
@@ -429,10 +429,13 @@ void split_tiles(const std::vector<u32>& off, const std::vector<u32>* weight, u3
             continue;
         }
         u32 k1 = k, tot = 0;
+        u64 totw = 0;
         while (k1 < k_end) {
             const u32 c = off[k1 + 1] - off[k1];
-            if (wgt(k1) <= warp_max || c > cta_cap || (tot + c > cta_cap && k1 > k)) break;
+            if (wgt(k1) <= warp_max || c > cta_cap) break;
+            if (k1 > k && (tot + c > cta_cap || totw + wgt(k1) > cta_weight)) break;
             tot += c;
+            totw += wgt(k1);
             k1++;
         }
         ct.k0.push_back(k);
@@ -443,6 +446,30 @@ void split_tiles(const std::vector<u32>& off, const std::vector<u32>* weight, u3
         ct.fixidx.push_back(-1);
         k = k1;
     }
+}
+
+void heavy_first(TileList& t, const std::vector<u32>& first_row, u64 limit) {
+    const size_t n = t.k0.size();
+    std::vector<u32> order;
+    auto heavy = [&](size_t i) {
+        return u64(first_row.empty() ? t.e1[i] - t.e0[i] : first_row[t.e1[i]] - first_row[t.e0[i]]) > limit;
+    };
+    for (size_t i = 0; i < n; i++)
+        if (heavy(i)) order.push_back(u32(i));
+    t.nheavy = u32(order.size());
+    if (t.nheavy == 0 || t.nheavy == n) return;
+    for (size_t i = 0; i < n; i++)
+        if (!heavy(i)) order.push_back(u32(i));
+    auto permute = [&](auto& v) {
+        auto in = v;
+        for (size_t i = 0; i < n; i++) v[i] = in[order[i]];
+    };
+    permute(t.k0);
+    permute(t.k1);
+    permute(t.e0);
+    permute(t.e1);
+    permute(t.part);
+    permute(t.fixidx);
 }
 
 }  // namespace fereg

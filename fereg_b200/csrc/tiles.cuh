@@ -41,6 +41,7 @@ struct TileSet {
     const u32* fix_p0;
     const u32* fix_np;
     u32 nparts;
+    u32 nheavy;          // the first tiles are taken by whole CTAs where light ones go to warps (long.cuh)
 };
 
 struct DevStruct {
