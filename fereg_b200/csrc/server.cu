@@ -10,11 +10,55 @@
 
 namespace fereg {
 
+namespace {
+
+constexpr u64 SMALL_SUMMED = 16;  // small coordinates summed in the segment passes (tiles.cuh SACC_MAX)
+
+// The request's largest sum of buffers alive together, from its sizes: while the structure is built,
+// while the clusters are grouped, and in the call. The cells are not known before the build, so the
+// call counts for the largest of: one row a cell without weights (the ordered assembly of a small
+// block of at most 32 coordinates holds its counts by segment before the vectors are there), nearly as
+// many cells as rows with weights, and half as many with the right-hand side's sums by cell.
+u64 itemized_bytes(const ServeRequest& r, u64 ms, u64 dense) {
+    const u64 n = r.n, R = 1 + r.nx + r.ne + r.ni, rv = (R + 3) / 4 * 4;
+    const u64 nt = r.codes.size(), nc = r.cl_codes.size(), nb = nt > 0 ? nt - 1 : 0, no = nb > 0 ? nb - 1 : 0;
+    const bool glm = r.model >= 2, weighted = glm || r.w;
+    u64 levels = 0, g1 = 1;
+    for (u32 x : r.g) {
+        levels += x;
+        g1 = std::max<u64>(g1, x);
+    }
+    const u64 m = levels - (nt > 0 ? g1 : 0), acc = std::min(ms, SMALL_SUMMED);
+    // a row: codes and row order, cluster permutations, blocks, GLM's y, eta, mu and the like or
+    // residuals, score weights and weights, partials of the slices
+    const u64 codes = 4 * (nt + nc + 1), perms = 4 * ((u64(1) << std::min<u64>(nc, 8)) - 1);
+    const u64 columns = 8 * (glm ? 8 : r.w ? 5 : 2);
+    const u64 call = codes + perms + 8 * R * (glm ? 3 : 2) + columns + rv / 16;
+    // a cell: coordinates, the lists' cells, segments and other coordinates; first row, weight, the
+    // weights in list order
+    const u64 cell = nb * (12 + 4 * no), wcell = cell + 12 + 8 * nb;
+    // the reduced system's vectors and per-level state
+    const u64 half = r.precision ? 1 : 0;
+    const u64 vec = 8 * (m * (2 * R + 6 * rv + 4 * half * rv + 4 + acc) + g1 * (2 * R + rv + half * rv / 2 + 2 + acc));
+    u64 most = std::max(n * (call + wcell) + vec, n * call + n / 2 * (wcell + 8 * R) + vec);
+    if (!weighted) most = std::max(most, n * (call + cell) + std::max(vec, 8 * g1 * (ms <= 32 ? ms : 0)));
+    // the sort of the cells' list entries; the stable sorts of the (combined) cluster codes
+    most = std::max(most, n * (codes + 20 + nb * (32 + 4 * no)));
+    most = std::max(most, n * (codes + perms + wcell + (nc > 1 ? 36 : nc > 0 ? 24 : 0)));
+    const u64 fixed = 8 * (592 * (R + 2) * (R + 2) + 2368 * acc * R + 888 * 5 * rv) + (u64(ms > 0 ? 28 : 8) << 20);
+    return most + 40 * levels + dense + fixed;
+}
+
+}  // namespace
+
 // Device bytes a request's session holds, from its sizes (an upper estimate): the kept-order
-// columns and the row-order block (a third block for GLM's raw copy), per-row state (term and
+// columns and the row-order block (a third, GLM's working block), per-row state (term and
 // cluster codes, row order, cluster permutations, structure tables, residuals, weights, GLM
 // working vectors), the PCG vectors of the reduced system (m <= sum of levels, ~10 m x R
-// doubles) and a fixed 32 MiB for tiles, partials and the small block.
+// doubles) and a fixed 32 MiB for tiles, partials and the small block; or the itemized sum where
+// that is larger (many terms, whose lists and weights in list order grow with the square of their
+// number, or a wide block on cells of several rows: 4e6 weighted rows in five terms hold 903 MiB,
+// 750 by the first sum).
 u64 request_bytes(const ServeRequest& r) {
     const u64 n = r.n, R = 1 + r.nx + r.ne + r.ni;
     const u64 blocks = r.model >= 2 ? 3 : 2;
@@ -35,7 +79,8 @@ u64 request_bytes(const ServeRequest& r) {
         ms += x;
     }
     const u64 dense = ms > 0 && ms <= 1024 ? (4 * ms * ms + (4096 + ms) * ms) * 8 : 0;
-    return n * per_row + levels * R * 8 * 10 + dense + (32ull << 20);
+    const u64 sum = n * per_row + levels * R * 8 * 10 + dense + (u64(32) << 20);
+    return std::max(sum, itemized_bytes(r, ms, dense));
 }
 
 Server::Server(int workers, u64 budget, bool dry_run) : dry_(dry_run), t0_(std::chrono::steady_clock::now()) {
