@@ -40,6 +40,12 @@ double finite_or_nan(double x) { return std::isfinite(x) ? x : nanv(); }
 
 int blocks_for(size_t n, int tb) { return int(std::max<size_t>(1, std::min<size_t>((n + tb - 1) / tb, 148 * 16))); }
 
+// Rows up to which the clusters are grouped on the host: a subset's dozen small kernels and read-backs
+// take 0.2 ms (single) to 0.5 ms (combined) at any size, the host's sort 0.5 ms at 4,000 rows (three
+// dimensions: 200 rows 3.6 ms a session by the host and 4.5 on the device, 4,000 the same, 20,000 13.0
+// and 5.2).
+constexpr size_t HOST_GROUP_ROWS = 4096;
+
 // Interaction codes of several dimensions (factor.rs:255 combine): the tuple key in mixed radix
 // (first dimension most significant), distinct keys numbered in ascending order.
 void combine_codes(const std::vector<const std::vector<u32>*>& dims, const std::vector<u32>& gs, size_t n,
@@ -180,33 +186,57 @@ GpuSession::GpuSession(const std::vector<const u32*>& codes, const std::vector<u
     // cluster subsets (inclusion-exclusion of vcov.rs:480-560): every non-empty subset of the
     // dimensions, its rows grouped by the combined code
     const size_t q = cg_.size();
+    std::vector<std::vector<u32>> hcodes;
+    if (n <= HOST_GROUP_ROWS)
+        for (size_t c = 0; c < q; c++) {
+            hcodes.emplace_back(cl_codes[c], cl_codes[c] + n);
+            for (u32 x : hcodes.back())
+                if (x >= cg_[c]) throw Error(RC_INVALID_INPUT, "cluster code out of range of its level count");
+        }
     for (u32 mask = 1; mask < (1u << q); mask++) {
-        std::vector<const u32*> dims;
+        std::vector<size_t> dims;
         std::vector<u32> gs;
         for (size_t c = 0; c < q; c++)
             if (mask & (1u << c)) {
-                dims.push_back(d.ccodes[c].p);
+                dims.push_back(c);
                 gs.push_back(cg_[c]);
             }
+        d.subsets.emplace_back();
+        auto& s = d.subsets.back();
+        s.sign = dims.size() % 2 == 1 ? 1.0 : -1.0;
+        s.mask = mask;
         // the combined code, its levels numbered in ascending order of the tuple (factor.rs:255)
-        const u32* kc = dims[0];
-        u32 G = gs[0];
+        if (n <= HOST_GROUP_ROWS) {
+            std::vector<const std::vector<u32>*> parts;
+            for (size_t c : dims) parts.push_back(&hcodes[c]);
+            std::vector<u32> kc;
+            combine_codes(parts, gs, n, kc, s.G);
+            const std::vector<u32>& pi = ab_->row_order();
+            std::vector<u32> coff(size_t(s.G) + 1, 0);
+            for (size_t i = 0; i < n; i++) coff[kc[i] + 1]++;
+            for (u32 k = 0; k < s.G; k++) coff[k + 1] += coff[k];
+            std::vector<int> perm(n);
+            std::vector<u32> at(coff.begin(), coff.end() - 1);
+            for (size_t i = 0; i < n; i++) perm[at[kc[pi[i]]]++] = int(i);
+            s.perm.upload(perm, d.st);
+            s.coff.upload(coff, d.st);
+            continue;
+        }
+        std::vector<const u32*> parts;
+        for (size_t c : dims) parts.push_back(d.ccodes[c].p);
+        const u32* kc = parts[0];
+        s.G = gs[0];
         DBuf<u32> comb;
         if (dims.size() > 1) {
             for (size_t i = 0; i < dims.size(); i++)
-                check_codes_device(dims[i], n, gs[i], "cluster code out of range of its level count", d.st);
+                check_codes_device(parts[i], n, gs[i], "cluster code out of range of its level count", d.st);
             comb.alloc(n);
-            G = device_combine(dims, gs, n, comb.p, d.st);
+            s.G = device_combine(parts, gs, n, comb.p, d.st);
             kc = comb.p;
         }
-        d.subsets.emplace_back();
-        auto& s = d.subsets.back();
         s.perm.alloc(n);
-        s.coff.alloc(size_t(G) + 1);
-        group_rows_device(kc, pi_device(), n, G, reinterpret_cast<u32*>(s.perm.p), s.coff.p, d.st);
-        s.G = G;
-        s.sign = dims.size() % 2 == 1 ? 1.0 : -1.0;
-        s.mask = mask;
+        s.coff.alloc(size_t(s.G) + 1);
+        group_rows_device(kc, pi_device(), n, s.G, reinterpret_cast<u32*>(s.perm.p), s.coff.p, d.st);
     }
     CK(cudaStreamSynchronize(d.st));
 }
