@@ -1442,7 +1442,7 @@ void GpuSession::wildboot(double* rows, bool on_device, size_t nx, const OlsSpec
     const size_t tile = std::min(bs.tile, reps);
     DBuf<u64> Wd;
     Wd.alloc(tile * nwords);
-    const size_t ldz = (tile + 3) / 4 * 4;  // the block's columns rounded up to 4: 16-byte rows
+    const size_t ldz = tile < 4 ? tile : (tile + 3) / 4 * 4;  // 16-byte rows from four columns on
     DBuf<u32> Bd;
     Bd.alloc(size_t(G0) * ((tile + 31) / 32));
     U.alloc(tile * k + 1);
@@ -1456,10 +1456,13 @@ void GpuSession::wildboot(double* rows, bool on_device, size_t nx, const OlsSpec
         const u32 bt = u32(std::min(tile, reps - b0));
         k_boot_words<<<std::max(1, int((size_t(bt) * nwords + 255) / 256)), 256, 0, st>>>(bs.seed, b0, bt, nwords,
                                                                                          full ? 1 : 0, Wd.p);
-        const u32 btp = (bt + 3) / 4 * 4, cw32 = (bt + 31) / 32;
+        const u32 btp = bt < 4 ? bt : (bt + 3) / 4 * 4, cw32 = (bt + 31) / 32;
         k_boot_bits<<<blocks_for(size_t(G0) * cw32, 256), 256, 0, st>>>(Wd.p, nwords, bt, G0, cw32, Bd.p);
-        k_boot_gen<<<int(std::min<size_t>((n * (btp / 4) + BOOT_TB - 1) / BOOT_TB, 148 * 16)), BOOT_TB, 0, st>>>(
-            n, bt, btp, er.p, bcode_d.p, Bd.p, cw32, Z.p);
+        if (bt < 4)
+            k_boot_gen_few<<<blocks_for(n, BOOT_TB), BOOT_TB, 0, st>>>(n, bt, er.p, bcode_d.p, Bd.p, Z.p);
+        else
+            k_boot_gen<<<int(std::min<size_t>((n * (btp / 4) + BOOT_TB - 1) / BOOT_TB, 148 * 16)), BOOT_TB, 0, st>>>(
+                n, bt, btp, er.p, bcode_d.p, Bd.p, cw32, Z.p);
         d.launches += 3;
         ab_->residualize_device(Z.p, btp, bs.tol, bs.maxiter, false, nullptr, nullptr, bs.prec);
         if (k) {
