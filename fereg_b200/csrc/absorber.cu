@@ -222,7 +222,7 @@ struct Scratch {
     DBuf<double> rhsv, xv;  // the padded right-hand side and iterate of the PCG
     // inner FP32 buffers of the refined solve
     DBuf<float> fx, fb, fr, fz, fp, fq, ft, fpart, frhs, fx0;
-    DBuf<double> cg_rho, cg_rho_new, cg_pq, cg_gamma, cg_beta, cg_xb, cg_ss1, cg_floor, cg_ring, cg_xconst, cg_pfloor;
+    DBuf<double> cg_rho, cg_pq, cg_gamma, cg_beta, cg_xb, cg_ss1, cg_floor, cg_ring, cg_xconst, cg_pfloor;
     DBuf<int> cg_active, cg_nactive;
     DBuf<double> cg_ss0;
     int* h_nactive = nullptr;  // pinned: the loop control words (CgLoop::ctl) read back
@@ -290,7 +290,7 @@ struct Scratch {
     }
     DevWeights dw() const { return DevWeights{w_rows.p, cell_w.p, n1inv.p, nr.p, pl_w.p}; }
     CgState cg() {
-        return CgState{cg_rho.p, cg_rho_new.p, cg_pq.p,   cg_gamma.p,  cg_beta.p,   cg_xb.p,     cg_ss1.p,
+        return CgState{cg_rho.p,   cg_pq.p,   cg_gamma.p,  cg_beta.p,   cg_xb.p,     cg_ss1.p,
                        cg_floor.p, cg_ring.p, cg_xconst.p, cg_pfloor.p, cg_active.p, cg_nactive.p};
     }
     // The PCG loop's device state for R columns; the buffers of the vector kernels.
@@ -1030,12 +1030,12 @@ void allow_smem(K kernel, size_t bytes) {
 // into x (k x k), on `st`: by one CTA up to LDLT_WHOLE rows, else by panels of NB columns (16 up to
 // k = 1024, 8 beyond), each followed by its trailing update; the inverse by columns in registers up
 // to 1024 rows. keep_order (a hierarchy's coarsest level; blocks of at most 16 rows, where the
-// launches are all there is to gain) takes the elementwise divisions and row sums instead: on the
+// launches are all there is to gain, and of more than 1024) takes the elementwise divisions and row sums instead: on the
 // ill-conditioned graphs that reach a hierarchy the last bits of the preconditioner decide the
 // answer's eighth digit, and the same graph should give the same answer on every release.
 void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st, u64& launches, bool keep_order) {
     if (k <= 0) return;
-    keep_order = keep_order || k <= 16;
+    keep_order = keep_order || k <= 16 || k > 1024;
     auto factor = [&](auto nbc) {
         constexpr int NB = decltype(nbc)::value;
         for (int jb = 0; jb < k; jb += NB) {
@@ -1043,7 +1043,7 @@ void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st,
             if (keep_order) {
                 allow_smem(k_ldlt_panel_div<NB>, size_t(k) * NB * sizeof(double));
                 k_ldlt_panel_div<NB><<<1, 1024, size_t(k - jb) * NB * sizeof(double), st>>>(a, d, k, jb);
-            } else {
+            } else if constexpr (NB == 16) {
                 k_ldlt_panel<NB><<<1, 1024, 0, st>>>(a, d, k, jb);
             }
             launches++;
@@ -1071,7 +1071,7 @@ void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st,
     };
     using std::integral_constant;
     const integral_constant<int, 1> one;
-    if (keep_order || k > 1024) {
+    if (keep_order) {
         allow_smem(k_ldlt_inverse_rows, size_t(8) * k * sizeof(double));
         k_ldlt_inverse_rows<<<(k + 7) / 8, 256, size_t(8) * k * sizeof(double), st>>>(a, d, k, x);
     } else if (k <= 32) inverse(one, one);
@@ -1756,7 +1756,7 @@ std::vector<u64> body_key(Scratch& d, const Op& op, const T* x, const T* rhs_tru
                             (const void*)d.cg_rho.p, (const void*)d.cg_active.p, (const void*)d.cg_ring.p,
                             (const void*)d.cg_xb.p, (const void*)d.cg_beta.p, (const void*)d.cg_gamma.p,
                             (const void*)d.cg_pfloor.p, (const void*)d.cg_xconst.p, (const void*)d.cg_floor.p,
-                            (const void*)d.cg_ss1.p, (const void*)d.cg_pq.p, (const void*)d.cg_rho_new.p,
+                            (const void*)d.cg_ss1.p, (const void*)d.cg_pq.p,
                             (const void*)d.cg_nactive.p, (const void*)d.lp_rho_from.p, (const void*)d.lp_rho_at.p,
                             (const void*)d.lp_act.p})
         put(ptr);
@@ -2079,7 +2079,7 @@ SolveInfo GpuAbsorber::solve(double* rows, size_t r, double tol, size_t maxiter,
         d.z.alloc(tot);
         d.p.alloc(tot);
         d.q.alloc(tot);
-        for (auto* b : {&d.cg_rho, &d.cg_rho_new, &d.cg_pq, &d.cg_gamma, &d.cg_beta, &d.cg_ss1, &d.cg_floor, &d.cg_xconst,
+        for (auto* b : {&d.cg_rho, &d.cg_pq, &d.cg_gamma, &d.cg_beta, &d.cg_ss1, &d.cg_floor, &d.cg_xconst,
                         &d.cg_pfloor})
             b->alloc(rv);
         d.cg_xb.alloc(3 * rv);
@@ -2410,7 +2410,7 @@ u64 PcgDriver::run(DevOperator& op, double* x, const double* b, int R, const std
     d.p.alloc(tot);
     d.q.alloc(tot);
     d.cta.alloc(size_t(std::max(GRID_T, GRID_V)) * 3 * rv);
-    for (auto* buf : {&d.cg_rho, &d.cg_rho_new, &d.cg_pq, &d.cg_gamma, &d.cg_beta, &d.cg_ss1, &d.cg_floor, &d.cg_xconst,
+    for (auto* buf : {&d.cg_rho, &d.cg_pq, &d.cg_gamma, &d.cg_beta, &d.cg_ss1, &d.cg_floor, &d.cg_xconst,
                       &d.cg_pfloor})
         buf->alloc(rv);
     d.cg_xb.alloc(3 * rv);

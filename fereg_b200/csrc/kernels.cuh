@@ -90,7 +90,6 @@ __global__ void __launch_bounds__(TALL_TB) k_reduce_tall(const double* __restric
 // the reference's rules, 2 stopped at the FP32 precision floor of a refinement round.
 struct CgState {
     double* rho;
-    double* rho_new;
     double* pq;
     double* gamma;
     double* beta;
@@ -276,58 +275,44 @@ __global__ void k_small_apply(const double* __restrict__ minv, u32 ms, const T* 
 constexpr double PIVOT_TOL = 1e-10;
 constexpr double GROUND = 1e30;
 
-// The panel: thread t holds the panel elements of rows t, t + 1024, ... in registers, the pivot
-// rows' current column passes through shared memory, one barrier per column, the divisions by
-// the first warp alone. k = 910: the panel in shared memory with a division per element and two
+// The panel of a block of at most 1024 rows: thread t holds the panel elements of row t in registers,
+// the pivot rows' current column passes through shared memory, one barrier per column, the divisions
+// by the first warp alone. k = 910: the panel in shared memory with a division per element and two
 // barriers a column 59 us, here 19 us.
 template <int NB>
 __global__ void __launch_bounds__(1024) k_ldlt_panel(double* __restrict__ a, double* __restrict__ d, int k, int jb) {
-    constexpr int RPT = 16 / NB;  // rows per thread: k is at most 1024 with 16 columns, 2048 with 8
     __shared__ double top[2][NB], piv[2];
-    const int nb = min(NB, k - jb), rows = k - jb;
-    double p[RPT][NB];
+    const int nb = min(NB, k - jb), rows = k - jb, r = int(threadIdx.x);
+    double p[NB];
 #pragma unroll
-    for (int q = 0; q < RPT; q++) {
-        const int r = int(threadIdx.x) + 1024 * q;
-#pragma unroll
-        for (int c = 0; c < NB; c++) p[q][c] = (r < rows && c < nb && r >= c) ? a[size_t(jb + r) * k + jb + c] : 0.0;
-    }
+    for (int c = 0; c < NB; c++) p[c] = (r < rows && c < nb && r >= c) ? a[size_t(jb + r) * k + jb + c] : 0.0;
 #pragma unroll
     for (int jj = 0; jj < NB; jj++) {
         if (jj < nb) {
             // the pivot rows divide; the others would spend the FP64 pipe on the same quotients
-            if (int(threadIdx.x) < 32) {
-                double dj = __shfl_sync(FULL, p[0][jj], jj);
+            if (r < 32) {
+                double dj = __shfl_sync(FULL, p[jj], jj);
                 if (dj <= PIVOT_TOL) dj = GROUND;
-                if (threadIdx.x == 0) {
+                if (r == 0) {
                     d[jb + jj] = dj;
                     piv[jj & 1] = 1.0 / dj;
                 }
-                if (int(threadIdx.x) < NB) top[jj & 1][threadIdx.x] = p[0][jj] / dj;
+                if (r < NB) top[jj & 1][r] = p[jj] / dj;
             }
             __syncthreads();
-            const double inv = piv[jj & 1];
+            const double inv = piv[jj & 1], m = p[jj];
 #pragma unroll
-            for (int q = 0; q < RPT; q++) {
-                const int r = int(threadIdx.x) + 1024 * q;
-                const double m = p[q][jj];
-#pragma unroll
-                for (int l = jj + 1; l < NB; l++)
-                    if (l < nb) p[q][l] -= m * top[jj & 1][l];
-                if (r > jj) p[q][jj] = m * inv;  // L
-            }
+            for (int l = jj + 1; l < NB; l++)
+                if (l < nb) p[l] -= m * top[jj & 1][l];
+            if (r > jj) p[jj] = m * inv;  // L
         }
     }
 #pragma unroll
-    for (int q = 0; q < RPT; q++) {
-        const int r = int(threadIdx.x) + 1024 * q;
-#pragma unroll
-        for (int c = 0; c < NB; c++)
-            if (r < rows && c < nb && r > c) {
-                a[size_t(jb + r) * k + jb + c] = p[q][c];
-                a[size_t(jb + c) * k + jb + r] = p[q][c];
-            }
-    }
+    for (int c = 0; c < NB; c++)
+        if (r < rows && c < nb && r > c) {
+            a[size_t(jb + r) * k + jb + c] = p[c];
+            a[size_t(jb + c) * k + jb + r] = p[c];
+        }
 }
 
 // The panel in shared memory with a division per element: the rounding of the blocks that keep it
@@ -363,8 +348,6 @@ __global__ void __launch_bounds__(1024) k_ldlt_panel_div(double* __restrict__ a,
     }
 }
 
-// Tile (ti, tl), tl <= ti, of the trailing lower triangle (rows and columns from jb + nb): a[i][l]
-// -= sum over the panel's columns p of L[i][p] d_p L[l][p], for l <= i.
 // The whole factor by one CTA for k up to LDLT_WHOLE, without a launch per panel: thread (x, y)
 // holds the elements (y + 16 p, x + 16 q) of what is left of the matrix in registers, the current
 // column passes through shared memory, one barrier and one reciprocal per column. After 16 columns
@@ -433,6 +416,8 @@ __global__ void __launch_bounds__(256) k_ldlt_whole(double* __restrict__ a, doub
     }
 }
 
+// Tile (ti, tl), tl <= ti, of the trailing lower triangle (rows and columns from jb + nb): a[i][l]
+// -= sum over the panel's columns p of L[i][p] d_p L[l][p], for l <= i.
 template <int NB>
 __global__ void __launch_bounds__(256) k_ldlt_trail(double* __restrict__ a, const double* __restrict__ d, int k, int jb,
                                                     int nb) {

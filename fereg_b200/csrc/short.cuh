@@ -41,7 +41,7 @@ constexpr int WPB = 8;                // warps per CTA
 constexpr u32 PULL_WARP_MAX = 256;    // entries of the coordinate lists of one list tile
 constexpr int WLIST = 32;             // lists per list tile
 constexpr int WNB = 4;                // blocks whose coordinates a segment tile stages
-constexpr int WNO = WNB - 1;          // other blocks whose coordinates a list tile stages
+constexpr int WNO = WNB - 1;          // other blocks whose coordinates the operator's list pass stages
 
 // Warp tiles over short lists: (k0, k1, e0, e1) = lists [k0, k1) covering entries [e0, e1).
 struct WarpTiles {
@@ -354,11 +354,8 @@ struct PullStage {
     u32* kend;  // local end (entry) of each list (WLIST lists at most)
     u32* seg;   // PULL_WARP_MAX entries
     u32* cell;
-    u32* oth;   // WNO x PULL_WARP_MAX
 };
-__host__ __device__ constexpr size_t pull_bytes() {
-    return al16(WLIST * 4) + al16(PULL_WARP_MAX * 4) * 2 + al16(WNO * PULL_WARP_MAX * 4);
-}
+__host__ __device__ constexpr size_t pull_bytes() { return al16(WLIST * 4) + al16(PULL_WARP_MAX * 4) * 2; }
 __device__ __forceinline__ PullStage pull_stage_at(unsigned char* p) {
     PullStage s;
     s.kend = reinterpret_cast<u32*>(p);
@@ -366,23 +363,15 @@ __device__ __forceinline__ PullStage pull_stage_at(unsigned char* p) {
     s.seg = reinterpret_cast<u32*>(p);
     p += al16(PULL_WARP_MAX * 4);
     s.cell = reinterpret_cast<u32*>(p);
-    p += al16(PULL_WARP_MAX * 4);
-    s.oth = reinterpret_cast<u32*>(p);
     return s;
 }
 
-__device__ __forceinline__ void stage_pull(const DevStruct& S, u32 k0, u32 k1, u32 e0, u32 e1, const PullStage& st,
-                                           bool cells, u32 nstage) {
+__device__ __forceinline__ void stage_pull(const DevStruct& S, u32 k0, u32 k1, u32 e0, u32 e1, const PullStage& st) {
     const u32 lane = wlane();
     if (lane < k1 - k0) st.kend[lane] = S.pl_off[k0 + lane + 1] - e0;
-    const u32 no = S.nb - 1;
     for (u32 i = lane; i < e1 - e0; i += 32) {
-        const u32 e = e0 + i;
-        st.seg[i] = __ldcs(S.pl_seg + e);
-        if (cells) st.cell[i] = __ldcs(S.pl_cell + e);
-#pragma unroll
-        for (u32 o = 0; o < u32(WNO); o++)
-            if (o < nstage) st.oth[o * PULL_WARP_MAX + i] = __ldcs(S.pl_other + size_t(e) * no + o);
+        st.seg[i] = __ldcs(S.pl_seg + e0 + i);
+        st.cell[i] = __ldcs(S.pl_cell + e0 + i);
     }
 }
 
@@ -715,7 +704,7 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_wpull_rhs(DevStruct S, DevWeigh
     uint4 tb = wid < wt.n ? wt.t[wid] : make_uint4(0, 0, 0, 0);
     for (u32 tile = wid; tile < wt.n; tile += nw) {
         const u32 k0 = tb.x, k1 = tb.y;
-        stage_pull(S, k0, k1, tb.z, tb.w, st, true, 0u);
+        stage_pull(S, k0, k1, tb.z, tb.w, st);
         if (tile + nw < wt.n) tb = wt.t[tile + nw];
         __syncwarp();
         // this lane's column summed over the entries ib, ib + step, ... < ie of a list

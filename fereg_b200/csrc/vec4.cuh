@@ -43,13 +43,6 @@ __device__ __forceinline__ void add4(V4<T>& s, const V4<T>& v) {
     s.d += v.d;
 }
 template <class T>
-__device__ __forceinline__ void sub4(V4<T>& s, const V4<T>& v) {
-    s.a -= v.a;
-    s.b -= v.b;
-    s.c -= v.c;
-    s.d -= v.d;
-}
-template <class T>
 __device__ __forceinline__ void fma4(V4<T>& s, T w, const V4<T>& v) {
     s.a += w * v.a;
     s.b += w * v.b;
