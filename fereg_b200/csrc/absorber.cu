@@ -189,11 +189,11 @@ struct Scratch {
     u64 escalations = 0;
     // structure
     DBuf<u32> seg_off, coord, cell_row, pl_off, pl_cell, pl_seg, pl_other;
-    DevTiles seg_tiles, pull_tiles;      // CTA tiles of the long lists
+    DevTiles seg_tiles, pull_tiles;      // tiles of the long segments and lists
     DevWarpTiles wseg, wpull;            // warp tiles of the short lists
     DBuf<u32> wseg_segs;                 // the segments of the warp tiles, in order
     DBuf<u32> aseg_segs;                 // the operator's lane-group segments (at most LONG_SEG cells)
-    DevTiles aseg_tiles;                 // the operator's CTA tiles (longer segments)
+    DevTiles aseg_tiles;                 // the operator's tiles of longer segments
     u32 ms_acc = 0, ns_acc = 0;  // small coordinates / blocks summed in the segment passes
     size_t nrows = 0;
     // weights
@@ -439,7 +439,7 @@ GpuAbsorber::GpuAbsorber(const std::vector<const u32*>& codes, const std::vector
         d_->wseg_segs.upload(segs, stream_);
         d_->seg_tiles.upload(ct, stream_);
         // the operator's segment pass: lane groups walk every segment of at most LONG_SEG cells (in
-        // order), CTA tiles take the longer ones
+        // order), a warp per tile the longer ones
         std::vector<u32> asegs;
         for (u32 s = 0; s < hs_.g1; s++)
             if (hs_.seg_off[s + 1] - hs_.seg_off[s] <= LONG_SEG) asegs.push_back(s);
@@ -1029,10 +1029,10 @@ void allow_smem(K kernel, size_t bytes) {
 // Grounded LDL^T of the k x k row-major `a` (lower triangle read, overwritten) and its inverse
 // into x (k x k), on `st`: by one CTA up to LDLT_WHOLE rows, else by panels of NB columns (16 up to
 // k = 1024, 8 beyond), each followed by its trailing update; the inverse by columns in registers up
-// to 1024 rows. keep_order (a hierarchy's coarsest level; blocks of at most 16 rows, where the
-// launches are all there is to gain, and of more than 1024) takes the elementwise divisions and row sums instead: on the
-// ill-conditioned graphs that reach a hierarchy the last bits of the preconditioner decide the
-// answer's eighth digit, and the same graph should give the same answer on every release.
+// to 1024 rows. keep_order takes the elementwise divisions and row sums instead: blocks of at most
+// 16 rows, where the launches are all there is to gain, those of more than 1024, and a hierarchy's
+// coarsest level, whose rounding is frozen like the narrow vector steps' (pcg.cuh) at 59 us a panel
+// for 19.
 void dense_ldlt_inverse(double* a, double* d, int k, double* x, cudaStream_t st, u64& launches, bool keep_order) {
     if (k <= 0) return;
     keep_order = keep_order || k <= 16 || k > 1024;
@@ -1135,10 +1135,10 @@ void launch_small_rows(Scratch& d, const DevStruct& S, const T* P, int Rv, T* Y,
 }
 
 // Y = S P on the PCG's padded vectors (Rv a multiple of 4). Short segments: one lane group per
-// segment (k_vseg_apply); long segments: CTA tiles, their slices' partials completed by k_fix.
-// Short coordinate lists: warp tiles (k_vpull_apply); long ones: CTA tiles and k_fix. The small
-// coordinates' rows (ms_acc > 0) come from the dense rows of S: here, or, without small_rows_too,
-// from the caller's k_wide_pq.
+// segment (k_vseg_apply); long segments: a warp per tile (k_ltile_apply), their slices' partials
+// completed by k_fix. Short coordinate lists: warp tiles (k_vpull_apply); long ones: a CTA per tile
+// (k_ltile_pull) and k_fix. The small coordinates' rows (ms_acc > 0) come from the dense rows of S:
+// here, or, without small_rows_too, from the caller's k_wide_pq.
 template <class T>
 void launch_apply(Scratch& d, const DevStruct& S, const DevWeights& W, const T* P, int Rv, T* Y, T* t, T* part,
                   cudaStream_t st, bool small_rows_too = true) {
@@ -1706,7 +1706,8 @@ struct FeOp {
     }
     // The vector steps by column tiles (k_wide_*): wide blocks, and weighted systems with a small
     // preconditioner, where fewer kernels pay (1.07e6 weighted rows, 8 columns, an iteration's vector
-    // kernels: 43 us by the narrow ones, 30). Unweighted ones keep the narrow kernels' order of sums.
+    // kernels: 43 us by the narrow ones, 30). Unweighted ones stay on the narrow kernels, whose order
+    // of sums is frozen (pcg.cuh), at that cost.
     bool tiled(int R) const { return R > WIDE_R || (W.cell_w && fused(R)); }
     u32 ms_acc() const { return S.ms_acc; }
     // iterations in a graph's body: a hierarchy's V-cycle does not look at the halt word

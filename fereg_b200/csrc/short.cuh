@@ -1,5 +1,5 @@
 // Kernels for the short lists: segments of at most WT cells (and WT rows) and coordinate lists
-// of at most PULL_WARP_MAX entries. Longer lists go to the CTA tiles (tiles.cuh).
+// of at most PULL_WARP_MAX entries. Longer ones go to the tiles of long.cuh.
 //
 // The operator's passes (k_vseg_apply, k_vpull_apply) run on the PCG's padded vectors (a row
 // stride that is a multiple of 4): lane j of a group of L lanes holds 4 consecutive columns,

@@ -1,11 +1,12 @@
-// Tile kernels over the cell structure: the segment passes (per FE1 level) and the coordinate
-// pulls (per reduced coordinate) of the rhs, operator and residualize steps.
+// The cell structure's device tables, and the CTA-tile kernels over the long segments (per FE1 level):
+// the right-hand side where small coordinates are summed (k_seg_rhs, k_rhs_small_slices), the slices'
+// partials and their completion.
 //
-// A CTA takes one tile at a time: up to TILE consecutive cells of whole segments (or TILE
-// consecutive entries of the coordinate-sorted lists), or a TILE-sized slice of one long list.
-//   phase A  thread (slot, column) over the tile's cells/entries: independent gathers, the
-//            per-cell value goes to shared memory;
-//   phase B  thread (segment or coordinate, column): the sum over its cells in list order.
+// A CTA takes one tile at a time: up to TILE consecutive cells of whole segments, or a TILE-sized
+// slice of one long segment.
+//   phase A  thread (slot, column) over the tile's cells: independent gathers, the per-cell value
+//            goes to shared memory;
+//   phase B  thread (segment, column): the sum over its cells in list order.
 // Slices of long lists write partial sums that k_fix adds in slice order. Column blocks wider
 // than RC_MAX are walked in chunks.
 //

@@ -311,8 +311,8 @@ __global__ void __launch_bounds__(256) k_small_rows(const u32* __restrict__ seg_
 // For every entry S[k][k] += 1; once per segment s of the run S[k][l] -= c_{s,k} / n1_s for each of the
 // c_{s,l} cells that hold l (csk: the counts, g1 x ms). A lane's sum is one chain over the item, in
 // entry order; the loads of 8 entries are in flight together. This is the block of a panel's years
-// on a one-row-per-cell panel; its rounding steers the PCG's path, which on an ill-conditioned graph
-// decides the answer's eighth digit, so the order of the sums is the one this block always had.
+// on a one-row-per-cell panel, whose order of sums is frozen as that of the vector steps is (pcg.cuh);
+// blocks of every other shape take the faster forms above.
 // 1e6 segments of 10 cells, 10 coordinates: 7.5 ms with one lane an item, 0.70 ms here (0.16 as tiles).
 __global__ void __launch_bounds__(256) k_small_ordered(u32 ms, const double* __restrict__ n1inv,
                                                        const double* __restrict__ csk, const u32* __restrict__ pl_seg,
