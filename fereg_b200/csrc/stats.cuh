@@ -920,9 +920,15 @@ __global__ void __launch_bounds__(256) k_uf_count(const u32* __restrict__ parent
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(total, c);
 }
 
+// Every vertex's parent set to its root. The walk writes nothing but the vertex's own entry (uf_find's
+// halving could put an older ancestor back over an entry that its thread has set), and no link runs
+// beside it, so every entry is a root afterwards.
 __global__ void k_uf_flatten(u32* parent, u32 nv) {
-    for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
-        parent[v] = uf_find(parent, v);
+    for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
+        u32 r = v;
+        for (u32 p = __ldca(parent + r); p != r; p = __ldca(parent + r)) r = p;
+        if (r != v) parent[v] = r;
+    }
 }
 
 // flags[l] = 1 when a-level l is its component's root.
