@@ -699,11 +699,11 @@ void GpuAbsorber::build_amg() {
             }
             A.lv.push_back(dl);
         }
-        // generalized inverse of the coarsest level: unit-diagonal scaling over the nodes with a
-        // positive diagonal, grounded LDL^T, explicit inverse (the small block's kernels)
+        // generalized inverse of the coarsest level: unit-diagonal scaling over the nodes that are not
+        // left out, grounded LDL^T, explicit inverse (the small block's kernels)
         std::vector<u32> keep;
         for (u32 i = 0; i < nL; i++)
-            if (H.coarse[size_t(i) * nL + i] > 0.0) keep.push_back(i);
+            if (H.levels.back().dinv[i] > 0.0) keep.push_back(i);
         const size_t k = keep.size();
         std::vector<double> scale(k), ak(k * k);
         for (size_t i = 0; i < k; i++) scale[i] = 1.0 / std::sqrt(H.coarse[size_t(keep[i]) * (nL + 1)]);

@@ -159,6 +159,8 @@ AmgLevel assemble_block(const HostStructure& hs, size_t b, const double* cw, con
     AmgLevel L;
     L.n = g;
     L.A = rl.to_csr(g);
+    L.mag.assign(g, 0.0);
+    for (size_t c = 0; c < M; c++) L.mag[coord[c] - off] += cw ? cw[c] : 1.0;
     set_dinv(L, out);
     return L;
 }
@@ -216,6 +218,22 @@ u32 aggregate(const AmgLevel& L, std::vector<int>& agg) {
     for (u32 i = 0; i < n; i++)
         if (agg[i] == FREE) agg[i] = int(nc++);
     return nc;
+}
+
+// Coarse nodes that stand for a whole component of the fine level: the row sums there are 0, so their
+// diagonal P'A P is the round-off of the entries it was formed from (1e-31 next to entries of order 1),
+// and its reciprocal would swamp the cycle. Like the redundant coordinates of the finest level they are
+// left out, at 1e-12 of the weights behind them (mag, carried along as P'mag P's diagonal).
+std::vector<bool> null_nodes(const AmgLevel& fine, AmgLevel& coarse) {
+    const std::vector<double> d = diagonal(coarse.A);
+    std::vector<bool> out(coarse.n);
+    coarse.mag.assign(coarse.n, 0.0);
+    for (u32 I = 0; I < coarse.n; I++) {
+        for (u32 e = fine.Pt.ptr[I]; e < fine.Pt.ptr[I + 1]; e++)
+            coarse.mag[I] += fine.Pt.val[e] * fine.Pt.val[e] * fine.mag[fine.Pt.col[e]];
+        out[I] = !(d[I] > 1e-12 * coarse.mag[I]);
+    }
+    return out;
 }
 
 // P = (I - (2/3) D^-1 A) P0 for the piecewise-constant P0 of `agg` (rows of left-out nodes empty).
@@ -282,8 +300,7 @@ AmgHierarchy amg_build(const HostStructure& hs, size_t block, const double* cell
         AmgLevel C;
         C.n = nc;
         C.A = spgemm(fine.Pt, spgemm(fine.A, fine.P));
-        std::vector<bool> out(nc, false);
-        set_dinv(C, out);
+        set_dinv(C, null_nodes(fine, C));
         H.levels.push_back(std::move(C));
     }
     // the coarsest level as a dense matrix (its generalized inverse is formed on the device)

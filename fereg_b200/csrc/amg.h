@@ -18,10 +18,11 @@
 // spectrum in [0, 2]) and the coarse operator A_c = P^T A P, until at most AMG_COARSE nodes
 // remain. P0 and P both keep the constants, so every level is again a Laplacian. The coarsest
 // level is inverted densely with the grounded LDL^T of the small block (pivots below 1e-10 of the
-// unit-scaled diagonal grounded, precond/dense.rs:1-38), which handles the null space.
-// Redundant coordinates (operator.rs:21) are left out (their preconditioned value is 0, as under
-// Jacobi). On ring and band firm graphs the smoothed hierarchy keeps PCG at ~15 iterations
-// independent of size, where Jacobi needs thousands.
+// unit-scaled diagonal grounded, precond/dense.rs:1-38), which handles the null space of components
+// that reach it with several nodes. Redundant coordinates (operator.rs:21) are left out (their
+// preconditioned value is 0, as under Jacobi), and so is a coarse node that is all of its component. On
+// ring and band firm graphs the smoothed hierarchy keeps PCG at ~15 iterations independent of size,
+// where Jacobi needs thousands.
 #pragma once
 
 #include <vector>
@@ -44,6 +45,7 @@ struct AmgLevel {
     u32 n = 0;
     Csr A;                     // the level's operator (diagonal included)
     std::vector<double> dinv;  // AMG_OMEGA / a_ii (0: left out)
+    std::vector<double> mag;   // the weights the diagonal was formed from (its round-off is of this size)
     Csr P, Pt;                 // prolongation to this level from the next (n x n_c) and its transpose
 };
 
